@@ -1,5 +1,5 @@
-"""The packed Plummer sum at the edges of its tiles and of the rules that choose
-it, against sums in numpy."""
+"""The packed Plummer sum and the row-wise FP64 mollified sum at the edges of
+their tiles and of the rules that choose them, against sums in numpy."""
 import numpy as np
 import pytest
 
@@ -71,3 +71,34 @@ def test_plummer_general_tiles(cuda, what):
             assert np.isfinite(got[100]).all()
             if what == "inf":
                 assert not np.isfinite(np.delete(got, 100, 0)).any()
+
+
+@pytest.mark.parametrize("n,m,param,Lx,Ly", [(1, 3, 0.05, 1.0, 1.0), (255, 1, 0.3, 1.0, 1.0), (256, 257, 0.05, 0.7, 1.3),
+                                             (257, 256, 1e-5, 1.0, 1.0), (3000, 100, 0.02, 1.0, 2.0)])
+def test_mollified_rows(cuda, n, m, param, Lx, Ly):
+    from vortexparticlemc_cuda_gb300 import phash as P
+    rng = np.random.default_rng(n)
+    L = np.array([Lx, Ly])
+    pos = (rng.random((n, 2)) * L).astype(np.float32)
+    om = rng.normal(size=n).astype(np.float32)
+    om[::5] = 0.0
+    pts = (rng.random((m, 2)) * L).astype(np.float32)
+    pts[0] = pos[0]                                   # an image at r = 0
+    got = P.direct_velocity(to_dev(pos, cuda), to_dev(om, cuda), pts=to_dev(pts, cuda), param=param, Lx=Lx,
+                            Ly=Ly).cpu().numpy()
+    u, size = np.zeros((m, 2)), np.zeros((m, 2))
+    for a in (-1, 0, 1):
+        for b in (-1, 0, 1):
+            d = pts[:, None, :].astype(np.float64) - (pos.astype(np.float64) + np.array([a * Lx, b * Ly]))[None]
+            r2 = (d ** 2).sum(-1)
+            q = np.minimum(np.sqrt(r2) / param, 1.0)
+            inner = 1.2 * q ** 5 - 1.5 * q ** 4 + 0.5 * q ** 2
+            outer = q ** 2 - 2 * q ** 3 + 1.5 * q ** 4 - 0.4 * q ** 5 - 0.0125
+            mass = np.where(r2 < param ** 2, 80 / 7 * np.where(q <= 0.5, inner, outer), 1.0)
+            with np.errstate(divide="ignore", invalid="ignore"):
+                k = np.where(r2 > 0, om.astype(np.float64) / (2 * np.pi) * mass / r2, 0.0)
+            t = np.stack([-k * d[..., 1], k * d[..., 0]], -1)
+            u += t.sum(1)
+            size += np.abs(np.sqrt(r2) * k).sum(1)[:, None]
+    # ~20 roundings a term, one add a source and chunk; the mass near the edge of the inner pieces cancels ~10 digits' units
+    assert (np.abs(got - u) <= (n + 60) * 2.0 ** -52 * size + 1e-300).all()
