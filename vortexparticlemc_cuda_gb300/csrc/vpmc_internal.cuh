@@ -71,7 +71,8 @@ struct Carver {
 };
 
 constexpr int kScratchSlots = 8;
-enum ScratchSlot { SLOT_HASH = 0, SLOT_QUERY = 1, SLOT_CG = 2, SLOT_DIRECT = 3, SLOT_MISC = 4 };
+enum ScratchSlot { SLOT_HASH = 0, SLOT_QUERY = 1, SLOT_CG = 2, SLOT_DIRECT = 3, SLOT_MISC = 4,
+                   SLOT_MATRIX = 5, SLOT_SOLVE = 6 };
 
 }  // namespace vpmc
 
@@ -119,12 +120,6 @@ int radix_sort(vpmc_context* ctx, const uint32_t* keys_in, const uint32_t* vals_
 int exclusive_scan(vpmc_context* ctx, const uint32_t* in, uint32_t* out, long n, uint32_t* tmp,
                    bool write_total);
 int bits_for(uint64_t max_value_exclusive);
-
-// ---------------------------------------------------------- deterministic FP64
-// out[0] = sum_i a[i]*b[i] (b == nullptr: sum a[i]^2), fixed reduction tree.
-int dot_f64(vpmc_context* ctx, const double* a, const double* b, long n, double* out_dev,
-            double* tmp /* >= dot_tmp_elems(n) */);
-size_t dot_tmp_elems(long n);
 
 }  // namespace vpmc
 

@@ -1,4 +1,4 @@
-// vpmc_sort.cu -- exclusive scan, stable LSD radix sort, deterministic FP64 dot.
+// vpmc_sort.cu -- exclusive scan, stable LSD radix sort.
 //
 // Design: reduce-then-scan everywhere (no inter-block spin waits).  The radix
 // sort is the classic three-kernel pass (tile digit histograms, one scan of the
@@ -167,42 +167,6 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_downsweep(
     }
 }
 
-constexpr int kDotThreads = 256;
-constexpr int kDotMaxBlocks = 1024;
-
-__global__ void __launch_bounds__(kDotThreads) k_dot_partial(const double* __restrict__ a,
-                                                             const double* __restrict__ b, long n,
-                                                             double* __restrict__ part) {
-    __shared__ double sh[kDotThreads];
-    double s = 0.0;
-    for (long i = long(blockIdx.x) * kDotThreads + threadIdx.x; i < n; i += long(gridDim.x) * kDotThreads)
-        s += b ? a[i] * b[i] : a[i] * a[i];
-    sh[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = kDotThreads / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
-}
-
-__global__ void __launch_bounds__(kDotMaxBlocks) k_dot_final(const double* __restrict__ part, int nb,
-                                                             double* __restrict__ out) {
-    __shared__ double sh[kDotMaxBlocks];
-    sh[threadIdx.x] = threadIdx.x < nb ? part[threadIdx.x] : 0.0;
-    __syncthreads();
-    for (int o = kDotMaxBlocks / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[0] = sh[0];
-}
-
-int dot_blocks(long n) {
-    long b = (n + 4 * kDotThreads - 1) / (4 * kDotThreads);
-    return int(b < 1 ? 1 : (b > kDotMaxBlocks ? kDotMaxBlocks : b));
-}
-
 }  // namespace
 
 size_t scan_tmp_elems(long n) {
@@ -275,15 +239,6 @@ int radix_sort(vpmc_context* ctx, const uint32_t* keys_in, const uint32_t* vals_
     }
     *keys_out = const_cast<uint32_t*>(kc);
     *vals_out = const_cast<uint32_t*>(vc);
-    return VPMC_OK;
-}
-
-size_t dot_tmp_elems(long n) { return size_t(dot_blocks(n)) + 1; }
-
-int dot_f64(vpmc_context* ctx, const double* a, const double* b, long n, double* out_dev, double* tmp) {
-    const int nb = dot_blocks(n);
-    VPMC_LAUNCH(k_dot_partial, nb, kDotThreads, 0, ctx->stream, a, b, n, tmp);
-    VPMC_LAUNCH(k_dot_final, 1, kDotMaxBlocks, 0, ctx->stream, tmp, nb, out_dev);
     return VPMC_OK;
 }
 
