@@ -163,8 +163,7 @@ int vpmc_context_set_wait_limit(vpmc_context* c, uint32_t polls) {
 int vpmc_context_sync(vpmc_context* c) {
     if (!c) return VPMC_ERR_INVALID;
     VPMC_CUDA(cudaSetDevice(c->device));
-    VPMC_CUDA(cudaStreamSynchronize(c->stream));
-    return collect_flags(c);
+    return collect_flags(c);   // its copy is ordered after the stream's work, and waited for
 }
 
 size_t vpmc_context_scratch_bytes(vpmc_context* c) {

@@ -226,7 +226,6 @@ struct GridBufs {
     int rows = 1;               // candidate sub-rows per cell (candidates sorted by cell, then sub-row in y)
     long n = 0;                 // particles covered
     uint32_t* keys = nullptr;   // n
-    uint32_t* count = nullptr;  // nbins * rows + 1
     uint32_t* start = nullptr;  // nbins * rows + 1: candidate range of sub-row (bin * rows + r)
     uint32_t* cstart = nullptr; // nbins + 1: candidate range of a whole bin (= start when rows == 1)
     Cand* cand = nullptr;       // n

@@ -1,15 +1,15 @@
 // vpmc_hash.cu -- the reference-shaped spatial hash (FillCells / CountingSort)
 // and the sign subsets with their FP64 |omega| CDFs.
 //
-// Hash: one key kernel (cell of sub[i], histogram into cell_num), an exclusive
-// scan (cell_acc), and a stable radix sort of (cell, local index) pairs, whose
-// values are vp_sort.  The result equals the reference's sequential counting
+// Hash: one key kernel (cell of sub[i]), a stable radix sort of (cell, local index)
+// pairs, whose values are vp_sort, and each cell's first entry among the sorted
+// cells (cell_acc); FillCells alone counts the cells and scans the counts.  The result equals the reference's sequential counting
 // sort (src/cpu/hash.cpp:36-48) bit for bit: members of a cell ascend by local
 // index.  The reference's CUDA scatter (src/cuda/hash.cu:27-39) uses atomicSub
 // and is order-nondeterministic; this one is deterministic.
 #include <vector>
 
-#include "vpmc_internal.cuh"
+#include "vpmc_blocksort.cuh"
 
 namespace vpmc {
 namespace {
@@ -53,6 +53,48 @@ __global__ void __launch_bounds__(kHashThreads) k_fill_cells(int rshx, int rshy,
         for (int c = threadIdx.x; c < ncell; c += blockDim.x)
             if (hist[c]) atomicAdd(&cell_num[c], hist[c]);
     }
+}
+
+// The cells alone (the counts of a hash come from its sorted cells).
+__global__ void __launch_bounds__(kHashThreads) k_cells(int rshx, int rshy, float inv_hx, float inv_hy,
+                                                        const int* __restrict__ sub, const float2* __restrict__ pos,
+                                                        long N, int* __restrict__ vp_cell) {
+    for (long i = long(blockIdx.x) * blockDim.x + threadIdx.x; i < N; i += long(gridDim.x) * blockDim.x) {
+        const float2 p = pos[sub ? sub[i] : int(i)];
+        const int ix = min(max(floor_int(p.x * inv_hx), 0), rshx - 1);
+        const int iy = min(max(floor_int(p.y * inv_hy), 0), rshy - 1);
+        vp_cell[i] = ix * rshy + iy;
+    }
+}
+
+// A small hash (see vpmc_blocksort.cuh): cells, order and ranges in one launch of
+// one CTA.  11,003 particles on 128^2 cells, the whole call: 149 -> 52 us (kernel 15.6).
+__global__ void __launch_bounds__(kSmallThreads) k_hash_small(int rshx, int rshy, float inv_hx, float inv_hy,
+                                                              const int* __restrict__ sub,
+                                                              const float2* __restrict__ pos, int N, int ibits,
+                                                              int* __restrict__ cell_num, int* __restrict__ cell_acc,
+                                                              int* __restrict__ vp_cell, int* __restrict__ vp_sort) {
+    extern __shared__ uint32_t words[];
+#pragma unroll 4
+    for (int i = threadIdx.x; i < N; i += kSmallThreads) {
+        const float2 p = pos[sub ? sub[i] : i];
+        const int ix = min(max(floor_int(p.x * inv_hx), 0), rshx - 1);
+        const int iy = min(max(floor_int(p.y * inv_hy), 0), rshy - 1);
+        const int c = ix * rshy + iy;
+        vp_cell[i] = c;
+        words[i] = uint32_t(c);
+    }
+    if (cell_num)
+        for (int c = threadIdx.x; c < rshx * rshy; c += kSmallThreads) cell_num[c] = 0;
+    small_sort(words, N, rshx * rshy, ibits, reinterpret_cast<uint32_t*>(vp_sort), reinterpret_cast<uint32_t*>(cell_acc));
+}
+
+__global__ void k_cell_starts(const uint32_t* __restrict__ keys, int N, int ncell, int* __restrict__ cell_acc,
+                              int* __restrict__ cell_num) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= ncell) return;
+    cell_acc[c] = int(lower_bound_key(keys, uint32_t(N), uint32_t(c)));
+    if (cell_num) cell_num[c] = 0;
 }
 
 __global__ void k_max_key(const int* __restrict__ keys, long n, int* __restrict__ out) {
@@ -248,26 +290,11 @@ int hash_scratch(vpmc_context* ctx, long N, HashScratch* h) {
     return VPMC_OK;
 }
 
-int sort_cells(vpmc_context* ctx, long N, int ncell, const int* vp_cell, int* vp_sort) {
-    HashScratch h;
-    VPMC_TRY(hash_scratch(ctx, N, &h));
-    uint32_t *ks = nullptr, *vs = nullptr;
-    VPMC_TRY(radix_sort(ctx, reinterpret_cast<const uint32_t*>(vp_cell), nullptr, N, bits_for(uint64_t(ncell)), h.rs,
-                        &ks, &vs));
-    VPMC_CUDA(cudaMemcpyAsync(vp_sort, vs, sizeof(int) * size_t(N), cudaMemcpyDeviceToDevice, ctx->stream));
-    return VPMC_OK;
-}
-
-}  // namespace
-
-extern "C" {
-
-int vpmc_fill_cells(vpmc_context* ctx, int rshx, int rshy, float Lx, float Ly, int N, const int* sub,
-                    const float* pos, int* cell_num, int* cell_acc, int* vp_cell) {
-    if (!ctx || rshx < 1 || rshy < 1 || N < 0 || !(Lx > 0.f) || !(Ly > 0.f)) return VPMC_ERR_INVALID;
+// Cells, counts and their exclusive prefix, queued on the context's stream.
+int fill_cells_queued(vpmc_context* ctx, int rshx, int rshy, float Lx, float Ly, int N, const int* sub,
+                      const float* pos, int* cell_num, int* cell_acc, int* vp_cell) {
     if ((N > 0 && (!pos || !vp_cell)) || !cell_num || !cell_acc) return VPMC_ERR_INVALID;
     if (long(rshx) * rshy > (1L << 30)) return VPMC_ERR_CAPACITY;
-    VPMC_CUDA(cudaSetDevice(ctx->device));
     const int ncell = rshx * rshy;
     cudaStream_t st = ctx->stream;
     VPMC_CUDA(cudaMemsetAsync(cell_num, 0, sizeof(int) * size_t(ncell), st));
@@ -280,9 +307,33 @@ int vpmc_fill_cells(vpmc_context* ctx, int rshx, int rshy, float Lx, float Ly, i
     dry.take<uint32_t>(scan_tmp_elems(ncell) + 1);
     char* base = nullptr;
     VPMC_TRY(scratch(ctx, SLOT_MISC, dry.off, &base));
-    VPMC_TRY(exclusive_scan(ctx, reinterpret_cast<const uint32_t*>(cell_num), reinterpret_cast<uint32_t*>(cell_acc),
-                            ncell, reinterpret_cast<uint32_t*>(base), false));
-    VPMC_CUDA(cudaStreamSynchronize(st));
+    return exclusive_scan(ctx, reinterpret_cast<const uint32_t*>(cell_num), reinterpret_cast<uint32_t*>(cell_acc),
+                          ncell, reinterpret_cast<uint32_t*>(base), false);
+}
+
+// vp_sort, and (when asked for) the cells' first entries from the sorted cells.
+int sort_cells(vpmc_context* ctx, long N, int ncell, const int* vp_cell, int* vp_sort, int* cell_acc = nullptr,
+               int* cell_num = nullptr) {
+    HashScratch h;
+    VPMC_TRY(hash_scratch(ctx, N, &h));
+    uint32_t *ks = nullptr, *vs = nullptr;
+    VPMC_TRY(radix_sort(ctx, reinterpret_cast<const uint32_t*>(vp_cell), nullptr, N, bits_for(uint64_t(ncell)), h.rs,
+                        &ks, &vs));
+    if (cell_acc)
+        VPMC_LAUNCH(k_cell_starts, (ncell + 127) / 128, 128, 0, ctx->stream, ks, int(N), ncell, cell_acc, cell_num);
+    VPMC_CUDA(cudaMemcpyAsync(vp_sort, vs, sizeof(int) * size_t(N), cudaMemcpyDeviceToDevice, ctx->stream));
+    return VPMC_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int vpmc_fill_cells(vpmc_context* ctx, int rshx, int rshy, float Lx, float Ly, int N, const int* sub,
+                    const float* pos, int* cell_num, int* cell_acc, int* vp_cell) {
+    if (!ctx || rshx < 1 || rshy < 1 || N < 0 || !(Lx > 0.f) || !(Ly > 0.f)) return VPMC_ERR_INVALID;
+    VPMC_CUDA(cudaSetDevice(ctx->device));
+    VPMC_TRY(fill_cells_queued(ctx, rshx, rshy, Lx, Ly, N, sub, pos, cell_num, cell_acc, vp_cell));
     return collect_flags(ctx);
 }
 
@@ -308,7 +359,6 @@ int vpmc_counting_sort(vpmc_context* ctx, int N, int ncell, int* cell_num, const
     }
     VPMC_TRY(sort_cells(ctx, N, ncell, vp_cell, vp_sort));
     if (cell_num) VPMC_CUDA(cudaMemsetAsync(cell_num, 0, sizeof(int) * size_t(ncell), st));
-    VPMC_CUDA(cudaStreamSynchronize(st));
     return collect_flags(ctx);
 }
 
@@ -318,18 +368,28 @@ int vpmc_hash_build(vpmc_context* ctx, int rshx, int rshy, float Lx, float Ly, i
         return VPMC_ERR_INVALID;
     if (!(Lx > 0.f) || !(Ly > 0.f)) return VPMC_ERR_INVALID;
     VPMC_CUDA(cudaSetDevice(ctx->device));
-    const int ncell = rshx * rshy;
-    int* cn = cell_num;
-    if (!cn) {
-        // borrow scratch for the counts when the caller does not want them
-        char* base = nullptr;
-        VPMC_TRY(scratch(ctx, SLOT_QUERY, sizeof(int) * size_t(ncell) + 256, &base));
-        cn = reinterpret_cast<int*>(base);
+    if (small_sort_fits(N, long(rshx) * rshy)) {
+        static bool configured[64] = {};
+        if (ctx->device < 64 && !configured[ctx->device]) {
+            VPMC_CUDA(cudaFuncSetAttribute(k_hash_small, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmallSmem)));
+            configured[ctx->device] = true;
+        }
+        VPMC_LAUNCH(k_hash_small, 1, kSmallThreads, small_sort_smem(N, long(rshx) * rshy), ctx->stream, rshx, rshy,
+                    rshx / Lx, rshy / Ly, sub, reinterpret_cast<const float2*>(pos), N, bits_for(uint64_t(N)), cell_num,
+                    cell_acc, vp_cell, vp_sort);
+        return collect_flags(ctx);
     }
-    VPMC_TRY(vpmc_fill_cells(ctx, rshx, rshy, Lx, Ly, N, sub, pos, cn, cell_acc, vp_cell));
-    if (N > 0) VPMC_TRY(sort_cells(ctx, N, ncell, vp_cell, vp_sort));
-    VPMC_CUDA(cudaMemsetAsync(cn, 0, sizeof(int) * size_t(ncell), ctx->stream));
-    VPMC_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (long(rshx) * rshy > (1L << 30)) return VPMC_ERR_CAPACITY;
+    const int ncell = rshx * rshy;
+    cudaStream_t st = ctx->stream;
+    if (N == 0) {
+        if (cell_num) VPMC_CUDA(cudaMemsetAsync(cell_num, 0, sizeof(int) * size_t(ncell), st));
+        VPMC_CUDA(cudaMemsetAsync(cell_acc, 0, sizeof(int) * size_t(ncell), st));
+    } else {
+        VPMC_LAUNCH(k_cells, blocks_for(N), kHashThreads, 0, st, rshx, rshy, rshx / Lx, rshy / Ly, sub,
+                    reinterpret_cast<const float2*>(pos), long(N), vp_cell);
+        VPMC_TRY(sort_cells(ctx, N, ncell, vp_cell, vp_sort, cell_acc, cell_num));
+    }
     return collect_flags(ctx);
 }
 

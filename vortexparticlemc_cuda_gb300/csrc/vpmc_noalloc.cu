@@ -35,7 +35,7 @@ namespace {
 constexpr long kMaxN = 1L << 18;        // particles per call (262,144)
 constexpr long kMaxCells = 1L << 20;    // rshx * rshy
 // radix ping-pong keys/values (4 x kMaxN x 4 B) + digit counts + scan scratch + slack
-constexpr size_t kScratchBytes = size_t(4) * kMaxN * 4 + size_t(256) * (kMaxN / 4096) * 4 + (size_t(1) << 16) +
+constexpr size_t kScratchBytes = size_t(4) * kMaxN * 4 + size_t(256) * (kMaxN / 2048) * 4 + (size_t(1) << 16) +
                                  (size_t(1) << 13);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];

@@ -3,11 +3,14 @@
 // Design: reduce-then-scan everywhere (no inter-block spin waits).  The radix
 // sort is the classic three-kernel pass (tile digit histograms, one scan of the
 // [digit][tile] count matrix, stable scatter); within a tile, ranks come from
-// __match_any_sync over 32 consecutive keys, warp-private digit counters and a
-// cross-warp prefix, so equal keys keep their input order.  Stability is what
-// makes the spatial hash bit-identical to the reference's sequential counting
-// sort (src/cpu/hash.cpp:36-48).
-#include "vpmc_internal.cuh"
+// ballots over 32 consecutive keys, warp-private digit counters and a
+// cross-warp prefix, so equal keys keep their input order.  A tile is put in
+// order in shared memory and written as runs of equal digits: pairs stored one
+// by one touch eight times the sectors.  (match.any for the ballots, and single
+// stores, took 41 us a pass at 2.1 M pairs, this form 15 us.)  Stability is
+// what makes the spatial hash bit-identical to the reference's sequential
+// counting sort (src/cpu/hash.cpp:36-48).
+#include "vpmc_blocksort.cuh"
 
 namespace vpmc {
 
@@ -17,11 +20,13 @@ constexpr int kScanThreads = 256;
 constexpr int kScanItems = 16;
 constexpr int kScanTile = kScanThreads * kScanItems;   // 4096
 
-constexpr int kSortThreads = 256;
+constexpr int kSortThreads = 512;
 constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kSortItems = 16;                          // per thread
-constexpr int kSortTile = kSortThreads * kSortItems;    // 4096
-constexpr int kWarpSpan = 32 * kSortItems;              // 512 consecutive keys per warp
+// keys a thread: 8 (tiles of 4096) from kSortBig keys on, below it 4, so that
+// more SMs take part
+constexpr long kSortBig = 1L << 20;
+int sort_items(long n) { return n >= kSortBig ? 8 : 4; }
+long sort_tiles(long n) { return (n + long(kSortThreads) * sort_items(n) - 1) / (long(kSortThreads) * sort_items(n)); }
 
 __device__ __forceinline__ uint32_t lanemask_lt() {
     uint32_t m;
@@ -99,72 +104,138 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* in,
     }
 }
 
+// Up to kSmallScan elements by one CTA of 1024 threads, in place of the three
+// launches of the tiled scan (each a few microseconds of latency).
+constexpr int kSmallScan = 16384;
+
+__global__ void __launch_bounds__(1024) k_scan_small(const uint32_t* in, uint32_t* out, int n, int write_total) {
+    __shared__ uint32_t wt[33];
+    constexpr int kPer = kSmallScan / 1024;
+    const int per = (n + 1023) / 1024, base = int(threadIdx.x) * per;
+    uint32_t v[kPer], s = 0;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        v[i] = i < per && base + i < n ? in[base + i] : 0u;
+        s += v[i];
+    }
+    uint32_t tot;
+    uint32_t run = block_exclusive(s, wt, &tot);
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        if (i < per && base + i < n) out[base + i] = run;
+        run += v[i];
+    }
+    if (write_total && threadIdx.x == 0) out[n] = tot;
+}
+
+template <int ITEMS>
 __global__ void __launch_bounds__(kSortThreads) k_radix_upsweep(const uint32_t* __restrict__ keys, long n,
                                                                 int shift, uint32_t mask,
                                                                 uint32_t* __restrict__ counts, int ntiles) {
     __shared__ uint32_t hist[256];
-    hist[threadIdx.x] = 0;
-    __syncthreads();
-    const long base = long(blockIdx.x) * kSortTile;
-#pragma unroll 4
-    for (int i = 0; i < kSortItems; ++i) {
+    if (threadIdx.x < 256) hist[threadIdx.x] = 0;
+    const long base = long(blockIdx.x) * (kSortThreads * ITEMS);
+    uint32_t k[ITEMS];
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
         const long e = base + long(i) * kSortThreads + threadIdx.x;
-        if (e < n) atomicAdd(&hist[(keys[e] >> shift) & mask], 1u);
+        k[i] = e < n ? keys[e] : 0u;
+    }
+    __syncthreads();
+    const uint32_t lt = lanemask_lt();
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        const bool valid = base + long(i) * kSortThreads + threadIdx.x < n;
+        const uint32_t d = (k[i] >> shift) & mask;
+        const uint32_t peers = digit_peers(d, valid, __popc(mask));
+        if (valid && (peers & lt) == 0u) atomicAdd(&hist[d], uint32_t(__popc(peers)));
     }
     __syncthreads();
     if (threadIdx.x <= mask) counts[long(threadIdx.x) * ntiles + blockIdx.x] = hist[threadIdx.x];
 }
 
+template <int ITEMS>
 __global__ void __launch_bounds__(kSortThreads) k_radix_downsweep(
     const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint32_t* __restrict__ kout,
     uint32_t* __restrict__ vout, long n, int shift, uint32_t mask, const uint32_t* __restrict__ offs,
     int ntiles) {
-    __shared__ uint32_t wh[kSortWarps][256];
+    constexpr int kTile = kSortThreads * ITEMS;
+    __shared__ __align__(4) uint16_t wh[kSortWarps][256];   // counts and places inside the tile (<= 4096)
+    __shared__ uint32_t sk[kTile], sv[kTile];
+    __shared__ uint32_t goff[256];   // global place of a digit's first key, less its place in the tile
+    __shared__ uint32_t wt[33];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < kSortWarps * 256; i += kSortThreads) (&wh[0][0])[i] = 0;
-    __syncthreads();
-    const long base = long(blockIdx.x) * kSortTile + long(w) * kWarpSpan;
-    const uint32_t lt = lanemask_lt();
-    uint32_t k[kSortItems], v[kSortItems], lr[kSortItems];
+    const long t0 = long(blockIdx.x) * kTile, base = t0 + long(w) * (32 * ITEMS);
+    uint32_t k[ITEMS], v[ITEMS], lr[ITEMS];
 #pragma unroll
-    for (int r = 0; r < kSortItems; ++r) {
+    for (int r = 0; r < ITEMS; ++r) {
         const long e = base + long(r) * 32 + lane;
-        const bool valid = e < n;
-        k[r] = valid ? kin[e] : 0u;
-        v[r] = valid ? (vin ? vin[e] : uint32_t(e)) : 0u;
+        k[r] = e < n ? kin[e] : 0u;
+        v[r] = e < n ? (vin ? vin[e] : uint32_t(e)) : 0u;
+    }
+    for (int i = threadIdx.x; i < kSortWarps * 128; i += kSortThreads) reinterpret_cast<uint32_t*>(&wh[0][0])[i] = 0;
+    __syncthreads();
+    const uint32_t lt = lanemask_lt();
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r) {
+        const bool valid = base + long(r) * 32 + lane < n;
         const uint32_t d = (k[r] >> shift) & mask;
-        const uint32_t act = __ballot_sync(0xffffffffu, valid);
-        uint32_t peers = 0, rank = 0, b = 0;
-        if (valid) {
-            peers = __match_any_sync(act, d);
-            rank = __popc(peers & lt);
-            b = wh[w][d];
-        }
+        const uint32_t peers = digit_peers(d, valid, __popc(mask));
+        const uint32_t rank = __popc(peers & lt);
+        const uint32_t b = valid ? wh[w][d] : 0u;
         __syncwarp();
-        if (valid && rank == 0) wh[w][d] = b + __popc(peers);
+        if (valid && rank == 0) wh[w][d] = uint16_t(b + __popc(peers));
         __syncwarp();
         lr[r] = b + rank;
     }
     __syncthreads();
+    // per digit: the warps' first places inside the tile, and the tile's place in the output
+    uint32_t c = 0;
+    if (threadIdx.x <= mask)
+#pragma unroll
+        for (int q = 0; q < kSortWarps; ++q) c += wh[q][threadIdx.x];
+    uint32_t tot;
+    uint32_t run = block_exclusive(c, wt, &tot);
     if (threadIdx.x <= mask) {
-        uint32_t run = offs[long(threadIdx.x) * ntiles + blockIdx.x];
+        goff[threadIdx.x] = offs[long(threadIdx.x) * ntiles + blockIdx.x] - run;
 #pragma unroll
         for (int q = 0; q < kSortWarps; ++q) {
-            const uint32_t c = wh[q][threadIdx.x];
-            wh[q][threadIdx.x] = run;
-            run += c;
+            const uint32_t t = wh[q][threadIdx.x];
+            wh[q][threadIdx.x] = uint16_t(run);
+            run += t;
         }
     }
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < kSortItems; ++r) {
-        const long e = base + long(r) * 32 + lane;
-        if (e < n) {
-            const uint32_t p = wh[w][(k[r] >> shift) & mask] + lr[r];
-            kout[p] = k[r];
-            vout[p] = v[r];
-        }
+    for (int r = 0; r < ITEMS; ++r) {
+        if (base + long(r) * 32 + lane >= n) continue;
+        const uint32_t p = wh[w][(k[r] >> shift) & mask] + lr[r];
+        sk[p] = k[r];
+        sv[p] = v[r];
     }
+    __syncthreads();
+    const int cnt = int(min(long(kTile), n - t0));
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r) {
+        const int i = r * kSortThreads + int(threadIdx.x);
+        if (i >= cnt) break;
+        const uint32_t key = sk[i];
+        const uint32_t p = goff[(key >> shift) & mask] + uint32_t(i);
+        kout[p] = key;
+        vout[p] = sv[i];
+    }
+}
+
+template <int ITEMS>
+int radix_pass(vpmc_context* ctx, const uint32_t* kc, const uint32_t* vc, uint32_t* ko, uint32_t* vo, long n, int shift,
+               uint32_t mask, const RadixScratch& rs) {
+    const int ntiles = int(sort_tiles(n));
+    VPMC_LAUNCH(k_radix_upsweep<ITEMS>, unsigned(ntiles), kSortThreads, 0, ctx->stream, kc, n, shift, mask, rs.counts,
+                ntiles);
+    VPMC_TRY(exclusive_scan(ctx, rs.counts, rs.counts, long(mask + 1) * ntiles, rs.scan_tmp, false));
+    VPMC_LAUNCH(k_radix_downsweep<ITEMS>, unsigned(ntiles), kSortThreads, 0, ctx->stream, kc, vc, ko, vo, n, shift, mask,
+                rs.counts, ntiles);
+    return VPMC_OK;
 }
 
 }  // namespace
@@ -181,11 +252,11 @@ int exclusive_scan(vpmc_context* ctx, const uint32_t* in, uint32_t* out, long n,
         if (write_total) VPMC_CUDA(cudaMemsetAsync(out, 0, sizeof(uint32_t), ctx->stream));
         return VPMC_OK;
     }
-    const long nb = (n + kScanTile - 1) / kScanTile;
-    if (nb == 1) {
-        VPMC_LAUNCH(k_scan_apply, 1, kScanThreads, 0, ctx->stream, in, out, n, nullptr, write_total ? 1 : 0);
+    if (n <= kSmallScan) {
+        VPMC_LAUNCH(k_scan_small, 1, 1024, 0, ctx->stream, in, out, int(n), write_total ? 1 : 0);
         return VPMC_OK;
     }
+    const long nb = (n + kScanTile - 1) / kScanTile;
     uint32_t* sums = tmp;
     uint32_t* offs = tmp + nb;
     VPMC_LAUNCH(k_scan_reduce, unsigned(nb), kScanThreads, 0, ctx->stream, in, n, sums);
@@ -195,10 +266,7 @@ int exclusive_scan(vpmc_context* ctx, const uint32_t* in, uint32_t* out, long n,
     return VPMC_OK;
 }
 
-size_t radix_counts_elems(long n) {
-    const long t = (n + kSortTile - 1) / kSortTile;
-    return size_t(256) * size_t(t < 1 ? 1 : t);
-}
+size_t radix_counts_elems(long n) { return size_t(256) * size_t(n < 1 ? 1 : sort_tiles(n)); }
 
 void carve_radix(Carver& c, long n, RadixScratch* rs) {
     const size_t m = size_t(n < 1 ? 1 : n);
@@ -218,7 +286,6 @@ int radix_sort(vpmc_context* ctx, const uint32_t* keys_in, const uint32_t* vals_
     const int passes = (key_bits + 7) / 8;
     const int dbits = (key_bits + passes - 1) / passes;
     const uint32_t mask = (dbits >= 32) ? 0xffffffffu : ((1u << dbits) - 1u);
-    const long ntiles = (n + kSortTile - 1) / kSortTile;
     const uint32_t* kc = keys_in;
     const uint32_t* vc = vals_in;
     *keys_out = rs.kbuf[0];
@@ -226,14 +293,10 @@ int radix_sort(vpmc_context* ctx, const uint32_t* keys_in, const uint32_t* vals_
     if (n <= 0) return VPMC_OK;
     for (int p = 0; p < passes; ++p) {
         const int shift = p * dbits;
-        VPMC_LAUNCH(k_radix_upsweep, unsigned(ntiles), kSortThreads, 0, ctx->stream, kc, n, shift, mask,
-                    rs.counts, int(ntiles));
-        const long ce = long(mask + 1) * ntiles;
-        VPMC_TRY(exclusive_scan(ctx, rs.counts, rs.counts, ce, rs.scan_tmp, false));
         uint32_t* ko = rs.kbuf[p & 1];
         uint32_t* vo = rs.vbuf[p & 1];
-        VPMC_LAUNCH(k_radix_downsweep, unsigned(ntiles), kSortThreads, 0, ctx->stream, kc, vc, ko, vo, n, shift,
-                    mask, rs.counts, int(ntiles));
+        if (sort_items(n) == 8) VPMC_TRY(radix_pass<8>(ctx, kc, vc, ko, vo, n, shift, mask, rs));
+        else VPMC_TRY(radix_pass<4>(ctx, kc, vc, ko, vo, n, shift, mask, rs));
         kc = ko;
         vc = vo;
     }
