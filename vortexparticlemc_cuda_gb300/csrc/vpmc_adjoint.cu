@@ -263,14 +263,12 @@ int adjoint_step(vpmc_sim* s, AdjBufs& A, const double* lam_in, double* lam_out,
     for (long t0 = 0; t0 < s->N; t0 += s->chunk_targets) {
         const long nt = std::min(s->chunk_targets, s->N - t0);
         const long ns = nt * 2 * Q;
-        VPMC_CUDA(cudaMemsetAsync(s->q.qcount, 0, sizeof(uint32_t) * size_t(s->g.nbins + 1), st));
+        VPMC_TRY(clear_counts(ctx, s->q));
         GenArgs ga{s->d_mc, s->n_inst, s->g.inst, s->pos, nullptr, nullptr, s->sub, s->cdf, s->guide, s->jit, s->d_step, t0,
-                   nt, s->N1, s->N2, 1, A.src, s->ys, s->q.qbin, s->q.qcount, s->q.tmp ? nullptr : s->q.qrank};
-        VPMC_LAUNCH(k_gen, blocks_for(ns), 256, 0, st, ga);
-        VPMC_TRY(scatter_ranked(ctx, s->g, s->q, s->ys, ns));
+                   nt, s->N1, s->N2, 1, A.src, s->ys, s->q.qbin, s->q.qcount, s->q.qsub, s->q.qrank, nullptr, A.fg, 3};
+        VPMC_TRY(launch_gen(st, ga));
         // f and grad f at every sample (FP64)
-        VPMC_TRY(make_items(ctx, s->g, s->q.qstart, s->it, query_chunk(4)));
-        VPMC_CUDA(cudaMemsetAsync(A.fg, 0, 3 * sizeof(double) * size_t(ns), st));
+        VPMC_TRY(place_samples(ctx, s->g, s->q, s->ys, ns, s->it, query_chunk(4)));
         EvalLaunch L;
         // field values and gradients at the samples: the FP32 path's adjoint sums
         // its pairs in FP32 (into FP64 run sums; the candidates are the particles
@@ -287,7 +285,7 @@ int adjoint_step(vpmc_sim* s, AdjBufs& A, const double* lam_in, double* lam_out,
         // transposed sums from the sample side: the same items, each sample
         // weighted by its dc/df, every in-support (sample, particle) pair adding
         // a_s W and a_s dW/dx_p to the particle's slot
-        VPMC_TRY(make_items(ctx, s->g, s->q.qstart, s->it, query_chunk(4)));
+        VPMC_CUDA(cudaMemsetAsync(s->it.counter, 0, sizeof(uint32_t), st));
         VPMC_CUDA(cudaMemsetAsync(A.dual_out, 0, 3 * sizeof(double) * size_t(s->N), st));
         EvalLaunch D;
         D.mode = unb ? (f32 ? EVAL_SCAT9_32 : EVAL_SCAT9_64) : (f32 ? EVAL_SCAT32 : EVAL_SCAT64);

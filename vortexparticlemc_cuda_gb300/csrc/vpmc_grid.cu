@@ -233,15 +233,29 @@ __global__ void k_scatter_points(const float2* __restrict__ pts, long M, const G
     }
 }
 
-// Scatter with precomputed in-bin ranks: slot = qstart[bin] + rank.
-__global__ void k_scatter_ranked(const float2* __restrict__ pts, long M, const GridInst* __restrict__ inst,
-                                 int n_inst, const uint32_t* __restrict__ qbin, const uint32_t* __restrict__ qrank,
-                                 const uint32_t* __restrict__ qstart, QRec* __restrict__ qrec) {
+// Direct placement of binned samples: the generator counted them per (bin,
+// sub-cell) and kept each one's rank there, so a sample's slot is its bin's start
+// plus the counts of the sub-cells before its own plus its rank.  One pass over
+// the samples instead of three, for as long as the records (16 bytes, stored in
+// no order) and the counters stay in L2; beyond, the staged passes below.
+__global__ void k_place_direct(const float2* __restrict__ pts, long M, const GridInst* __restrict__ inst, int n_inst,
+                               const uint32_t* __restrict__ qbin, const uint32_t* __restrict__ qrank,
+                               const uint32_t* __restrict__ qstart, const uint32_t* __restrict__ qsub,
+                               QRec* __restrict__ qrec) {
     for (long m = long(blockIdx.x) * blockDim.x + threadIdx.x; m < M; m += long(gridDim.x) * blockDim.x) {
         const uint32_t b = qbin[m];
         if (b == kNoBin) continue;
-        const GridInst& G = inst[inst_of_bin(inst, n_inst, b)];
+        const uint32_t rk = qrank[m], sub = rk & 15u;
         float2 p = pts[m];
+        const uint4* c4 = reinterpret_cast<const uint4*>(qsub + size_t(b) * 16);
+        uint32_t slot = qstart[b] + (rk >> 4);
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) {
+            if (4u * i >= sub) break;
+            const uint4 c = c4[i];
+            slot += c.x + (4u * i + 1u < sub ? c.y : 0u) + (4u * i + 2u < sub ? c.z : 0u) + (4u * i + 3u < sub ? c.w : 0u);
+        }
+        const GridInst& G = inst[n_inst == 1 ? 0 : inst_of_bin(inst, n_inst, b)];
         uint32_t fl = (2u) | (2u << 3);
         if (G.periodic) {
             const float kx = floorf(p.x / G.Lx), ky = floorf(p.y / G.Ly);
@@ -250,7 +264,20 @@ __global__ void k_scatter_ranked(const float2* __restrict__ pts, long M, const G
             const int ikx = min(max(int(kx), -2), 2), iky = min(max(int(ky), -2), 2);
             fl = uint32_t(ikx + 2) | (uint32_t(iky + 2) << 3);
         }
-        qrec[qstart[b] + qrank[m]] = QRec{p.x, p.y, uint32_t(m), fl};
+        qrec[slot] = QRec{p.x, p.y, uint32_t(m), fl};
+    }
+}
+
+// Samples per bin from the counts per (bin, sub-cell).
+__global__ void k_bin_totals(const uint32_t* __restrict__ qsub, long nbins, uint32_t* __restrict__ qcount) {
+    for (long b = long(blockIdx.x) * blockDim.x + threadIdx.x; b < nbins; b += long(gridDim.x) * blockDim.x) {
+        uint32_t t = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint4 c = reinterpret_cast<const uint4*>(qsub)[4 * b + i];
+            t += c.x + c.y + c.z + c.w;
+        }
+        qcount[b] = t;
     }
 }
 
@@ -388,17 +415,6 @@ __device__ __forceinline__ QRec make_qrec(uint4 r, const GridInst* __restrict__ 
         fl = uint32_t(ikx + 2) | (uint32_t(iky + 2) << 3);
     }
     return QRec{p.x, p.y, r.z, fl};
-}
-
-// Sub-cell of a query (wrapped point p in the cell of its bin): 4 x 4
-// sub-cells in serpentine order (rows of sub-cells, alternate rows reversed),
-// so that any run of consecutive keys covers a compact part of the cell.
-// c = {cx, cy, gx / Lx, gy / Ly} of the bin's cell.
-constexpr int kSubCells = 16;
-__device__ __forceinline__ uint32_t subcell_key(float px, float py, float4 c) {
-    const int ix = min(max(int((px * c.z - c.x) * 4.f), 0), 3);
-    const int iy = min(max(int((py * c.w - c.y) * 4.f), 0), 3);
-    return uint32_t(iy * 4 + ((iy & 1) ? 3 - ix : ix));
 }
 
 // Pass 2: the same per tile of the super-bin-grouped records, by window
@@ -621,24 +637,20 @@ __global__ void k_items_fill(const uint32_t* __restrict__ qstart, long nbins, in
     }
 }
 
-// Few bins: counts, their scan and the items in one launch of one CTA.
-constexpr long kSmallItemBins = 16384;
+// Few bins and items: the items (and with qsub first the bins' totals and starts) in
+// one launch of one CTA.  (8,192 bins of 3,000 samples: 428 us in one CTA, 27 us in
+// the general three launches.)
+bool items_in_one(long nbins, long queries) { return nbins <= 4096 && queries <= (1L << 19); }
 
-__global__ void __launch_bounds__(1024) k_items_small(const uint32_t* __restrict__ qstart, int nbins, int chunk,
-                                                      const GridInst* __restrict__ inst, int n_inst,
-                                                      Item* __restrict__ items, uint32_t* __restrict__ n_items,
-                                                      uint32_t* __restrict__ counter, long max_items) {
-    __shared__ uint32_t s_warp[32];
+__device__ __forceinline__ uint32_t scan_1024(uint32_t v, uint32_t* s_warp, uint32_t* total) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int per = (nbins + 1023) / 1024, b0 = min(nbins, int(threadIdx.x) * per), b1 = min(nbins, b0 + per);
-    uint32_t sum = 0u;
-    for (int b = b0; b < b1; ++b) sum += (qstart[b + 1] - qstart[b] + uint32_t(chunk) - 1u) / uint32_t(chunk);
-    uint32_t inc = sum;
+    uint32_t inc = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
         if (lane >= o) inc += t;
     }
+    __syncthreads();   // s_warp may still be read from the previous scan
     if (lane == 31) s_warp[w] = inc;
     __syncthreads();
     if (w == 0) {
@@ -651,16 +663,49 @@ __global__ void __launch_bounds__(1024) k_items_small(const uint32_t* __restrict
         s_warp[lane] = t;
     }
     __syncthreads();
-    uint32_t it = inc - sum + (w > 0 ? s_warp[w - 1] : 0u);
+    *total = s_warp[31];
+    return inc - v + (w > 0 ? s_warp[w - 1] : 0u);
+}
+
+__global__ void __launch_bounds__(1024) k_items_small(const uint32_t* __restrict__ qsub, uint32_t* qstart, int nbins,
+                                                      int chunk, const GridInst* __restrict__ inst, int n_inst,
+                                                      Item* __restrict__ items, uint32_t* __restrict__ n_items,
+                                                      uint32_t* __restrict__ counter, long max_items) {
+    __shared__ uint32_t s_warp[32];
+    const int per = (nbins + 1023) / 1024, b0 = min(nbins, int(threadIdx.x) * per), b1 = min(nbins, b0 + per);
+    uint32_t total = 0u;
+    if (qsub) {
+        const uint4* c4 = reinterpret_cast<const uint4*>(qsub);
+        auto bin_total = [&](int b) {
+            uint32_t t = 0u;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint4 c = c4[4 * b + i];
+                t += c.x + c.y + c.z + c.w;
+            }
+            return t;
+        };
+        uint32_t sum = 0u;
+        for (int b = b0; b < b1; ++b) sum += bin_total(b);
+        uint32_t run = scan_1024(sum, s_warp, &total);
+        for (int b = b0; b < b1; ++b) {
+            qstart[b] = run;
+            run += bin_total(b);
+        }
+        if (threadIdx.x == 0) qstart[nbins] = total;
+        __syncthreads();   // the starts are read back by the threads of this CTA
+    }
+    uint32_t sum = 0u;
+    for (int b = b0; b < b1; ++b) sum += (qstart[b + 1] - qstart[b] + uint32_t(chunk) - 1u) / uint32_t(chunk);
+    uint32_t it = scan_1024(sum, s_warp, &total);
     for (int b = b0; b < b1; ++b) {
         const uint32_t q0 = qstart[b], c = qstart[b + 1] - q0;
-        const uint32_t ib = c ? uint32_t(inst_of_bin(inst, n_inst, uint32_t(b))) : 0u;
+        const uint32_t ib = c && n_inst > 1 ? uint32_t(inst_of_bin(inst, n_inst, uint32_t(b))) : 0u;
         for (uint32_t o = 0; o < c; o += uint32_t(chunk), ++it)
             if (it < max_items) items[it] = Item{uint32_t(b), q0 + o, min(uint32_t(chunk), c - o), ib};
     }
     if (threadIdx.x == 0) {
-        const uint32_t t = s_warp[31];
-        *n_items = t < max_items ? t : uint32_t(max_items);
+        *n_items = total < max_items ? total : uint32_t(max_items);
         *counter = 0;
     }
 }
@@ -1666,11 +1711,11 @@ void carve_items(Carver& c, long nbins, long max_queries, ItemBufs* it) {
     it->scan_tmp = c.take<uint32_t>(scan_tmp_elems(nbins + 1) + 1);
 }
 
-int make_items(vpmc_context* ctx, const GridBufs& g, const uint32_t* qstart, ItemBufs& it, int chunk) {
+int make_items(vpmc_context* ctx, const GridBufs& g, const uint32_t* qstart, ItemBufs& it, int chunk, long queries) {
     cudaStream_t st = ctx->stream;
-    if (g.nbins <= kSmallItemBins) {
-        VPMC_LAUNCH(k_items_small, 1, 1024, 0, st, qstart, int(g.nbins), chunk, g.inst, g.n_inst, it.items, it.n_items,
-                    it.counter, it.max_items);
+    if (items_in_one(g.nbins, queries)) {
+        VPMC_LAUNCH(k_items_small, 1, 1024, 0, st, static_cast<const uint32_t*>(nullptr), const_cast<uint32_t*>(qstart),
+                    int(g.nbins), chunk, g.inst, g.n_inst, it.items, it.n_items, it.counter, it.max_items);
         return VPMC_OK;
     }
     VPMC_LAUNCH(k_items_count, blocks_for(g.nbins), 256, 0, st, qstart, g.nbins, chunk, it.per_bin);
@@ -1680,18 +1725,34 @@ int make_items(vpmc_context* ctx, const GridBufs& g, const uint32_t* qstart, Ite
     return VPMC_OK;
 }
 
-void carve_queries(Carver& c, long nbins, long max_points, QueryBufs* q, bool two_pass) {
+// Samples are placed directly up to this many a chunk (the records in L2), in
+// three streaming passes beyond: a step of 0.26 M samples takes 105 us direct and
+// 112 us staged, of 2.1 M 381 and 413 us, of 4.2 M 675 and 656 us.
+constexpr long kDirectSamples = 1L << 21;
+// Up to this many bins (32 MB of counters) the generator counts per (bin, sub-cell).
+constexpr long kSubBins = 1L << 19;
+
+void carve_queries(Carver& c, long nbins, long max_points, QueryBufs* q, bool samples) {
     const size_t m = size_t(max_points < 1 ? 1 : max_points);
+    const bool sub = samples && nbins <= kSubBins, direct = sub && max_points <= kDirectSamples;
+    const bool staged = samples && !direct;
     q->qbin = c.take<uint32_t>(m);
-    q->qcount = c.take<uint32_t>(size_t(nbins + 1));
+    // the counters that are zeroed for every pass lie together (clear_counts)
+    const size_t n_sub = sub ? size_t(nbins) * kSubCells : 0, n_fill = staged ? size_t(nbins + 1) + kTargetSuper + 1 : 0;
+    const size_t n_count = size_t(nbins + 1);
+    uint32_t* counts = c.take<uint32_t>(n_sub + n_fill + n_count);
+    q->qsub = sub ? counts : nullptr;
+    q->super_fill = staged ? counts + n_sub : nullptr;
+    q->win_fill = staged ? counts + n_sub + kTargetSuper + 1 : nullptr;
+    q->qcount = counts + n_sub + n_fill;
+    q->clear = counts;
+    q->n_clear = n_sub + n_fill + (sub ? 0 : n_count);
     q->qstart = c.take<uint32_t>(size_t(nbins + 1));
-    q->qfill = c.take<uint32_t>(size_t(nbins + 1));
-    q->qrank = two_pass ? nullptr : c.take<uint32_t>(m);   // ranks are only needed without the staged placement
+    q->qfill = samples ? nullptr : c.take<uint32_t>(size_t(nbins + 1));
+    q->qrank = direct ? c.take<uint32_t>(m) : nullptr;
     q->qrec = c.take<QRec>(m);
-    q->tmp = two_pass ? c.take<uint4>(m) : nullptr;
-    q->tmp2 = two_pass ? c.take<uint4>(m) : nullptr;
-    q->super_fill = two_pass ? c.take<uint32_t>(kTargetSuper + 1) : nullptr;
-    q->win_fill = two_pass ? c.take<uint32_t>(size_t(nbins + 1)) : nullptr;
+    q->tmp = staged ? c.take<uint4>(m) : nullptr;
+    q->tmp2 = staged ? c.take<uint4>(m) : nullptr;
     q->scan_tmp = c.take<uint32_t>(scan_tmp_elems(nbins + 1) + 1);
 }
 
@@ -1705,43 +1766,51 @@ int scatter_points(vpmc_context* ctx, const GridBufs& g, QueryBufs& q, const flo
     return VPMC_OK;
 }
 
-int scatter_ranked(vpmc_context* ctx, const GridBufs& g, QueryBufs& q, const float2* pts, long M) {
-    VPMC_TRY(exclusive_scan(ctx, q.qcount, q.qstart, g.nbins, q.scan_tmp, true));
+int clear_counts(vpmc_context* ctx, QueryBufs& q) {
+    VPMC_CUDA(cudaMemsetAsync(q.clear, 0, sizeof(uint32_t) * q.n_clear, ctx->stream));
+    return VPMC_OK;
+}
+
+int place_samples(vpmc_context* ctx, const GridBufs& g, QueryBufs& q, const float2* pts, long M, ItemBufs& it,
+                  int chunk) {
     cudaStream_t st = ctx->stream;
-    if (q.tmp) {
-        int shift = 0;
-        while (((g.nbins - 1) >> shift) + 1 > kTargetSuper) ++shift;
-        const int nsuper = int(((g.nbins - 1) >> shift) + 1);
-        // windows of 2^W bins holding about half the assembly capacity on average
-        const double per_bin = double(M) / double(std::max<long>(g.nbins, 1));
-        int wshift = 0;
-        while ((1 << (wshift + 1)) <= kWinBinsMax && per_bin * double(2L << wshift) <= 0.5 * kWinCap) ++wshift;
-        const long nwin = ((g.nbins - 1) >> wshift) + 1;
-        VPMC_CUDA(cudaMemsetAsync(q.super_fill, 0, sizeof(uint32_t) * size_t(nsuper), st));
-        VPMC_CUDA(cudaMemsetAsync(q.win_fill, 0, sizeof(uint32_t) * size_t(nwin), st));
-        static bool configured[64] = {};
-        const size_t tile_smem = sizeof(uint4) * size_t(kTileRecs), win_smem = sizeof(QRec) * size_t(kWinCap);
-        if (ctx->device < 64 && !configured[ctx->device]) {
-            VPMC_CUDA(cudaFuncSetAttribute(k_scatter_coarse, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           int(tile_smem)));
-            VPMC_CUDA(cudaFuncSetAttribute(k_scatter_window, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           int(tile_smem)));
-            VPMC_CUDA(cudaFuncSetAttribute(k_scatter_assemble, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           int(win_smem)));
-            configured[ctx->device] = true;
-        }
-        const long tiles = (M + kTileRecs - 1) / kTileRecs;
-        const int tgrid = int(std::max<long>(1, std::min<long>(tiles, 2L * ctx->sm_count)));
-        VPMC_LAUNCH(k_scatter_coarse, tgrid, kPlaceThreads, tile_smem, st, pts, M, q.qbin, q.qstart, shift, nsuper,
-                    q.super_fill, q.tmp);
-        VPMC_LAUNCH(k_scatter_window, tgrid, kPlaceThreads, tile_smem, st, q.tmp, q.qstart + g.nbins, M, wshift,
-                    q.qstart, q.win_fill, q.tmp2);
-        VPMC_LAUNCH(k_scatter_assemble, int(std::max<long>(1, std::min<long>(nwin, 2L * ctx->sm_count))), kAsmThreads, win_smem,
-                    st, q.tmp2, g.nbins, wshift, q.qstart, g.inst, g.n_inst, q.qrec);
+    if (q.qrank && items_in_one(g.nbins, M)) {
+        VPMC_LAUNCH(k_items_small, 1, 1024, 0, st, q.qsub, q.qstart, int(g.nbins), chunk, g.inst, g.n_inst, it.items,
+                    it.n_items, it.counter, it.max_items);
+    } else {
+        if (q.qsub) VPMC_LAUNCH(k_bin_totals, blocks_for(g.nbins), 256, 0, st, q.qsub, g.nbins, q.qcount);
+        VPMC_TRY(exclusive_scan(ctx, q.qcount, q.qstart, g.nbins, q.scan_tmp, true));
+        VPMC_TRY(make_items(ctx, g, q.qstart, it, chunk, M));
+    }
+    if (q.qrank) {
+        VPMC_LAUNCH(k_place_direct, blocks_for(M), 256, 0, st, pts, M, g.inst, g.n_inst, q.qbin, q.qrank, q.qstart, q.qsub,
+                    q.qrec);
         return VPMC_OK;
     }
-    VPMC_LAUNCH(k_scatter_ranked, blocks_for(M), 256, 0, st, pts, M, g.inst, g.n_inst, q.qbin, q.qrank, q.qstart,
-                q.qrec);
+    int shift = 0;
+    while (((g.nbins - 1) >> shift) + 1 > kTargetSuper) ++shift;
+    const int nsuper = int(((g.nbins - 1) >> shift) + 1);
+    // windows of 2^W bins holding about half the assembly capacity on average
+    const double per_bin = double(M) / double(std::max<long>(g.nbins, 1));
+    int wshift = 0;
+    while ((1 << (wshift + 1)) <= kWinBinsMax && per_bin * double(2L << wshift) <= 0.5 * kWinCap) ++wshift;
+    const long nwin = ((g.nbins - 1) >> wshift) + 1;
+    static bool configured[64] = {};
+    const size_t tile_smem = sizeof(uint4) * size_t(kTileRecs), win_smem = sizeof(QRec) * size_t(kWinCap);
+    if (ctx->device < 64 && !configured[ctx->device]) {
+        VPMC_CUDA(cudaFuncSetAttribute(k_scatter_coarse, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tile_smem)));
+        VPMC_CUDA(cudaFuncSetAttribute(k_scatter_window, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tile_smem)));
+        VPMC_CUDA(cudaFuncSetAttribute(k_scatter_assemble, cudaFuncAttributeMaxDynamicSharedMemorySize, int(win_smem)));
+        configured[ctx->device] = true;
+    }
+    const long tiles = (M + kTileRecs - 1) / kTileRecs;
+    const int tgrid = int(std::max<long>(1, std::min<long>(tiles, 2L * ctx->sm_count)));
+    VPMC_LAUNCH(k_scatter_coarse, tgrid, kPlaceThreads, tile_smem, st, pts, M, q.qbin, q.qstart, shift, nsuper,
+                q.super_fill, q.tmp);
+    VPMC_LAUNCH(k_scatter_window, tgrid, kPlaceThreads, tile_smem, st, q.tmp, q.qstart + g.nbins, M, wshift, q.qstart,
+                q.win_fill, q.tmp2);
+    VPMC_LAUNCH(k_scatter_assemble, int(std::max<long>(1, std::min<long>(nwin, 2L * ctx->sm_count))), kAsmThreads, win_smem,
+                st, q.tmp2, g.nbins, wshift, q.qstart, g.inst, g.n_inst, q.qrec);
     return VPMC_OK;
 }
 

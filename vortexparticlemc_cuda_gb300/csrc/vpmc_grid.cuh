@@ -257,7 +257,7 @@ struct ItemBufs {
 };
 void carve_items(Carver& c, long nbins, long max_queries, ItemBufs* it);
 // chunk = queries per item = 256 * queries-per-thread of the eval launch.
-int make_items(vpmc_context* ctx, const GridBufs& g, const uint32_t* qstart, ItemBufs& it, int chunk);
+int make_items(vpmc_context* ctx, const GridBufs& g, const uint32_t* qstart, ItemBufs& it, int chunk, long queries);
 int query_chunk(int qpt);
 
 // Query binning for points/samples: bin ids (kNoBin = skip) -> counts -> scan
@@ -267,15 +267,19 @@ struct QueryBufs {
     uint32_t* qcount = nullptr;  // nbins + 1
     uint32_t* qstart = nullptr;  // nbins + 1
     uint32_t* qfill = nullptr;   // nbins
-    uint32_t* qrank = nullptr;   // per point: rank inside its bin (only without the staged placement)
+    uint32_t* qrank = nullptr;   // direct placement: rank in (bin, sub-cell) << 4 | sub-cell, per point
+    uint32_t* qsub = nullptr;    // points per (bin, sub-cell)
     QRec* qrec = nullptr;        // max points
-    uint4* tmp = nullptr;        // max points (staged placement of ranked points: super-bins)
+    uint4* tmp = nullptr;        // max points (staged placement: super-bins)
     uint4* tmp2 = nullptr;       // max points (staged placement: slot windows)
     uint32_t* super_fill = nullptr;
     uint32_t* win_fill = nullptr;
+    uint32_t* clear = nullptr;   // the words to zero before the samples are counted
+    size_t n_clear = 0;
     uint32_t* scan_tmp = nullptr;
 };
-void carve_queries(Carver& c, long nbins, long max_points, QueryBufs* q, bool two_pass = false);
+// samples: binned samples of the MIS step (place_samples) instead of points.
+void carve_queries(Carver& c, long nbins, long max_points, QueryBufs* q, bool samples = false);
 // Bin arbitrary points (one instance `inst_of` lookup per point by index range
 // `point_inst` == nullptr -> instance 0).  set = candidate set to query.
 int bin_points(vpmc_context* ctx, const GridBufs& g, QueryBufs& q, const float2* pts, long M, int set,
@@ -283,11 +287,27 @@ int bin_points(vpmc_context* ctx, const GridBufs& g, QueryBufs& q, const float2*
 // Scatter points whose bins are already in q.qbin (counts in q.qcount).
 int scatter_points(vpmc_context* ctx, const GridBufs& g, QueryBufs& q, const float2* pts, long M,
                    int field9);
-// Same for points whose bins are counted in q.qcount: with q.tmp carved
-// through super-bins and bin windows in three streaming passes (slots inside
-// a bin assigned in shared memory); otherwise each point's rank inside its
-// bin must be in q.qrank.
-int scatter_ranked(vpmc_context* ctx, const GridBufs& g, QueryBufs& q, const float2* pts, long M);
+// The MIS samples: zero the counters before the generator bins them, then place
+// the samples into query records by bin and make the work items (`chunk` queries
+// each).  The generator writes q.qbin and counts per bin (q.qcount) or, where
+// q.qsub is carved, per (bin, sub-cell), there with each sample's rank where
+// q.qrank is carved (direct placement).
+int clear_counts(vpmc_context* ctx, QueryBufs& q);
+int place_samples(vpmc_context* ctx, const GridBufs& g, QueryBufs& q, const float2* pts, long M, ItemBufs& it,
+                  int chunk);
+
+#ifdef __CUDACC__
+// Sub-cell of a query (wrapped point p in the cell of its bin): 4 x 4
+// sub-cells in serpentine order (rows of sub-cells, alternate rows reversed),
+// so that any run of consecutive keys covers a compact part of the cell.
+// c = {cx, cy, gx / Lx, gy / Ly} of the bin's cell.
+constexpr int kSubCells = 16;
+__device__ __forceinline__ uint32_t subcell_key(float px, float py, float4 c) {
+    const int ix = min(max(int((px * c.z - c.x) * 4.f), 0), 3);
+    const int iy = min(max(int((py * c.w - c.y) * 4.f), 0), 3);
+    return uint32_t(iy * 4 + ((iy & 1) ? 3 - ix : ix));
+}
+#endif
 
 // sigma_max over F[0..n) (+inf if some F is non-finite or has det <= 0);
 // d_words: 2 device words of scratch.  Synchronises the stream.

@@ -53,7 +53,7 @@ int vpmc_query_vorticity(vpmc_context* ctx, int N, const float* pos, const float
     VPMC_TRY(grid_build(ctx, w.g, reinterpret_cast<const float2*>(pos), omega, set_mode,
                         reinterpret_cast<const float4*>(F)));
     VPMC_TRY(bin_points(ctx, w.g, w.q, reinterpret_cast<const float2*>(pts), M, 0, 0));
-    VPMC_TRY(make_items(ctx, w.g, w.q.qstart, w.it, query_chunk(4)));
+    VPMC_TRY(make_items(ctx, w.g, w.q.qstart, w.it, query_chunk(4), M));
     EvalLaunch L;
     if (F) L.mode = exclude_center ? EVAL_FIELD_F_EXC : EVAL_FIELD_F;
     else L.mode = exclude_center ? EVAL_FIELD_EXC : EVAL_FIELD;
@@ -78,7 +78,7 @@ int vpmc_query_vorticity_f64(vpmc_context* ctx, int N, const float* pos, const f
                                    : (sign < 0 ? SET_NEG_ONLY : (use_signed ? SET_ONE_SIGNED : SET_ONE_ABS));
     VPMC_TRY(grid_build(ctx, w.g, reinterpret_cast<const float2*>(pos), omega, set_mode));
     VPMC_TRY(bin_points(ctx, w.g, w.q, reinterpret_cast<const float2*>(pts), M, 0, 0));
-    VPMC_TRY(make_items(ctx, w.g, w.q.qstart, w.it, query_chunk(4)));
+    VPMC_TRY(make_items(ctx, w.g, w.q.qstart, w.it, query_chunk(4), M));
     EvalLaunch L;
     L.mode = EVAL_FIELD64;
     L.out_f64 = out;

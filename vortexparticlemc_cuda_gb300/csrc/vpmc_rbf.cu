@@ -557,7 +557,7 @@ int begin(vpmc_context* ctx, Solver& s, int N, const float* pos, const float* b,
     if (!s.kept) {
         VPMC_LAUNCH(k_self_queries, work_blocks(N), 256, 0, st, w.g.cand, w.g.cstart, long(N), uint32_t(w.g.nbins),
                     w.self);
-        VPMC_TRY(make_items(ctx, w.g, w.g.cstart, w.it, query_chunk(4)));
+        VPMC_TRY(make_items(ctx, w.g, w.g.cstart, w.it, query_chunk(4), N));
     }
     double *bs = w.vec[0], *x = w.vec[1];
     if (b64) VPMC_LAUNCH(k_gather_to_sorted<double>, work_blocks(N), 256, 0, st, b64, w.g.perm, long(N), bs);
@@ -723,7 +723,7 @@ int vpmc_rbf_matvec(vpmc_context* ctx, int N, const float* pos, const float* x, 
     VPMC_TRY(grid_build(ctx, w.g, reinterpret_cast<const float2*>(pos), nullptr, SET_ONE_SIGNED));
     VPMC_LAUNCH(k_self_queries, work_blocks(N), 256, 0, st, w.g.cand, w.g.cstart, long(N), uint32_t(w.g.nbins),
                 w.self);
-    VPMC_TRY(make_items(ctx, w.g, w.g.cstart, w.it, query_chunk(4)));
+    VPMC_TRY(make_items(ctx, w.g, w.g.cstart, w.it, query_chunk(4), N));
     VPMC_LAUNCH(k_gather_to_sorted<float>, work_blocks(N), 256, 0, st, x, w.g.perm, long(N), w.vec[0]);
     // FP64 pairs use W with its sigma; the FP32 form evaluates W / (2 sigma)
     VPMC_TRY(grid_set_weights_sorted(ctx, w.g, w.vec[0], precise ? 1.0 : double(w.plan.two_sigma)));

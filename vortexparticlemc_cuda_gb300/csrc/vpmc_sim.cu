@@ -161,6 +161,11 @@ __device__ __forceinline__ float2 aux_point(float2 x, int a, float dx) {
     }
 }
 
+// COUNT: 0 = per bin, 1 = per (bin, sub-cell), 2 = per (bin, sub-cell) with ranks.
+// A few thousand bins make the counts collide (thousands of samples a bin: the
+// atomics of one address go one by one): 8.4 M samples in 8,192 bins took 219 us
+// counted per bin, 114 us per (bin, sub-cell).
+template <int COUNT>
 __global__ void __launch_bounds__(256) k_gen(GenArgs a) {
     const int Q = a.N1 + a.naux * a.N2;
     const uint32_t Q2 = uint32_t(2 * Q);
@@ -265,14 +270,33 @@ __global__ void __launch_bounds__(256) k_gen(GenArgs a) {
                 const int cx = min(max(floor_int(px * G.inv_sx), 0), G.gx - 1);
                 const int cy = min(max(floor_int(py * G.inv_sy), 0), G.gy - 1);
                 b = uint32_t(G.bin_base) + uint32_t(s) * uint32_t(G.gx * G.gy) + uint32_t(cx * G.gy + cy);
-                if (a.qrank) a.qrank[sid] = atomicAdd(&a.qcount[b], 1u);   // rank in its bin
-                else atomicAdd(&a.qcount[b], 1u);                            // count only
+                if constexpr (COUNT == 0) {
+                    atomicAdd(&a.qcount[b], 1u);
+                } else {
+                    const uint32_t sub = subcell_key(px, py, make_float4(float(cx), float(cy), G.inv_sx, G.inv_sy));
+                    uint32_t* c = &a.qsub[size_t(b) * kSubCells + sub];
+                    if constexpr (COUNT == 1) atomicAdd(c, 1u);
+                    else a.qrank[sid] = (atomicAdd(c, 1u) << 4) | sub;
+                }
             }
+        }
+        if (b == kNoBin) {   // no query will write its value
+            if (a.f32) a.f32[sid] = 0.f;
+            if (a.f64)
+                for (int v = 0; v < a.nf64; ++v) a.f64[size_t(sid) * a.nf64 + v] = 0.0;
         }
         a.ys[sid] = y;
         a.qbin[sid] = b;
         if (a.src) a.src[sid] = src;
     }
+}
+
+int launch_gen(cudaStream_t st, const GenArgs& a) {
+    const int grid = blocks_for(a.nt * 2 * (a.N1 + long(a.naux) * a.N2));
+    if (!a.qsub) VPMC_LAUNCH(k_gen<0>, grid, 256, 0, st, a);
+    else if (!a.qrank) VPMC_LAUNCH(k_gen<1>, grid, 256, 0, st, a);
+    else VPMC_LAUNCH(k_gen<2>, grid, 256, 0, st, a);
+    return VPMC_OK;
 }
 
 }  // namespace sim
@@ -291,7 +315,8 @@ struct AccArgs {
     int N1, N2;
     int advect;
     float2* vel;
-    float2* pos_out;
+    float2* pos_out;              // may be pos: a target reads only its own
+    unsigned long long* step;     // stepped by this launch, or nullptr
 };
 
 // mis_contrib_dev (src/cuda/monte_carlo_bs.cu:35-51) for the reference law;
@@ -334,6 +359,7 @@ __device__ __forceinline__ float2 mis_term(int law, float2 x, float2 y, float f,
 constexpr int kAccLanes = 8;
 
 __global__ void __launch_bounds__(256) k_accum(AccArgs a) {
+    if (a.step && blockIdx.x == 0 && threadIdx.x == 0) *a.step += 1ull;
     const int lane = threadIdx.x & 31, sub = lane & (kAccLanes - 1), grp = lane / kAccLanes;
     constexpr int kPerWarp = 32 / kAccLanes;
     const long warp = (long(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
@@ -425,9 +451,11 @@ struct Acc5Args {
     float4* F_out;
     unsigned* sig;         // [0] = max sigma_max(F_out) (float bits), [1] = targets with sigma_max > cap
     float cap;
+    unsigned long long* step;
 };
 
 __global__ void __launch_bounds__(256) k_accum5(Acc5Args a) {
+    if (a.step && blockIdx.x == 0 && threadIdx.x == 0) *a.step += 1ull;
     const int lane = threadIdx.x & 31;
     const long warp = (long(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const long nwarps = (long(gridDim.x) * blockDim.x) >> 5;
@@ -566,9 +594,11 @@ struct AccArgs64 {
     int advect;
     float2* vel;
     float2* pos_out;
+    unsigned long long* step;
 };
 
 __global__ void __launch_bounds__(256) k_accum64(AccArgs64 a) {
+    if (a.step && blockIdx.x == 0 && threadIdx.x == 0) *a.step += 1ull;
     const int lane = threadIdx.x & 31;
     const long warp = (long(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const long nwarps = (long(gridDim.x) * blockDim.x) >> 5;
@@ -623,8 +653,6 @@ __global__ void __launch_bounds__(256) k_accum64(AccArgs64 a) {
         }
     }
 }
-
-__global__ void k_inc_step(unsigned long long* s) { *s += 1ull; }
 
 // sum over targets of |u|^2 in FP64 (one atomic per warp)
 __global__ void k_vel_sumsq(const float2* __restrict__ v, long n, double* __restrict__ out) {
@@ -825,8 +853,7 @@ void mark_samples(vpmc_sim* s) {
     s->ys_nt = s->t_end - s->ys_t0;
 }
 
-// Issue one MIS pass over all targets (advect: positions -> pos_next, then
-// copied back, step counter incremented).  No host synchronisation inside, so
+// Issue one MIS pass over all targets (advect: positions and step counter move on).  No host synchronisation inside, so
 // it can be captured.  Returns launches issued.
 int issue_pass(vpmc_sim* s, bool advect, bool timed, int* nlaunch) {
     vpmc_context* ctx = s->ctx;
@@ -837,6 +864,12 @@ int issue_pass(vpmc_sim* s, bool advect, bool timed, int* nlaunch) {
     VPMC_CUDA(cudaStreamIsCapturing(st, &cap));
     const unsigned ev_flags = cap == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : cudaEventRecordDefault;
     const bool def = s->deform != 0;
+    // the positions (and F) advance in place unless a later chunk's generator reads
+    // other targets' (the plain method's reads the copy in subset order); the last
+    // chunk's sums step the counter
+    const bool in_place = !def || s->t_end - s->t_begin <= s->chunk_targets;
+    float2* const pos_out = in_place ? s->pos : s->pos_next;
+    float4* const F_out = in_place ? s->F : s->F_next;
     VPMC_TRY(grid_build(ctx, s->g, s->pos, s->omega, SET_SIGN_SPLIT, def ? s->F : nullptr));
     if (def && advect) VPMC_CUDA(cudaMemsetAsync(s->d_sig, 0, 2 * sizeof(unsigned), st));
     const long Q = samples_per(s);
@@ -845,17 +878,14 @@ int issue_pass(vpmc_sim* s, bool advect, bool timed, int* nlaunch) {
     for (long t0 = s->t_begin; t0 < s->t_end; t0 += s->chunk_targets) {
         const long nt = std::min(s->chunk_targets, s->t_end - t0);
         const long ns = nt * 2 * Q;
-        VPMC_CUDA(cudaMemsetAsync(s->q.qcount, 0, sizeof(uint32_t) * size_t(s->g.nbins + 1), st));
+        const bool f64 = s->precision == 64;
+        VPMC_TRY(clear_counts(ctx, s->q));
         GenArgs ga{s->d_mc, s->n_inst, s->g.inst, s->pos, def ? s->F : nullptr, def ? nullptr : s->pos_sub, s->sub,
                    s->cdf, s->guide, s->jit,
                    s->d_step, t0, nt, s->N1, s->N2, def ? 5 : 1, nullptr, s->ys, s->q.qbin, s->q.qcount,
-                   s->q.tmp ? nullptr : s->q.qrank};
-        VPMC_LAUNCH(k_gen, blocks_for(ns), 256, 0, st, ga);
-        VPMC_TRY(scatter_ranked(ctx, s->g, s->q, s->ys, ns));
-        VPMC_TRY(make_items(ctx, s->g, s->q.qstart, s->it, query_chunk(s->precision == 64 ? 4 : s->qpt)));
-        const bool f64 = s->precision == 64;
-        if (f64) VPMC_CUDA(cudaMemsetAsync(s->fv64, 0, sizeof(double) * size_t(ns), st));
-        else VPMC_CUDA(cudaMemsetAsync(s->fv, 0, sizeof(float) * size_t(ns), st));
+                   s->q.qsub, s->q.qrank, f64 ? nullptr : s->fv, f64 ? s->fv64 : nullptr, 1};
+        VPMC_TRY(launch_gen(st, ga));
+        VPMC_TRY(place_samples(ctx, s->g, s->q, s->ys, ns, s->it, query_chunk(f64 ? 4 : s->qpt)));
         EvalLaunch L;
         const bool unb = s->mc[0].law == VPMC_LAW_UNBIASED;
         L.mode = f64 ? (unb ? EVAL_FIELD9_64 : EVAL_FIELD64)
@@ -867,28 +897,28 @@ int issue_pass(vpmc_sim* s, bool advect, bool timed, int* nlaunch) {
         if (timed) VPMC_CUDA(cudaEventRecordWithFlags(s->chunk_ev[2 * ci], st, ev_flags));
         VPMC_TRY(launch_eval(ctx, s->g, s->q.qrec, s->it, L));
         if (timed) VPMC_CUDA(cudaEventRecordWithFlags(s->chunk_ev[2 * ci + 1], st, ev_flags));
+        unsigned long long* const count_step = advect && t0 + nt >= s->t_end ? s->d_step : nullptr;
         if (def) {
             Acc5Args aa{s->d_mc, s->n_inst, s->pos, s->ys, s->fv, t0, nt, s->N1, s->N2, advect ? 1 : 0, s->vel,
-                        s->vel5, s->pos_next, s->F_next, s->d_sig, kCoverCap};
+                        s->vel5, pos_out, F_out, s->d_sig, kCoverCap, count_step};
             VPMC_LAUNCH(k_accum5, blocks_for(nt * 32), 256, 0, st, aa);
         } else if (f64) {
             AccArgs64 aa{s->d_mc, s->n_inst, s->pos, s->ys, s->fv64, s->cum64, t0, nt, s->N1, s->N2, advect ? 1 : 0,
-                         s->vel, s->pos_next};
+                         s->vel, pos_out, count_step};
             VPMC_LAUNCH(k_accum64, blocks_for(nt * 32), 256, 0, st, aa);
         } else {
             AccArgs aa{s->d_mc, s->n_inst, s->pos, s->ys, s->fv, t0, nt, s->N1, s->N2, advect ? 1 : 0, s->vel,
-                       s->pos_next};
+                       pos_out, count_step};
             VPMC_LAUNCH(k_accum, blocks_for(nt * kAccLanes), 256, 0, st, aa);
         }
     }
     mark_samples(s);
-    if (advect) {
+    if (advect && !in_place) {
         // only the pass's targets moved (a shard leaves the others to the exchange)
         const size_t tb = size_t(s->t_begin), tn = size_t(s->t_end - s->t_begin);
         VPMC_CUDA(cudaMemcpyAsync(s->pos + tb, s->pos_next + tb, sizeof(float2) * tn, cudaMemcpyDeviceToDevice, st));
         if (def)
             VPMC_CUDA(cudaMemcpyAsync(s->F + tb, s->F_next + tb, sizeof(float4) * tn, cudaMemcpyDeviceToDevice, st));
-        VPMC_LAUNCH(k_inc_step, 1, 1, 0, st, s->d_step);
     }
     *nlaunch = int(vpmc_kernel_launch_count() - l0);
     return VPMC_OK;

@@ -67,12 +67,17 @@ struct GenArgs {
     float2* ys;
     uint32_t* qbin;
     uint32_t* qcount;
-    uint32_t* qrank;
+    uint32_t* qsub;               // counts per (bin, sub-cell), or nullptr: per bin in qcount
+    uint32_t* qrank;              // with each sample's rank there << 4 | sub-cell, or nullptr
+    float* f32;                   // field values and (adjoint) FP64 values: zeroed where a sample is dropped
+    double* f64;
+    int nf64;                     // FP64 values a sample
 };
 
 // One thread per (target, sign, sample): Philox draw, branch-1 CDF / image /
 // jitter or disk draw, bin + rank (vpmc_sim.cu).
-__global__ void k_gen(GenArgs a);
+// Queued on `st`.
+int launch_gen(cudaStream_t st, const GenArgs& a);
 
 inline int blocks_for(long n, int threads = 256) {
     long b = (n + threads - 1) / threads;
