@@ -1591,18 +1591,38 @@ int blocks_for(long n, int threads = 256) {
 
 int default_k() { return 2; }
 
+// Cells of about 2.6 particle spacings (both signs: 7 particles), as long as a bin
+// still gathers 150 samples: smaller cells trim the walk closer to the disk of
+// radius h_w, but each bin costs a walk, a sort key and its items.  Measured (ms a
+// step, k = 2 -> the rule's k): 512^2, h_w 16 spacings, 64 + 64 samples: 27.0 -> 19.4
+// (k = 6; best 18.9 at 7); 256^2, h_w 8, 32 + 32: 1.25 -> 1.18 (3, the best); 24
+// ensemble members, h_w 8: 27.0 -> 25.5 (3); 256^2, h_w 4, 16 + 16: 0.52 -> 0.50 (1).
+// The rule looks at one instance alone, so that a member of an ensemble sums as a
+// run of its own does.
+int sample_k(long n, double samples, float Lx, float Ly, float hw) {
+    if (n < 1) return default_k();
+    const double spacing = std::sqrt(double(Lx) * Ly / double(n));
+    int k = int(std::lround(double(hw) / (2.6 * spacing)));
+    k = std::min(std::max(k, 1), kMaxK);
+    for (; k > 1; --k) {
+        const double cells = double(k) * Lx / hw * (double(k) * Ly / hw);
+        if (samples >= 150.0 * cells && cells <= double(1L << 22)) break;
+    }
+    return k;
+}
+
 int query_chunk(int qpt) { return (qpt == 8 ? 8 : qpt == 6 ? 6 : 4) * kEvalThreads; }   // qpt 1 (tensor cores): 128
 
 long grid_plan(const InstDesc* in, int n, int k, int nsets, GridInst* out) {
-    if (k <= 0) k = default_k();
     if (k > kMaxK) k = kMaxK;
     long base = 0;
     for (int i = 0; i < n; ++i) {
         const InstDesc& d = in[i];
+        const int k_i = k > 0 ? k : d.k > 0 ? std::min(d.k, kMaxK) : default_k();
         if (!(d.hw > 0.f) || !(d.Lx > 0.f) || !(d.Ly > 0.f)) return -VPMC_ERR_INVALID;
         if (!(d.cover >= 1.f)) return -VPMC_ERR_INVALID;
         const double reach = double(d.hw) * double(d.cover);   // physical support radius to cover
-        int kk = k, gx = 0, gy = 0;
+        int kk = k_i, gx = 0, gy = 0;
         for (; kk >= 1; --kk) {
             gx = int(std::floor(double(kk) * double(d.Lx) / reach + 1e-9));
             gy = int(std::floor(double(kk) * double(d.Ly) / reach + 1e-9));

@@ -211,12 +211,17 @@ struct InstDesc {
     int periodic;
     int p_begin, p_end;
     float cover = 1.f;   // the walk covers cover * h_w: the largest stretch sigma_max(F) of a deformed kernel
+    int k = 0;           // walk cells when the plan is asked for its own choice (0: default_k)
 };
 
 // Plan the grid: fills `out` (n entries) and returns the bin count, or a
-// negative vpmc_status on geometry errors.  k <= 0 selects the default.
+// negative vpmc_status on geometry errors.  k <= 0 selects each instance's own
+// choice.
 long grid_plan(const InstDesc* in, int n, int k, int nsets, GridInst* out);
 int default_k();
+// Walk cells per h_w for an instance of n particles that evaluates `samples` points
+// of each sign set a pass.
+int sample_k(long n, double samples, float Lx, float Ly, float hw);
 
 // Device-side working set of one grid (caller owns the memory).
 struct GridBufs {

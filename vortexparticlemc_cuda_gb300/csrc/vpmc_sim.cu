@@ -778,7 +778,9 @@ int alloc_work(vpmc_sim* s) {
     std::vector<InstDesc> d(s->n_inst);
     for (int i = 0; i < s->n_inst; ++i)
         d[i] = InstDesc{s->prm[i].Lx, s->prm[i].Ly, s->mc[i].hw, s->prm[i].periodic, int(s->begin[i]),
-                        int(s->begin[i] + s->counts[i]), s->deform ? s->cover : 1.f};
+                        int(s->begin[i] + s->counts[i]), s->deform ? s->cover : 1.f,
+                        sample_k(s->counts[i], std::min(double(s->counts[i]) * samples_per(s), double(1L << 29)),
+                                 s->prm[i].Lx, s->prm[i].Ly, s->mc[i].hw)};
     s->plan.resize(s->n_inst);
     const long nb = grid_plan(d.data(), s->n_inst, s->k_walk, 2, s->plan.data());
     if (nb < 0) return int(-nb);
