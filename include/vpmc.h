@@ -440,7 +440,8 @@ int vpmc_sim_set_precision(vpmc_sim* sim, int bits);
  * queries per thread in the field-evaluation kernel (4, 6 or 8), or 1 for the
  * tensor-core evaluation (squared distances of 128 queries x 128 candidates
  * per tcgen05 multiply; plain kernels only, deformed kernels keep 4).
- * 0 = default (k = 2, 4 queries per thread). */
+ * 0 = the library's choice (k by the particle spacing and the samples per bin,
+ * 4 queries per thread). */
 int vpmc_sim_set_tuning(vpmc_sim* sim, int k_walk, int queries_per_thread);
 int vpmc_sim_get_tuning(vpmc_sim* sim, int* k_walk, int* queries_per_thread);
 

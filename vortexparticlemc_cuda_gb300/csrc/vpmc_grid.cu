@@ -7,6 +7,7 @@
 
 #include "vpmc_blocksort.cuh"
 #include "vpmc_grid.cuh"
+#include "vpmc_wide.cuh"
 
 namespace vpmc {
 
@@ -932,13 +933,42 @@ __device__ __forceinline__ void scat_batch(const Cand* __restrict__ s_cand, cons
     }
 }
 
+// One query's sum over one staged run to FP64 precision on the FP32 pipe (see
+// vpmc_wide.cuh): records {xh, xl, yh, yl, w, ., wl, .} already shifted by the
+// run's image.  LOW: some difference may need a second float.  A pair's error is
+// below 1e-20 of W(0) (the FP64 form's: 3.5e-16), at ~190 FP32 instructions for a
+// pair inside the support, 10 outside.
+template <bool LOW>
+__device__ __forceinline__ void wide_run(const Cand* __restrict__ cs, int cnt, float qx, float qy, float h, float lim,
+                                         const wide::W3& half_h3, wide::W3& acc) {
+    for (int c = 0; c < cnt; ++c) {
+        const float4 p = *reinterpret_cast<const float4*>(&cs[c].x);
+        float xh, xl = 0.f, yh, yl = 0.f;
+        if (LOW) {
+            float e;
+            wide::two_sum(p.x, -qx, xh, e);
+            wide::fast_two_sum(xh, wide::add(e, p.y), xh, xl);
+            wide::two_sum(p.z, -qy, yh, e);
+            wide::fast_two_sum(yh, wide::add(e, p.w), yh, yl);
+        } else {
+            xh = p.x - qx;
+            yh = p.z - qy;
+        }
+        if (fmaf(xh, xh, yh * yh) < lim) {
+            const wide::W3 v = wide::spline_h3(wide::norm2<LOW>(xh, xl, yh, yl), h, half_h3);
+            if (v.a > 0.f) wide::add_product(acc, cs[c].w, cs[c].wl, v);
+        }
+    }
+}
+
 // The packed FP32 kernels run one-warp CTAs, 24 per SM (their 6.5 KB staging
 // buffers fit 24 times in shared memory; 85 registers a thread at most) with 4
 // queries per thread, 16 per SM with 6 and 12 with 8.  One warp per CTA: no warp of an item
 // waits at a barrier for another.
 constexpr int eval_min_blocks(int mode, int qpt) {
     return (mode == EVAL_FIELD || mode == EVAL_FIELD9 || mode == EVAL_FIELD_F || mode == EVAL_FIELD9_F)
-               ? (qpt == 4 ? 24 : qpt == 6 ? 16 : 12) : 1;
+               ? (qpt == 4 ? 24 : qpt == 6 ? 16 : 12)
+               : (mode == EVAL_FIELD64 || mode == EVAL_FIELD9_64) ? 20 : 1;
 }
 
 template <int MODE, int QPT>
@@ -960,6 +990,12 @@ __global__ void __launch_bounds__(kEvalThreads, eval_min_blocks(MODE, QPT)) k_ev
     constexpr bool kF64 = MODE == EVAL_SPMV64;
     constexpr bool kComp = MODE == EVAL_SPMV32;
     constexpr bool kField64 = MODE == EVAL_FIELD64 || MODE == EVAL_FIELD9_64;
+    constexpr bool kTrim = kField64 || MODE == EVAL_FIELD || MODE == EVAL_FIELD9 || MODE == EVAL_FIELD_F ||
+                           MODE == EVAL_FIELD9_F;
+    // FP64 field: the item's queries and sums, slot j 32 + lane
+    constexpr int kF64Q = kField64 ? kEvalThreads * QPT : 1;
+    __shared__ float4 s_fq[kF64Q];      // x, y, image flags, id
+    __shared__ double s_fd[kF64Q];
     constexpr bool kGrad = eval_grad(MODE);
     constexpr bool kGrad32 = MODE == EVAL_GRAD32 || MODE == EVAL_GRAD9_32;
     constexpr bool kGrad9 = MODE == EVAL_GRAD9_64 || MODE == EVAL_GRAD9_32;
@@ -1127,8 +1163,18 @@ __global__ void __launch_bounds__(kEvalThreads, eval_min_blocks(MODE, QPT)) k_ev
             }
             if (tid == 0 && it.qcnt > uint32_t(kScatQ)) atomicOr(a.flags, FLAG_CAPACITY);
         }
+        if constexpr (kField64) {
+#pragma unroll
+            for (int j = 0; j < QPT; ++j) {
+                const int k = j * 32 + (tid & 31);
+                const float nan = __int_as_float(0x7fffffff);   // an empty slot is near nothing
+                s_fq[k] = make_float4(qv[j] ? qx[j] : nan, qv[j] ? qy[j] : nan,
+                                      __uint_as_float(uint32_t(qfl >> (6 * j)) & 63u), __uint_as_float(qid[j]));
+                s_fd[k] = 0.0;
+            }
+        }
         __syncthreads();
-        if constexpr (kPacked) {
+        if constexpr (kTrim) {
             // bounding box of this warp's queries in the bin's frame
             float bx0 = INFINITY, bx1 = -INFINITY, by0 = INFINITY, by1 = -INFINITY;
 #pragma unroll
@@ -1186,7 +1232,7 @@ __global__ void __launch_bounds__(kEvalThreads, eval_min_blocks(MODE, QPT)) k_ev
             __syncthreads();
             }
             if (s_btot == 0) break;
-            if constexpr (kPacked) {
+            if constexpr (kTrim) {
                 // this warp's part of each staged run: the sub-rows within reach of
                 // its queries' bounding box (reach widened by 0.1%, sub-row bounds by
                 // 1% of a sub-row, so no pair with a non-zero term is dropped: the
@@ -1222,7 +1268,7 @@ __global__ void __launch_bounds__(kEvalThreads, eval_min_blocks(MODE, QPT)) k_ev
             // packed modes rewrite them first, so their barrier follows that pass
             if (!mbar_wait_bounded(&s_bar, phase, a.wait_limit)) atomicOr(&s_abort, 1);
             phase ^= 1u;
-            if constexpr (!kPacked) {
+            if constexpr (!kPacked && !kField64) {
                 __syncthreads();
                 if (tid == 0) s_pre = 0;
                 if (s_abort) break;
@@ -1272,7 +1318,96 @@ __global__ void __launch_bounds__(kEvalThreads, eval_min_blocks(MODE, QPT)) k_ev
                 if (tid == 0) s_pre = 0;
                 if (s_abort) break;   // (a thread whose wait expired rewrote stale bytes: unused)
             }
-            for (int b = 0; b < (kScat ? 0 : nbp); ++b) {
+            if constexpr (kField64) {
+                static_assert(kEvalThreads == 32, "one warp an item");
+                // candidates -> the image of their run, exactly (two floats); the weights'
+                // range, and whether every difference within reach is one float
+                const float h3 = 2.f * G.half_h3[0], near = G.reach * 1.01f;
+                float most = 0.f, least = INFINITY;
+                bool finite = true, exact = true;
+                for (int b = 0; b < nbp; ++b) {
+                    const BatchPiece bp = s_bp[b];
+                    const Piece pc = s_pc[bp.piece];
+                    for (uint32_t c = threadIdx.x; c < bp.cnt; c += kEvalThreads) {
+                        Cand& cd = s_cand[bp.soff + c];
+                        float xh, xl, yh, yl;
+                        wide::two_sum(cd.x, -pc.qdx, xh, xl);
+                        wide::two_sum(cd.y, -pc.qdy, yh, yl);
+                        cd.x = xh;
+                        cd.x2 = xl;
+                        cd.y = yh;
+                        cd.y2 = yl;
+                        const float a = fabsf(cd.w);
+                        finite = finite && a <= 3.0e38f;
+                        most = fmaxf(most, a);
+                        if (a > 0.f) least = fminf(least, a);
+                        exact = exact && xl == 0.f && yl == 0.f && fabsf(xh) >= near && fabsf(yh) >= near;
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < QPT; ++j) exact = exact && (!qv[j] || (fabsf(qx[j]) >= near && fabsf(qy[j]) >= near));
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+                    least = fminf(least, __shfl_xor_sync(0xffffffffu, least, o));
+                }
+                // weights times a power of two: the largest product h^3 w is about 1, and the
+                // smallest keeps its three floats above the underflow
+                const int ex = min(max(254 - int(__float_as_uint(most) >> 23) + 127 - int(__float_as_uint(h3) >> 23), 1), 253);
+                const float scale = __uint_as_float(uint32_t(ex) << 23);
+                const bool fits = __all_sync(0xffffffffu, finite) && G.hw >= 1e-6f && G.hw <= 1e6f &&
+                                  (most == 0.f || (least * scale * h3 >= 1e-20f && most * scale * h3 <= 1e20f));
+                exact = __all_sync(0xffffffffu, exact);
+                __syncthreads();
+                if (tid == 0) s_pre = 0;
+                if (s_abort) break;   // (a thread whose wait expired rewrote stale bytes: unused)
+                if (fits)
+                    for (uint32_t c = threadIdx.x; c < s_btot; c += kEvalThreads) {
+                        s_cand[c].w *= scale;
+                        s_cand[c].wl *= scale;
+                    }
+                __syncthreads();
+                const double unit = G.inv_h3 / double(scale);
+                const float lim = G.hw * G.hw * 1.00001f;
+                const wide::W3 half_h3{G.half_h3[0], G.half_h3[1], G.half_h3[2]};
+#pragma unroll 1
+                for (int j = 0; j < 2 * npw; ++j) {
+                    const int k = j * 32 + (tid & 31);
+                    const float4 q = s_fq[k];
+                    const uint32_t fl = __float_as_uint(q.z);
+                    wide::W3 acc3{0.f, 0.f, 0.f};
+                    double accd = 0.0;
+#pragma unroll 1
+                    for (int b = 0; b < nbp; ++b) {
+                        const uint2 rg = s_rng[0][b];
+                        const BatchPiece bp = s_bp[b];
+                        if (kField9) {
+                            const Piece pc = s_pc[bp.piece];
+                            const int mx = int(fl & 7u) - 2 + pc.mx, my = int((fl >> 3) & 7u) - 2 + pc.my;
+                            if (!(mx >= -1 && mx <= 1 && my >= -1 && my <= 1)) continue;
+                        }
+                        const Cand* cs = s_cand + bp.soff + rg.x;
+                        const int cnt = int(rg.y) - int(rg.x);
+                        if (fits && exact) wide_run<false>(cs, cnt, q.x, q.y, G.hw, lim, half_h3, acc3);
+                        else if (fits) wide_run<true>(cs, cnt, q.x, q.y, G.hw, lim, half_h3, acc3);
+                        else {
+                            const double ih = 1.0 / double(G.hw), A = 3.0 * ih * ih * ih, B = -3.0 * ih * ih;
+                            const double px = q.x, py = q.y;
+                            for (int c = 0; c < cnt; ++c) {
+                                const Cand cv = cs[c];
+                                const double dx = (double(cv.x) + double(cv.x2)) - px;
+                                const double dy = (double(cv.y) + double(cv.y2)) - py;
+                                const double r2 = dx * dx + dy * dy, r = sqrt(r2);
+                                const double inner = 0.5 + r2 * (A * r + B), t = 1.0 - ih * r;
+                                accd += (double(cv.w) + double(cv.wl)) * fmax(fmin(inner, t * t * t), 0.0);
+                            }
+                        }
+                    }
+                    if (fits) accd = ((double(acc3.a) + double(acc3.b)) + double(acc3.c)) * unit;
+                    s_fd[k] += accd;
+                }
+            }
+            for (int b = 0; b < (kScat || kField64 ? 0 : nbp); ++b) {
                 const BatchPiece bp = s_bp[b];
                 const Piece pc = s_pc[bp.piece];
                 int cnt = int(bp.cnt);
@@ -1440,31 +1575,6 @@ __global__ void __launch_bounds__(kEvalThreads, eval_min_blocks(MODE, QPT)) k_ev
                         accg[j][1] += double(pgy[j]);
                         part[j] = 0.0;
                     }
-                } else if constexpr (kField64) {
-                    // the plain FP64 path: every pair and the sum in FP64
-                    const double hw = double(G.hw), ih = 1.0 / hw;
-                    const double A = 3.0 * ih * ih * ih, B = -3.0 * ih * ih;
-                    double px[QPT], py[QPT];
-#pragma unroll
-                    for (int j = 0; j < QPT; ++j) {
-                        px[j] = double(qx[j]) + double(pc.qdx);
-                        py[j] = double(qy[j]) + double(pc.qdy);
-                        part[j] = 0.0;
-                    }
-                    for (int c = 0; c < cnt; ++c) {
-                        const Cand cv = cs[c];
-                        const double cxd = cv.x, cyd = cv.y, wd = double(cv.w) + double(cv.wl);
-#pragma unroll
-                        for (int j = 0; j < QPT; ++j) {
-                            const double dx = cxd - px[j], dy = cyd - py[j];
-                            const double r2 = dx * dx + dy * dy;
-                            const double r = sqrt(r2);
-                            const double inner = 0.5 + r2 * (A * r + B);
-                            const double t = 1.0 - ih * r;
-                            const double v = fmax(fmin(inner, t * t * t), 0.0);
-                            part[j] += wd * v;
-                        }
-                    }
                 } else if constexpr (kF64) {
                     float px[QPT], py[QPT];
 #pragma unroll
@@ -1548,7 +1658,10 @@ __global__ void __launch_bounds__(kEvalThreads, eval_min_blocks(MODE, QPT)) k_ev
                 a.out_f64[3 * size_t(qid[j])] = acc[j];
                 a.out_f64[3 * size_t(qid[j]) + 1] = accg[j][0];
                 a.out_f64[3 * size_t(qid[j]) + 2] = accg[j][1];
-            } else if constexpr (kF64 || kField64) a.out_f64[qid[j]] = acc[j];
+            } else if constexpr (kField64) {
+                const int k = j * 32 + (tid & 31);
+                a.out_f64[qid[j]] = s_fd[k];
+            } else if constexpr (kF64) a.out_f64[qid[j]] = acc[j];
             else if constexpr (kComp) a.out_f64[qid[j]] = double(acc[j]) - double(acc_c[j]);
             else a.out_f32[qid[j]] = acc[j];
         }
@@ -1650,6 +1763,13 @@ long grid_plan(const InstDesc* in, int n, int k, int nsets, GridInst* out) {
         g.two_sigma = float(2.0 * 40.0 / (7.0 * kPiD * h * h));
         g.p_begin = d.p_begin;
         g.p_end = d.p_end;
+        // h^3 / 2 exactly (72 bits) as three floats: h^2 is exact in FP64, its product
+        // with h as a value and an error
+        const double h2 = h * h, c = h2 * h * 0.5, ce = std::fma(h2, h * 0.5, -c);
+        g.half_h3[0] = float(c);
+        g.half_h3[1] = float((c - double(g.half_h3[0])) + ce);
+        g.half_h3[2] = float(((c - double(g.half_h3[0])) - double(g.half_h3[1])) + ce);
+        g.inv_h3 = 1.0 / (h * h * h);
         out[i] = g;
         base += long(nsets) * gx * gy;
         if (base >= (1L << 31)) return -VPMC_ERR_CAPACITY;

@@ -33,6 +33,8 @@ struct GridInst {
     float A, B;             // 3/h_w^3, -3/h_w^2: W/(2 sigma) = min(0.5 + r^2 (A r + B), (1 - r/h_w)^3)
     float two_sigma;        // 2 * 40 / (7 pi h_w^2)
     int p_begin, p_end;     // particle range of the instance
+    float half_h3[3];       // h_w^3 / 2 as a sum of three floats (vpmc_wide.cuh)
+    double inv_h3;          // 1 / h_w^3
 };
 
 // Candidate record (32 bytes): coordinates and weight duplicated so that one
@@ -157,8 +159,8 @@ enum EvalMode : int {
     EVAL_FIELD_EXC = 2,  // as FIELD, pairs closer than 1e-6 skipped (exclude_center)
     EVAL_SPMV64 = 3,     // out_f64[id] = sum (w + w_lo) W, in-support pairs in FP64
     EVAL_SPMV32 = 4,     // out_f64[id] = compensated FP32 sum
-    EVAL_FIELD64 = 5,    // as FIELD, every pair in FP64 (weight w + wl), out_f64[id]
-    EVAL_FIELD9_64 = 6,  // as FIELD9 in FP64
+    EVAL_FIELD64 = 5,    // as FIELD, every pair to FP64 precision or better (weight w + wl), out_f64[id]
+    EVAL_FIELD9_64 = 6,  // as FIELD9, likewise
     EVAL_FIELD_F = 7,    // as FIELD with deformed kernels W(|F^-1 d|) (CandF records)
     EVAL_FIELD9_F = 8,   // as FIELD9 with deformed kernels
     EVAL_FIELD_F_EXC = 9,// as FIELD_EXC with deformed kernels (pairs with |F^-1 d| < 1e-6 skipped)
