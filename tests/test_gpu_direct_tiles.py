@@ -73,15 +73,23 @@ def test_plummer_general_tiles(cuda, what):
                 assert not np.isfinite(np.delete(got, 100, 0)).any()
 
 
-@pytest.mark.parametrize("n,m,param,Lx,Ly", [(1, 3, 0.05, 1.0, 1.0), (255, 1, 0.3, 1.0, 1.0), (256, 257, 0.05, 0.7, 1.3),
-                                             (257, 256, 1e-5, 1.0, 1.0), (3000, 100, 0.02, 1.0, 2.0)])
-def test_mollified_rows(cuda, n, m, param, Lx, Ly):
+# periods that are floats take the three-float sums, 0.7 and 1.3 the FP64 rows; a
+# core of 0.3 has many images inside it (more than a thread notes); "range" has a
+# tile of strengths too far apart for the floats
+@pytest.mark.parametrize("n,m,param,Lx,Ly,what", [
+    (1, 3, 0.05, 1.0, 1.0, ""), (255, 1, 0.3, 1.0, 1.0, ""), (256, 257, 0.05, 0.7, 1.3, ""), (257, 256, 1e-5, 1.0, 1.0, ""),
+    (3000, 100, 0.02, 1.0, 2.0, ""), (600, 40, 0.05, 1.0, 1.0, "range"), (300, 40, 0.05, 1.0, 1.0, "small")])
+def test_mollified_periodic(cuda, n, m, param, Lx, Ly, what):
     from vortexparticlemc_cuda_gb300 import phash as P
     rng = np.random.default_rng(n)
     L = np.array([Lx, Ly])
     pos = (rng.random((n, 2)) * L).astype(np.float32)
     om = rng.normal(size=n).astype(np.float32)
     om[::5] = 0.0
+    if what == "range":
+        om[1] = 1e25
+    if what == "small":
+        om *= np.float32(1e-33)
     pts = (rng.random((m, 2)) * L).astype(np.float32)
     pts[0] = pos[0]                                   # an image at r = 0
     got = P.direct_velocity(to_dev(pos, cuda), to_dev(om, cuda), pts=to_dev(pts, cuda), param=param, Lx=Lx,

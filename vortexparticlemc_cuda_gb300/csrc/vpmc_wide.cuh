@@ -30,12 +30,18 @@ VPMC_WIDE_FN float rsqrt_est(float a) {
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
     return r;
 }
+VPMC_WIDE_FN float rcp_est(float a) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
 #else
 VPMC_WIDE_FN float add(float a, float b) { return a + b; }
 VPMC_WIDE_FN float sub(float a, float b) { return a - b; }
 VPMC_WIDE_FN float mul(float a, float b) { return a * b; }
 VPMC_WIDE_FN float fma(float a, float b, float c) { return std::fmaf(a, b, c); }
 VPMC_WIDE_FN float rsqrt_est(float a) { return 1.f / std::sqrt(a); }
+VPMC_WIDE_FN float rcp_est(float a) { return 1.f / a; }
 #endif
 
 VPMC_WIDE_FN void two_sum(float a, float b, float& s, float& e) {
@@ -93,6 +99,44 @@ VPMC_WIDE_FN W3 sub3(const W3& x, const W3& y) {
     two_sum(x.b, -y.b, m, em);
     two_sum(m, e, n, en);
     return W3{s, n, add(add(em, en), sub(x.c, y.c))};
+}
+
+// x + y (unnormalised).
+VPMC_WIDE_FN W3 add3(const W3& x, const W3& y) {
+    float s, e, m, em, n, en;
+    two_sum(x.a, y.a, s, e);
+    two_sum(x.b, y.b, m, em);
+    two_sum(m, e, n, en);
+    return W3{s, n, add(add(em, en), add(x.c, y.c))};
+}
+// (h + l) y and w y for single floats h, l, w.
+VPMC_WIDE_FN W3 mul2(float h, float l, const W3& y) {
+    float p, e, q, eq, s, es, n, en, m, em;
+    two_prod(h, y.a, p, e);
+    two_prod(h, y.b, q, eq);
+    two_prod(l, y.a, s, es);
+    two_sum(q, s, n, en);
+    two_sum(n, e, m, em);
+    float c = add(add(en, em), add(eq, es));
+    c = fma(l, y.b, c);
+    return W3{p, m, fma(h, y.c, c)};
+}
+VPMC_WIDE_FN W3 mul1(float w, const W3& y) {
+    float p, e, q, eq, n, en;
+    two_prod(w, y.a, p, e);
+    two_prod(w, y.b, q, eq);
+    two_sum(q, e, n, en);
+    return W3{p, n, fma(w, y.c, add(en, eq))};
+}
+// 1 / x: the estimate y, then y (1 + e + e^2) with the residual e = 1 - x y to 2^-70.
+VPMC_WIDE_FN W3 rcp3(const W3& x) {
+    const float y = rcp_est(x.a);
+    float f, fe, eh, el, p, pe;
+    two_prod(x.b, y, f, fe);
+    two_sum(fma(-x.a, y, 1.f), -f, eh, el);
+    el = fma(-x.c, y, sub(el, fe));
+    two_prod(y, eh, p, pe);
+    return W3{y, p, fma(y, fma(eh, eh, el), pe)};
 }
 
 // |d|^2 of d = (xh + xl, yh + yl), |xl| <= ulp(xh); LOW = false: xl = yl = 0.
