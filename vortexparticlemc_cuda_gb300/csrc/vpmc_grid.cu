@@ -1777,7 +1777,7 @@ long grid_plan(const InstDesc* in, int n, int k, int nsets, GridInst* out) {
     return base;
 }
 
-void carve_grid(Carver& c, long n, long nbins, int n_inst, GridBufs* g, bool deformed, int rows) {
+void carve_grid(Carver& c, long n, long nbins, int n_inst, GridBufs* g, bool deformed, int rows, bool records) {
     g->inst = c.take<GridInst>(size_t(n_inst));
     g->n_inst = n_inst;
     g->nbins = nbins;
@@ -1787,14 +1787,12 @@ void carve_grid(Carver& c, long n, long nbins, int n_inst, GridBufs* g, bool def
     g->keys = c.take<uint32_t>(size_t(n < 1 ? 1 : n));
     g->start = c.take<uint32_t>(size_t(nsub + 1));
     g->cstart = g->rows > 1 ? c.take<uint32_t>(size_t(nbins + 1)) : g->start;
-    g->cand = c.take<Cand>(size_t(n < 1 ? 1 : n));
+    g->cand = records ? c.take<Cand>(size_t(n < 1 ? 1 : n)) : nullptr;
     g->candf = deformed ? c.take<CandF>(size_t(n < 1 ? 1 : n)) : nullptr;
     carve_radix(c, n, &g->rs);
 }
 
-int grid_build(vpmc_context* ctx, GridBufs& g, const float2* pos, const float* omega, int set_mode,
-               const float4* F) {
-    if (F && !g.candf) return VPMC_ERR_INVALID;
+int grid_sort(vpmc_context* ctx, GridBufs& g, const float2* pos, const float* omega, int set_mode) {
     cudaStream_t st = ctx->stream;
     const long nsub = g.nbins * g.rows;
     uint32_t *ks = g.keys, *vs = g.rs.vbuf[0];
@@ -1813,6 +1811,16 @@ int grid_build(vpmc_context* ctx, GridBufs& g, const float2* pos, const float* o
         VPMC_LAUNCH(k_grid_starts, blocks_for(nsub + 1), 256, 0, st, ks, uint32_t(g.n), nsub, g.rows, g.start, g.cstart);
     }
     g.perm = vs;
+    return VPMC_OK;
+}
+
+int grid_build(vpmc_context* ctx, GridBufs& g, const float2* pos, const float* omega, int set_mode,
+               const float4* F) {
+    if (F && !g.candf) return VPMC_ERR_INVALID;
+    cudaStream_t st = ctx->stream;
+    VPMC_TRY(grid_sort(ctx, g, pos, omega, set_mode));
+    const long nsub = g.nbins * g.rows;
+    const uint32_t* vs = g.perm;
     if (F)
         VPMC_LAUNCH(k_grid_gather_f, blocks_for(g.n), 256, 0, st, vs, g.start, g.n, uint32_t(nsub), pos, omega, F,
                     g.inst, g.n_inst, set_mode, g.candf);

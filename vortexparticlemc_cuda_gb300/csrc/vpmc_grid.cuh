@@ -240,12 +240,15 @@ struct GridBufs {
     uint32_t* perm = nullptr;   // n: sorted slot -> particle (points into rs buffers)
     RadixScratch rs{};
 };
-void carve_grid(Carver& c, long n, long nbins, int n_inst, GridBufs* g, bool deformed = false, int rows = 1);
+void carve_grid(Carver& c, long n, long nbins, int n_inst, GridBufs* g, bool deformed = false, int rows = 1,
+                bool records = true);
 
 // Bin keys + counts + stable sort + ranges + gather.  weights == nullptr uses
 // omega (SET_SIGN_SPLIT scales |omega| by 2 sigma, SET_ONE_SIGNED by
 // 2 sigma too).  Writes g.cand / g.start / g.perm; with F (per particle,
 // row-major {F11, F12, F21, F22}) it writes the deformed records g.candf.
+// grid_sort: keys, sort and ranges alone.
+int grid_sort(vpmc_context* ctx, GridBufs& g, const float2* pos, const float* omega, int set_mode);
 int grid_build(vpmc_context* ctx, GridBufs& g, const float2* pos, const float* omega, int set_mode,
                const float4* F = nullptr);
 // Overwrite candidate weights from a vector in sorted order: cand[p].z/.w =

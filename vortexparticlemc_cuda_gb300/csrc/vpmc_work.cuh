@@ -23,13 +23,13 @@ inline int work_blocks(long n) {
 }
 
 inline int setup_work(vpmc_context* ctx, int slot, long N, float hw, float Lx, float Ly, int periodic, long M, int nvec,
-                      Work* w, int k = 0, float cover = 1.f, bool deformed = false) {
+                      Work* w, int k = 0, float cover = 1.f, bool deformed = false, int rows = 1) {
     InstDesc d{Lx, Ly, hw, periodic, 0, int(N), cover};
     const long nb = grid_plan(&d, 1, k, 1, &w->plan);
     if (nb < 0) return int(-nb);
     const long nq = M > N ? M : N;
     auto carve_all = [&](Carver& c) {
-        carve_grid(c, N, nb, 1, &w->g, deformed);
+        carve_grid(c, N, nb, 1, &w->g, deformed, rows);
         carve_items(c, nb, nq, &w->it);
         if (M > 0) carve_queries(c, nb, M, &w->q);
         w->self = c.take<QRec>(size_t(N < 1 ? 1 : N));
