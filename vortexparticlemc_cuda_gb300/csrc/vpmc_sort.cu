@@ -105,27 +105,50 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* in,
 }
 
 // Up to kSmallScan elements by one CTA of 1024 threads, in place of the three
-// launches of the tiled scan (each a few microseconds of latency).
-constexpr int kSmallScan = 16384;
+// launches of the tiled scan (each 3 us and more).  A warp takes a contiguous part,
+// in coalesced rows of 32 (a contiguous part per thread touches a sector per
+// element: 32,768 elements took 37 us that way, 9 us this way).
+constexpr int kSmallScan = 32768;
 
 __global__ void __launch_bounds__(1024) k_scan_small(const uint32_t* in, uint32_t* out, int n, int write_total) {
-    __shared__ uint32_t wt[33];
-    constexpr int kPer = kSmallScan / 1024;
-    const int per = (n + 1023) / 1024, base = int(threadIdx.x) * per;
-    uint32_t v[kPer], s = 0;
+    __shared__ uint32_t s_warp[32];
+    constexpr int kRows = kSmallScan / 1024;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int rows = (n + 1023) / 1024, base = w * rows * 32 + lane;
+    uint32_t v[kRows], s = 0;
 #pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-        v[i] = i < per && base + i < n ? in[base + i] : 0u;
-        s += v[i];
+    for (int r = 0; r < kRows; ++r) {
+        v[r] = r < rows && base + r * 32 < n ? in[base + r * 32] : 0u;
+        s += v[r];
     }
-    uint32_t tot;
-    uint32_t run = block_exclusive(s, wt, &tot);
+    s = __reduce_add_sync(0xffffffffu, s);
+    if (lane == 0) s_warp[w] = s;
+    __syncthreads();
+    if (w == 0) {
+        const uint32_t t = s_warp[lane];
+        uint32_t inc = t;
 #pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-        if (i < per && base + i < n) out[base + i] = run;
-        run += v[i];
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += y;
+        }
+        s_warp[lane] = inc - t;
+        if (lane == 31 && write_total) out[n] = inc;
     }
-    if (write_total && threadIdx.x == 0) out[n] = tot;
+    __syncthreads();
+    uint32_t run = s_warp[w];
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+        if (r >= rows) break;
+        uint32_t inc = v[r];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += y;
+        }
+        if (base + r * 32 < n) out[base + r * 32] = run + inc - v[r];
+        run += __shfl_sync(0xffffffffu, inc, 31);
+    }
 }
 
 template <int ITEMS>
