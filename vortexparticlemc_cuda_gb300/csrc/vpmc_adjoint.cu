@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "vpmc_sim.cuh"
+#include "vpmc_wide.cuh"
 
 namespace vpmc {
 namespace {
@@ -90,7 +91,8 @@ struct AdjArgs {
     int n_inst;
     const float2* pos;
     const float2* ys;
-    const double* fg;       // 3 per sample: f, df/dx, df/dy
+    const double* fg;       // 3 per sample: f, df/dx, df/dy (FP64 path)
+    const float* fg32;      // the same (FP32 path)
     const int* src;
     const double* cum64;    // 2 per instance (x9 when periodic)
     long t0, nt;
@@ -103,8 +105,23 @@ struct AdjArgs {
     double* csum;           // 2 per instance: sum of c over branch-1 samples
 };
 
+// A lane's sum: FP64, or (FP32 path) three floats, which add FP32 terms with more
+// digits than FP64 and without its 64-fold price.
+template <bool F32>
+struct AdjSum {
+    double d = 0.0;
+    __device__ __forceinline__ void add(double x) { d += x; }
+    __device__ __forceinline__ double value() const { return d; }
+};
+template <>
+struct AdjSum<true> {
+    float s[3] = {0.f, 0.f, 0.f};
+    __device__ __forceinline__ void add(float x) { wide::add_float(s, x); }
+    __device__ __forceinline__ double value() const { return (double(s[0]) + double(s[1])) + double(s[2]); }
+};
+
 // One warp per target: the MIS-term derivatives of all its samples, each in
-// FP32 (F32: the FP32 path) or FP64, every sum and atomic in FP64.
+// FP32 (F32: the FP32 path) or FP64, the sums as AdjSum, every atomic in FP64.
 template <bool F32>
 __global__ void __launch_bounds__(256) k_adj_terms(AdjArgs a) {
     using R_ = typename std::conditional<F32, float, double>::type;
@@ -113,6 +130,9 @@ __global__ void __launch_bounds__(256) k_adj_terms(AdjArgs a) {
     const long nwarps = (long(gridDim.x) * blockDim.x) >> 5;
     const int Q = a.N1 + a.N2;
     const double w1 = double(a.N1) / Q, w2 = double(a.N2) / Q, inv = 1.0 / Q;
+    const R_* fg;
+    if constexpr (F32) fg = a.fg32;
+    else fg = a.fg;
     for (long tl = warp; tl < a.nt; tl += nwarps) {
         const long t = a.t0 + tl;
         const int ii = inst_of(a.mc, a.n_inst, t);
@@ -121,52 +141,52 @@ __global__ void __launch_bounds__(256) k_adj_terms(AdjArgs a) {
         const double R = sqrt(double(I.Lx) * I.Lx + double(I.Ly) * I.Ly);   // as the FP64 path
         const double alpha = 1.0 / (2.0 * kPiD * R);
         const double mux = double(I.dt) * a.lam_next[2 * t], muy = double(I.dt) * a.lam_next[2 * t + 1];
-        double ltx = 0.0, lty = 0.0;
+        AdjSum<F32> ltx, lty;
         for (int s = 0; s < 2; ++s) {
             const double sg = (s == 0 ? inv : -inv);
-            const double vx = mux * sg, vy = muy * sg;
-            const double cum = a.cum64[2 * ii + s];
+            const R_ vx = R_(mux * sg), vy = R_(muy * sg);
+            const R_ cum = R_(a.cum64[2 * ii + s]);
             const long base = (tl * 2 + s) * Q;
-            double dca = 0.0, csa = 0.0;
+            AdjSum<F32> dca, csa;
             for (int j = lane; j < Q; j += 32) {
                 const long sid = base + j;
-                R_ gxr, gyr, dfr, dcr, cvr;
-                mis_term_adj<R_>(I.law, x, a.ys[sid], R_(a.fg[3 * sid]), R_(w1), R_(w2), R_(cum), R_(alpha), R_(R), I,
-                                 R_(vx), R_(vy), gxr, gyr, dfr, dcr, cvr);
-                const double gxx = gxr, gxy = gyr, df = dfr, dc = dcr, cv = cvr;
-                ltx += gxx;
-                lty += gxy;
-                const double dyx = -gxx + double(dfr * R_(a.fg[3 * sid + 1]));
-                const double dyy = -gxy + double(dfr * R_(a.fg[3 * sid + 2]));
+                R_ gxx, gxy, df, dc, cv;
+                mis_term_adj<R_>(I.law, x, a.ys[sid], fg[3 * sid], R_(w1), R_(w2), cum, R_(alpha), R_(R), I, vx, vy, gxx,
+                                 gxy, df, dc, cv);
+                const R_ fx = df * fg[3 * sid + 1], fy = df * fg[3 * sid + 2];   // dc/dy = -dc/dx|_f + dc/df grad f
+                ltx.add(gxx);
+                lty.add(gxy);
                 if (j >= a.N1) {
-                    ltx += dyx;
-                    lty += dyy;
+                    ltx.add(-gxx);
+                    ltx.add(fx);
+                    lty.add(-gxy);
+                    lty.add(fy);
                 } else {
+                    const double dyx = double(fx) - double(gxx), dyy = double(fy) - double(gxy);
                     const int p = a.src[sid];
                     if (p >= 0 && (dyx != 0.0 || dyy != 0.0)) {
                         atomicAdd(&a.lam[2 * p], dyx);
                         atomicAdd(&a.lam[2 * p + 1], dyy);
                     }
-                    if (a.gsc && p >= 0 && cv != 0.0) {
-                        atomicAdd(&a.gsc[p], cv);
-                        csa += cv;
+                    if (a.gsc && p >= 0 && cv != R_(0)) {
+                        atomicAdd(&a.gsc[p], double(cv));
+                        csa.add(cv);
                     }
                 }
-                a.as[sid] = df;
-                dca += dc;
+                a.as[sid] = double(df);
+                dca.add(dc);
             }
-            dca = warp_sum_d(dca);
-            if (lane == 0 && dca != 0.0) atomicAdd(&a.dcum[2 * ii + s], dca);
+            const double dcs = warp_sum_d(dca.value());
+            if (lane == 0 && dcs != 0.0) atomicAdd(&a.dcum[2 * ii + s], dcs);
             if (a.gsc) {
-                csa = warp_sum_d(csa);
-                if (lane == 0 && csa != 0.0) atomicAdd(&a.csum[2 * ii + s], csa);
+                const double css = warp_sum_d(csa.value());
+                if (lane == 0 && css != 0.0) atomicAdd(&a.csum[2 * ii + s], css);
             }
         }
-        ltx = warp_sum_d(ltx);
-        lty = warp_sum_d(lty);
+        const double lx = warp_sum_d(ltx.value()), ly = warp_sum_d(lty.value());
         if (lane == 0) {
-            atomicAdd(&a.lam[2 * t], ltx);
-            atomicAdd(&a.lam[2 * t + 1], lty);
+            atomicAdd(&a.lam[2 * t], lx);
+            atomicAdd(&a.lam[2 * t + 1], ly);
         }
     }
 }
@@ -263,22 +283,24 @@ int adjoint_step(vpmc_sim* s, AdjBufs& A, const double* lam_in, double* lam_out,
     for (long t0 = 0; t0 < s->N; t0 += s->chunk_targets) {
         const long nt = std::min(s->chunk_targets, s->N - t0);
         const long ns = nt * 2 * Q;
+        const bool f32 = s->precision == 32;
+        float* const fg32 = reinterpret_cast<float*>(A.fg);
         VPMC_TRY(clear_counts(ctx, s->q));
         GenArgs ga{s->d_mc, s->n_inst, s->g.inst, s->pos, nullptr, nullptr, s->sub, s->cdf, s->guide, s->jit, s->d_step, t0,
-                   nt, s->N1, s->N2, 1, A.src, s->ys, s->q.qbin, s->q.qcount, s->q.qsub, s->q.qrank, nullptr, A.fg, 3};
+                   nt, s->N1, s->N2, 1, A.src, s->ys, s->q.qbin, s->q.qcount, s->q.qsub, s->q.qrank, f32 ? fg32 : nullptr, f32 ? nullptr : A.fg, 3};
         VPMC_TRY(launch_gen(st, ga));
-        // f and grad f at every sample (FP64)
+        // f and grad f at every sample
         VPMC_TRY(place_samples(ctx, s->g, s->q, s->ys, ns, s->it, query_chunk(4)));
         EvalLaunch L;
         // field values and gradients at the samples: the FP32 path's adjoint sums
-        // its pairs in FP32 (into FP64 run sums; the candidates are the particles
-        // in grid order, so the sums are fixed-order), the FP64 path's in FP64
-        const bool f32 = s->precision == 32;
+        // its pairs in FP32 (its terms read them in FP32; the candidates are the
+        // particles in grid order, so the sums are fixed-order), the FP64 path's in FP64
         L.mode = unb ? (f32 ? EVAL_GRAD9_32 : EVAL_GRAD9_64) : (f32 ? EVAL_GRAD32 : EVAL_GRAD64);
         L.qpt = 4;
+        L.out_f32 = fg32;
         L.out_f64 = A.fg;
         VPMC_TRY(launch_eval(ctx, s->g, s->q.qrec, s->it, L));
-        AdjArgs aa{s->d_mc, s->n_inst, s->pos, s->ys, A.fg, A.src, s->cum64, t0, nt, s->N1, s->N2, lam_in, lam_out,
+        AdjArgs aa{s->d_mc, s->n_inst, s->pos, s->ys, A.fg, fg32, A.src, s->cum64, t0, nt, s->N1, s->N2, lam_in, lam_out,
                    A.as, A.dcum, score ? A.gsc : nullptr, A.csum};
         if (f32) VPMC_LAUNCH(k_adj_terms<true>, blocks_for(nt * 32), 256, 0, st, aa);
         else VPMC_LAUNCH(k_adj_terms<false>, blocks_for(nt * 32), 256, 0, st, aa);

@@ -94,18 +94,21 @@ __global__ void __launch_bounds__(kSmallThreads) k_grid_small(const float2* __re
 }
 
 // First candidate of every sub-row (and of every bin): the first sorted key >= k,
-// searched between the block's bounds (its 256 consecutive keys span few
-// candidates).  Counting the keys with an atomic each and scanning the counts
-// moves 16 bytes a sub-row and takes five launches; this writes 4.
+// searched between the bounds of the block's span of consecutive keys (few
+// candidates).  Counting the keys with an atomic each and scanning the counts moves
+// 16 bytes a sub-row and takes five launches; this writes 4.  A long span shares
+// the two full searches (14.5 M sub-rows: 212 us with spans of 256, 101 us with 4096).
 __global__ void __launch_bounds__(256) k_grid_starts(const uint32_t* __restrict__ keys, uint32_t n, long nsub, int rows,
-                                                     uint32_t* __restrict__ start, uint32_t* __restrict__ cstart) {
+                                                     int span, uint32_t* __restrict__ start,
+                                                     uint32_t* __restrict__ cstart) {
     __shared__ uint32_t s_b[2];
-    for (long k0 = long(blockIdx.x) * 256; k0 <= nsub; k0 += long(gridDim.x) * 256) {
-        if (threadIdx.x < 2) s_b[threadIdx.x] = lower_bound_key(keys, n, uint32_t(min(nsub, k0 + long(threadIdx.x) * 255)));
+    for (long k0 = long(blockIdx.x) * span; k0 <= nsub; k0 += long(gridDim.x) * span) {
+        if (threadIdx.x < 2)
+            s_b[threadIdx.x] = lower_bound_key(keys, n, uint32_t(min(nsub, k0 + long(threadIdx.x) * (span - 1))));
         __syncthreads();
-        const long k = k0 + threadIdx.x;
-        if (k <= nsub) {
-            const uint32_t lo = s_b[0], s = lo + lower_bound_key(keys + lo, s_b[1] - lo, uint32_t(k));
+        const uint32_t lo = s_b[0], hi = s_b[1];
+        for (long k = k0 + threadIdx.x; k <= nsub && k < k0 + span; k += 256) {
+            const uint32_t s = lo + lower_bound_key(keys + lo, hi - lo, uint32_t(k));
             start[k] = s;
             if (rows > 1 && k % rows == 0) cstart[k / rows] = s;
         }
@@ -828,19 +831,24 @@ __device__ __forceinline__ void two_sum_acc(float& s, float& e, float x) {
     s = t;
 }
 
-// W / 2 sigma of the cubic spline and its r-derivative over r, for FP32 pairs
-// without a branch: one reciprocal square root gives r and 1/r, the inner and
-// outer pieces are selected, and beyond the support t = (1 - r/h)+ = 0 makes
-// both exactly zero (r > h/2 there).  r2 is floored at 1e-30, where the inner
-// piece gives v = 1/2 and a zero gradient term (dx = dy = 0).
-__device__ __forceinline__ void spline_vdr_f32(float r2, float hw, float ih, float A, float B, float& v, float& dr) {
-    r2 = fmaxf(r2, 1e-30f);
-    const float rs = rsqrtf(r2);
-    const float r = r2 * rs;
-    const float t = fmaxf(fmaf(-ih, r, 1.f), 0.f);
-    const bool inner = r <= 0.5f * hw;
-    v = inner ? fmaf(r2, fmaf(A, r, B), 0.5f) : t * t * t;
-    dr = inner ? fmaf(3.f * A, r, 2.f * B) : -3.f * ih * (t * t) * rs;
+// The same for two sums at once.
+__device__ __forceinline__ void two_sum_acc2(f2x& s, f2x& e, f2x x) {
+    const f2x t = add2(s, x), bp = sub2(t, s);
+    e = add2(e, add2(sub2(s, sub2(t, bp)), sub2(x, bp)));
+    s = t;
+}
+
+// W / 2 sigma of the cubic spline and its r-derivative over r, divided by -3 / h, for
+// FP32 pairs without a branch: one reciprocal square root gives r and 1 / r; with
+// t = (1 - r/h)+ the value is min(1/2 - 3 (r/h)^2 t, t^3) (see packed_run) and the
+// derivative's pieces are (3 t - 1) / h inside r <= h / 2 (t >= 1/2) and t^2 / r
+// beyond, both exactly zero outside the support.  r2 > 0 (the caller adds 1e-30).
+__device__ __forceinline__ void spline_vdr_f32(float r2, float ih, float kap, float& v, float& dr) {
+    const float rs = wide::rsqrt_est(r2);
+    const float t = __saturatef(fmaf(-ih, r2 * rs, 1.f));
+    const float t2 = t * t;
+    v = fminf(fmaf(kap * r2, t, 0.5f), t2 * t);
+    dr = t >= 0.5f ? fmaf(3.f * ih, t, -ih) : t2 * rs;
 }
 
 // Images a sample may pair through (unbiased law): bit (sx + 1) * 3 + (sy + 1)
@@ -868,39 +876,59 @@ __device__ __forceinline__ uint32_t image_mask9(uint32_t flags) {
 // through the run's image is y + qdx, so x_p - y_s = (c - qdx) - q.
 template <typename ST, bool K9>
 __device__ __forceinline__ void scat_batch(const Cand* __restrict__ s_cand, const BatchPiece* s_bp,
-                                           const Piece* s_pc, int nbp, uint32_t btot, const float4* s_sq,
+                                           const Piece* s_pc, int nbp, const uint2* s_rng, const float4* s_sq,
                                            const uint16_t* s_sqm, int nq, const GridInst& G,
                                            double* __restrict__ out) {
     constexpr bool k32 = std::is_same<ST, float>::value;
     const int lane = threadIdx.x & 31;
     const ST hw = ST(G.hw), ih = ST(1) / hw;
     const ST A = ST(3) * ih * ih * ih, B = ST(-3) * ih * ih;
+    // the particles of the runs' parts within reach, one after the other
+    uint32_t total = 0u, off = 0u;
+    for (int k = 0; k < nbp; ++k) total += s_rng[k].y - s_rng[k].x;
     int b = 0;
-    for (uint32_t i = uint32_t(lane); i < btot; i += 32u) {
-        while (b + 1 < nbp && s_bp[b + 1].soff <= i) ++b;
+    for (uint32_t i = uint32_t(lane); i < total; i += 32u) {
+        while (i - off >= s_rng[b].y - s_rng[b].x) {
+            off += s_rng[b].y - s_rng[b].x;
+            ++b;
+        }
+        const uint32_t at = s_rng[b].x + (i - off);
         const BatchPiece bp = s_bp[b];
         const Piece pc = s_pc[bp.piece];
-        const Cand cv = s_cand[i];
+        const Cand cv = s_cand[bp.soff + at];
         const uint32_t pbit = uint32_t((pc.mx + 1) * 3 + (pc.my + 1));
         const ST cx = ST(cv.x) - ST(pc.qdx), cy = ST(cv.y) - ST(pc.qdy);
-        ST sv = ST(0), sgx = ST(0), sgy = ST(0);
-        float ev = 0.f, egx = 0.f, egy = 0.f;   // FP32 pairs: the sums' error terms
+        double gv, ggx, ggy;
         if constexpr (k32) {
+            float sv = 0.f, ev = 0.f;   // the sums and their error terms
+            f2x sg = pk2(0.f, 0.f), eg = sg;
+            const f2x C = pk2(cx, cy);
+            const float kap = G.B, m3ih = -3.f * ih;
+            const uint32_t bit = 1u << pbit;
             // branch-free: a pair outside the support or the sample's images adds
             // exact zeros, which leave the compensated sums unchanged
+#pragma unroll 4
             for (int j = 0; j < nq; ++j) {
-                const float4 q = s_sq[j];
-                float w = q.z;
-                if (K9) w = ((uint32_t(s_sqm[j]) >> pbit) & 1u) ? w : 0.f;
-                const float dx = cx - q.x, dy = cy - q.y;   // x_p - y_s
+                const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(&s_sq[j]);   // (x, y), (weight, images)
+                float w, m, dx, dy;
+                up2(q.y, w, m);
+                if (K9) w = (__float_as_uint(m) & bit) ? w : 0.f;
+                const f2x d = sub2(C, q.x);   // x_p - y_s
+                up2(d, dx, dy);
                 float v, dr;
-                spline_vdr_f32(fmaf(dx, dx, dy * dy), hw, ih, A, B, v, dr);
-                const float wdr = __fmul_rn(w, dr);
+                spline_vdr_f32(fmaf(dx, dx, fmaf(dy, dy, 1e-30f)), ih, kap, v, dr);
+                const float wdr = __fmul_rn(__fmul_rn(w, m3ih), dr);
                 two_sum_acc(sv, ev, __fmul_rn(w, v));
-                two_sum_acc(sgx, egx, __fmul_rn(wdr, dx));
-                two_sum_acc(sgy, egy, __fmul_rn(wdr, dy));
+                two_sum_acc2(sg, eg, mul2(pk2(wdr, wdr), d));
             }
+            gv = double(sv) + double(ev);
+            float gx, gy, hx, hy;
+            up2(sg, gx, gy);
+            up2(eg, hx, hy);
+            ggx = double(gx) + double(hx);
+            ggy = double(gy) + double(hy);
         } else {
+            gv = ggx = ggy = 0.0;
             for (int j = 0; j < nq; ++j) {
                 if (K9 && !((uint32_t(s_sqm[j]) >> pbit) & 1u)) continue;
                 const float4 q = s_sq[j];
@@ -918,14 +946,13 @@ __device__ __forceinline__ void scat_batch(const Cand* __restrict__ s_cand, cons
                     dr = -3.0 * t * t * ih / r;
                 }
                 const double w = double(q.z) + double(q.w);
-                sv += w * v;
-                sgx += w * dr * dx;
-                sgy += w * dr * dy;
+                gv += w * v;
+                ggx += w * dr * dx;
+                ggy += w * dr * dy;
             }
         }
-        const double gv = double(sv) + double(ev), ggx = double(sgx) + double(egx), ggy = double(sgy) + double(egy);
         if (gv != 0.0 || ggx != 0.0 || ggy != 0.0) {
-            double* o = out + 3 * (size_t(bp.gstart) + size_t(i - bp.soff));
+            double* o = out + 3 * (size_t(bp.gstart) + size_t(at));
             atomicAdd(o, gv);
             atomicAdd(o + 1, ggx);
             atomicAdd(o + 2, ggy);
@@ -933,6 +960,29 @@ __device__ __forceinline__ void scat_batch(const Cand* __restrict__ s_cand, cons
     }
 }
 
+// Value and gradient sums of NJ queries over one staged run, FP32 pairs; the
+// gradient in units of -3 / h.
+template <int NJ>
+__device__ __forceinline__ void grad32_run(const Cand* __restrict__ cs, int cnt, const f2x* pxy, const GridInst& G,
+                                           float* pv, f2x* pg) {
+    const float ih = G.inv_hw, kap = G.B;
+#pragma unroll 2
+    for (int c = 0; c < cnt; ++c) {
+        const float4 xy = *reinterpret_cast<const float4*>(&cs[c].x);   // x, x, y, y
+        const f2x C = pk2(xy.x, xy.z);
+        const float w = cs[c].w;
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+            const f2x d = sub2(pxy[j], C);   // q - c
+            float dx, dy, v, dr;             // zeros outside the support
+            up2(d, dx, dy);
+            spline_vdr_f32(fmaf(dx, dx, fmaf(dy, dy, 1e-30f)), ih, kap, v, dr);
+            const float wdr = w * dr;
+            pv[j] = fmaf(w, v, pv[j]);
+            pg[j] = fma2(pk2(wdr, wdr), d, pg[j]);
+        }
+    }
+}
 // One query's sum over one staged run to FP64 precision on the FP32 pipe (see
 // vpmc_wide.cuh): records {xh, xl, yh, yl, w, ., wl, .} already shifted by the
 // run's image.  LOW: some difference may need a second float.  A pair's error is
@@ -968,7 +1018,8 @@ __device__ __forceinline__ void wide_run(const Cand* __restrict__ cs, int cnt, f
 constexpr int eval_min_blocks(int mode, int qpt) {
     return (mode == EVAL_FIELD || mode == EVAL_FIELD9 || mode == EVAL_FIELD_F || mode == EVAL_FIELD9_F)
                ? (qpt == 4 ? 24 : qpt == 6 ? 16 : 12)
-               : (mode == EVAL_FIELD64 || mode == EVAL_FIELD9_64) ? 20 : 1;
+               : (mode == EVAL_FIELD64 || mode == EVAL_FIELD9_64) ? 20
+               : (mode == EVAL_GRAD32 || mode == EVAL_GRAD9_32) ? 16 : 1;
 }
 
 template <int MODE, int QPT>
@@ -990,7 +1041,7 @@ __global__ void __launch_bounds__(kEvalThreads, eval_min_blocks(MODE, QPT)) k_ev
     constexpr bool kF64 = MODE == EVAL_SPMV64;
     constexpr bool kComp = MODE == EVAL_SPMV32;
     constexpr bool kField64 = MODE == EVAL_FIELD64 || MODE == EVAL_FIELD9_64;
-    constexpr bool kTrim = kField64 || MODE == EVAL_FIELD || MODE == EVAL_FIELD9 || MODE == EVAL_FIELD_F ||
+    constexpr bool kTrim = kField64 || MODE == EVAL_GRAD32 || MODE == EVAL_GRAD9_32 || kScat || MODE == EVAL_FIELD || MODE == EVAL_FIELD9 || MODE == EVAL_FIELD_F ||
                            MODE == EVAL_FIELD9_F;
     // FP64 field: the item's queries and sums, slot j 32 + lane
     constexpr int kF64Q = kField64 ? kEvalThreads * QPT : 1;
@@ -1001,7 +1052,7 @@ __global__ void __launch_bounds__(kEvalThreads, eval_min_blocks(MODE, QPT)) k_ev
     constexpr bool kGrad9 = MODE == EVAL_GRAD9_64 || MODE == EVAL_GRAD9_32;
     constexpr bool kScat9 = MODE == EVAL_SCAT9_64 || MODE == EVAL_SCAT9_32;
     using ST = typename std::conditional<MODE == EVAL_SCAT32 || MODE == EVAL_SCAT9_32, float, double>::type;
-    using GT = typename std::conditional<kGrad32, float, double>::type;
+    using GT = double;
     constexpr bool kDef = eval_deformed(MODE);
     constexpr bool kDefExc = MODE == EVAL_FIELD_F_EXC;
     constexpr bool kPacked = MODE == EVAL_FIELD || MODE == EVAL_FIELD9 || MODE == EVAL_FIELD_F || MODE == EVAL_FIELD9_F;
@@ -1137,7 +1188,8 @@ __global__ void __launch_bounds__(kEvalThreads, eval_min_blocks(MODE, QPT)) k_ev
         bool qv[QPT];
         Acc acc[QPT];
         float acc_c[QPT];
-        double accg[kGrad ? QPT : 1][2];
+        double accg[kGrad && !kGrad32 ? QPT : 1][2];
+        float sums[kGrad32 ? 3 * QPT : 1][3];   // value and gradient, three floats each
 #pragma unroll
         for (int j = 0; j < QPT; ++j) {
             const uint32_t idx = uint32_t((u0 + (j >> 1)) * 64 + (j & 1) * 32 + (tid & 31));
@@ -1149,7 +1201,9 @@ __global__ void __launch_bounds__(kEvalThreads, eval_min_blocks(MODE, QPT)) k_ev
             qfl |= QFlags(r.flags & 63u) << (6 * j);
             acc[j] = Acc(0);
             acc_c[j] = 0.f;
-            if constexpr (kGrad) accg[j][0] = accg[j][1] = 0.0;
+            if constexpr (kGrad && !kGrad32) accg[j][0] = accg[j][1] = 0.0;
+            if constexpr (kGrad32)
+                for (int k = 0; k < 9; ++k) sums[3 * j + k / 3][k % 3] = 0.f;
         }
         if constexpr (kScat) {
             // the item's samples with their weights a_s 2 sigma (FP32 hi + lo)
@@ -1158,8 +1212,11 @@ __global__ void __launch_bounds__(kEvalThreads, eval_min_blocks(MODE, QPT)) k_ev
                 const QRec r = a.qrec[it.qbeg + k];
                 const double w = a.qweight[r.id] * sig2;
                 const float wh = float(w);
-                s_sq[k] = make_float4(r.x, r.y, wh, float(w - double(wh)));
-                s_sqm[k] = uint16_t(image_mask9(r.flags));
+                // FP32 pairs use the weight's first float and the images, FP64 pairs all
+                constexpr bool k32 = std::is_same<ST, float>::value;
+                const uint32_t images = image_mask9(r.flags);
+                s_sq[k] = make_float4(r.x, r.y, wh, k32 ? __uint_as_float(images) : float(w - double(wh)));
+                s_sqm[k] = uint16_t(images);
             }
             if (tid == 0 && it.qcnt > uint32_t(kScatQ)) atomicOr(a.flags, FLAG_CAPACITY);
         }
@@ -1276,8 +1333,8 @@ __global__ void __launch_bounds__(kEvalThreads, eval_min_blocks(MODE, QPT)) k_ev
 
             const int nbp = s_nbp;
             if constexpr (kScat)
-                scat_batch<ST, kScat9>(s_cand, s_bp, s_pc, nbp, s_btot, s_sq, s_sqm,
-                                       min(int(it.qcnt), kScatQ), G, a.out_f64);
+                scat_batch<ST, kScat9>(s_cand, s_bp, s_pc, nbp, s_rng[0], s_sq, s_sqm, min(int(it.qcnt), kScatQ), G,
+                                       a.out_f64);
             if constexpr (kPacked) {
                 // staged candidates -> image-shifted, bin-local coordinates + kappa c2
                 // (kappa = -3/h^2 scales every squared distance, see packed_run)
@@ -1513,9 +1570,36 @@ __global__ void __launch_bounds__(kEvalThreads, eval_min_blocks(MODE, QPT)) k_ev
                             part[j] = fmaf(cw, v, part[j]);
                         }
                     }
+                } else if constexpr (kGrad32) {
+                    const uint2 rg = s_rng[0][b];
+                    f2x pxy[QPT], pg[QPT];
+                    float pv[QPT];
+                    const float m3ih = -3.f * G.inv_hw;
+#pragma unroll
+                    for (int j = 0; j < QPT; ++j) {
+                        pxy[j] = pk2(qx[j] + pc.qdx, qy[j] + pc.qdy);
+                        pg[j] = pk2(0.f, 0.f);
+                        pv[j] = 0.f;
+                    }
+                    if (npw == 1) grad32_run<2>(cs + rg.x, int(rg.y) - int(rg.x), pxy, G, pv, pg);
+                    else grad32_run<QPT>(cs + rg.x, int(rg.y) - int(rg.x), pxy, G, pv, pg);
+#pragma unroll
+                    for (int j = 0; j < QPT; ++j) {
+                        bool use = (j >> 1) < npw;
+                        if (kGrad9) {
+                            const int mx = int(uint32_t(qfl >> (6 * j)) & 7u) - 2 + pc.mx;
+                            const int my = int(uint32_t(qfl >> (6 * j + 3)) & 7u) - 2 + pc.my;
+                            use = use && mx >= -1 && mx <= 1 && my >= -1 && my <= 1;
+                        }
+                        if (!use) continue;
+                        float gx, gy;
+                        up2(pg[j], gx, gy);
+                        wide::add_float(sums[3 * j], pv[j]);
+                        wide::add_float(sums[3 * j + 1], m3ih * gx);
+                        wide::add_float(sums[3 * j + 2], m3ih * gy);
+                    }
                 } else if constexpr (kGrad) {
-                    // value and gradient in q of sum w W(|q - c|), pair by pair in GT
-                    // (FP64, or FP32 for the FP32 path's adjoint; run sums into FP64):
+                    // value and gradient in q of sum w W(|q - c|), pair by pair in FP64:
                     // dW/dr / r = 2 sigma (3 A r + 2 B) for r < h/2, -6 sigma t^2/(h r) below h
                     const GT hw = GT(G.hw), ih = GT(1) / hw;
                     const GT A = GT(3) * ih * ih * ih, B = GT(-3) * ih * ih;
@@ -1536,20 +1620,10 @@ __global__ void __launch_bounds__(kEvalThreads, eval_min_blocks(MODE, QPT)) k_ev
                     for (int c = 0; c < cnt; ++c) {
                         const Cand cv = cs[c];
                         const GT cxd = cv.x, cyd = cv.y;
-                        const GT wd = kGrad32 ? GT(cv.w) : GT(double(cv.w) + double(cv.wl));
+                        const GT wd = GT(double(cv.w) + double(cv.wl));
 #pragma unroll
                         for (int j = 0; j < QPT; ++j) {
                             const GT dx = px[j] - cxd, dy = py[j] - cyd;   // q - c
-                            if constexpr (kGrad32) {
-                                // FP32 pairs without a branch (zeros outside the support)
-                                float v, dr;
-                                spline_vdr_f32(fmaf(dx, dx, dy * dy), hw, ih, A, B, v, dr);
-                                const float wdr = wd * dr;
-                                pv[j] = fmaf(wd, v, pv[j]);
-                                pgx[j] = fmaf(wdr, dx, pgx[j]);
-                                pgy[j] = fmaf(wdr, dy, pgy[j]);
-                                continue;
-                            }
                             const GT r2 = dx * dx + dy * dy;
                             const GT r = sqrt(r2);
                             if (r >= hw) continue;
@@ -1654,7 +1728,11 @@ __global__ void __launch_bounds__(kEvalThreads, eval_min_blocks(MODE, QPT)) k_ev
 #pragma unroll
         for (int j = 0; j < QPT && !kScat; ++j) {
             if (!qv[j]) continue;
-            if constexpr (kGrad) {
+            if constexpr (kGrad32) {
+#pragma unroll
+                for (int k = 0; k < 3; ++k)
+                    a.out_f32[3 * size_t(qid[j]) + k] = sums[3 * j + k][0] + (sums[3 * j + k][1] + sums[3 * j + k][2]);
+            } else if constexpr (kGrad) {
                 a.out_f64[3 * size_t(qid[j])] = acc[j];
                 a.out_f64[3 * size_t(qid[j]) + 1] = accg[j][0];
                 a.out_f64[3 * size_t(qid[j]) + 2] = accg[j][1];
@@ -1808,7 +1886,9 @@ int grid_sort(vpmc_context* ctx, GridBufs& g, const float2* pos, const float* om
         VPMC_LAUNCH(k_grid_keys, blocks_for(g.n), 256, 0, st, pos, omega, g.n, g.inst, g.n_inst, set_mode,
                     uint32_t(g.nbins), g.rows, g.keys);
         VPMC_TRY(radix_sort(ctx, g.keys, nullptr, g.n, bits_for(uint64_t(nsub) + 1), g.rs, &ks, &vs));
-        VPMC_LAUNCH(k_grid_starts, blocks_for(nsub + 1), 256, 0, st, ks, uint32_t(g.n), nsub, g.rows, g.start, g.cstart);
+        const int span = nsub < (1L << 20) ? 256 : 4096;
+        VPMC_LAUNCH(k_grid_starts, blocks_for(nsub + 1, span), 256, 0, st, ks, uint32_t(g.n), nsub, g.rows, span, g.start,
+                    g.cstart);
     }
     g.perm = vs;
     return VPMC_OK;

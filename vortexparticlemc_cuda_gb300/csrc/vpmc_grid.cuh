@@ -86,6 +86,11 @@ __device__ __forceinline__ f2x add2(f2x a, f2x b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
+__device__ __forceinline__ f2x sub2(f2x a, f2x b) {
+    f2x r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 __device__ __forceinline__ f2x mul2(f2x a, f2x b) {
     f2x r;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
@@ -167,8 +172,8 @@ enum EvalMode : int {
     // FP64 value and gradient (adjoint): out_f64[3 id + {0, 1, 2}] = {f, df/dqx, df/dqy}
     EVAL_GRAD64 = 10,    // f(q) = sum w W(|q - c|)
     EVAL_GRAD9_64 = 11,  // same with the FIELD9 image mask of the query
-    // the two GRAD modes with the pairs in FP32 (weights w only) and the run sums
-    // in FP64: the adjoint of the FP32-compensated step
+    // the two GRAD modes with the pairs in FP32 (weights w only), the run sums added
+    // without error and rounded once, to out_f32: the adjoint of the FP32 step
     EVAL_GRAD32 = 12,
     EVAL_GRAD9_32 = 13,
     // the transposed sums G(x_p) = sum_s a_s W(|x_p - y_s|) and its gradient,

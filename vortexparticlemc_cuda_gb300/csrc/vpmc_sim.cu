@@ -39,6 +39,7 @@
 #include <vector>
 
 #include "vpmc_sim.cuh"
+#include "vpmc_wide.cuh"
 
 namespace vpmc {
 
@@ -281,9 +282,10 @@ __global__ void __launch_bounds__(256) k_gen(GenArgs a) {
             }
         }
         if (b == kNoBin) {   // no query will write its value
-            if (a.f32) a.f32[sid] = 0.f;
-            if (a.f64)
-                for (int v = 0; v < a.nf64; ++v) a.f64[size_t(sid) * a.nf64 + v] = 0.0;
+            for (int v = 0; v < a.nval; ++v) {
+                if (a.f32) a.f32[size_t(sid) * a.nval + v] = 0.f;
+                if (a.f64) a.f64[size_t(sid) * a.nval + v] = 0.0;
+            }
         }
         a.ys[sid] = y;
         a.qbin[sid] = b;
@@ -323,21 +325,26 @@ struct AccArgs {
 // the balance-heuristic estimator with the true sampling densities for the
 // unbiased law.
 __device__ __forceinline__ float2 mis_term(int law, float2 x, float2 y, float f, float w1, float w2, float cum,
-                                           float alpha, float R, const InstMC& I) {
+                                           float inv_cum, float alpha, float R, const InstMC& I, float inv_Lx,
+                                           float inv_Ly) {
     if (!(f > 0.f)) return make_float2(0.f, 0.f);
     const float rx = x.x - y.x, ry = x.y - y.y;
     if (law == VPMC_LAW_REFERENCE) {
+        // K(x - y) f / (w1 f / cum + w2 alpha / rn) with rn the minimum-image distance,
+        // multiplied through by rn: one division a term, its quotient corrected by its
+        // residual (the separate quotients were five IEEE divisions and a root).  The
+        // image is rint(d / L) by a product: rn is the same on either side of a tie.
         float wx = rx, wy = ry;
         if (I.periodic) {
-            wx = rx - roundf(rx / I.Lx) * I.Lx;
-            wy = ry - roundf(ry / I.Ly) * I.Ly;
+            wx = fmaf(-rintf(rx * inv_Lx), I.Lx, rx);
+            wy = fmaf(-rintf(ry * inv_Ly), I.Ly, ry);
         }
         const float rn = fmaxf(sqrtf(wx * wx + wy * wy), 1e-6f);
-        const float inv_r2 = 1.f / (rx * rx + ry * ry + 1e-8f);
-        const float kx = -ry * inv_r2 / (2 * kPiF), ky = rx * inv_r2 / (2 * kPiF);
-        const float denom = w1 * f / cum + w2 * alpha / rn;
-        const float sc = f / denom;
-        return make_float2(kx * sc, ky * sc);
+        const float den = fmaf(w1 * (f * inv_cum), rn, w2 * alpha) * ((rx * rx + ry * ry + 1e-8f) * (2.f * kPiF));
+        const float num = f * rn, rc = wide::rcp_est(den);
+        float sc = num * rc;
+        sc = fmaf(fmaf(-sc, den, num), rc, sc);
+        return make_float2(-ry * sc, rx * sc);
     }
     const float r2 = rx * rx + ry * ry;
     if (!(r2 > 0.f)) return make_float2(0.f, 0.f);
@@ -375,11 +382,12 @@ __global__ void __launch_bounds__(256) k_accum(AccArgs a) {
         const InstMC& I = a.mc[inst_of(a.mc, a.n_inst, t)];
         const float2 x = a.pos[t];
         const float R = disk_radius(x, I.periodic != 0, I.Lx, I.Ly);
-        const float alpha = 1.f / (2.f * kPiF * R);
+        const float alpha = 1.f / (2.f * kPiF * R), inv_Lx = 1.f / I.Lx, inv_Ly = 1.f / I.Ly;
         float u[2][2], uc[2][2];
         for (int s = 0; s < 2; ++s) {
             KSum sx, sy;
             const long base = (tl * 2 + s) * Q;
+            const float cum = I.cum9[s], inv_cum = 1.f / cum;
             for (int j0 = sub; j0 < Q; j0 += 4 * kAccLanes) {
                 float2 y[4];
                 float f[4];
@@ -392,7 +400,7 @@ __global__ void __launch_bounds__(256) k_accum(AccArgs a) {
 #pragma unroll
                 for (int v = 0; v < 4; ++v) {
                     if (j0 + kAccLanes * v >= Q) break;
-                    const float2 c = mis_term(I.law, x, y[v], f[v], w1, w2, I.cum9[s], alpha, R, I);
+                    const float2 c = mis_term(I.law, x, y[v], f[v], w1, w2, cum, inv_cum, alpha, R, I, inv_Lx, inv_Ly);
                     sx.add(c.x);
                     sy.add(c.y);
                 }
@@ -431,10 +439,12 @@ __global__ void __launch_bounds__(256) k_accum(AccArgs a) {
     }
 }
 
-// Deformation mode: one warp per target, five estimates (C, L, R, T, B).
+// Deformation mode: five estimates per target (C, L, R, T, B), 8 lanes a target as in
+// k_accum (a warp a target spent more on its 20 five-step sums than on the terms:
+// 65,536 targets, 32 + 5 x 32 samples a sign, 798 us; 324 us this way, one division a term).
 // Branch-1 samples serve all five points, disk samples j in
 // [N1 + a N2, N1 + (a+1) N2) serve point a; the normalisation is 1/(N1+N2)
-// for each.  Lane 0 writes u = u(+) - u(-) at C (and the four auxiliary
+// for each.  A target's first lane writes u = u(+) - u(-) at C (and the four auxiliary
 // velocities), advects, and forms F_next = renorm_det1(I + dt grad u).
 struct Acc5Args {
     const InstMC* mc;
@@ -456,16 +466,21 @@ struct Acc5Args {
 
 __global__ void __launch_bounds__(256) k_accum5(Acc5Args a) {
     if (a.step && blockIdx.x == 0 && threadIdx.x == 0) *a.step += 1ull;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, sub = lane & (kAccLanes - 1), grp = lane / kAccLanes;
+    constexpr int kPerWarp = 32 / kAccLanes;
     const long warp = (long(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const long nwarps = (long(gridDim.x) * blockDim.x) >> 5;
     const int Q = a.N1 + 5 * a.N2;
     const float w1 = float(a.N1) / float(a.N1 + a.N2), w2 = float(a.N2) / float(a.N1 + a.N2);
     const float inv = 1.f / float(a.N1 + a.N2);
-    for (long tl = warp; tl < a.nt; tl += nwarps) {
-        const long t = a.t0 + tl;
+    // the loop runs the same trips in every lane of a warp (the group sums shuffle)
+    for (long tw = warp * kPerWarp; tw < a.nt; tw += nwarps * kPerWarp) {
+        const long tl = tw + grp;
+        const bool live = tl < a.nt;
+        const long t = a.t0 + (live ? tl : tw);
         const InstMC& I = a.mc[inst_of(a.mc, a.n_inst, t)];
         const float2 x = a.pos[t];
+        const float inv_Lx = 1.f / I.Lx, inv_Ly = 1.f / I.Ly;
         float2 xa[5];
         float R[5], alpha[5];
 #pragma unroll
@@ -475,15 +490,18 @@ __global__ void __launch_bounds__(256) k_accum5(Acc5Args a) {
             alpha[k] = 1.f / (2.f * kPiF * R[k]);
         }
         float u[5][2], su[2][5][2], cu[2][5][2];
+#pragma unroll
         for (int s = 0; s < 2; ++s) {
             KSum sx[5], sy[5];
             const long base = (tl * 2 + s) * Q;
-            for (int j = lane; j < a.N1; j += 32) {
-                const float2 y = a.ys[base + j];
-                const float f = a.fv[base + j];
+            const float cum = I.cum9[s], inv_cum = 1.f / cum;
+#pragma unroll 2
+            for (int j = sub; j < a.N1; j += kAccLanes) {
+                const float2 y = live ? a.ys[base + j] : make_float2(0.f, 0.f);
+                const float f = live ? a.fv[base + j] : 0.f;
 #pragma unroll
                 for (int k = 0; k < 5; ++k) {
-                    const float2 c = mis_term(I.law, xa[k], y, f, w1, w2, I.cum9[s], alpha[k], R[k], I);
+                    const float2 c = mis_term(I.law, xa[k], y, f, w1, w2, cum, inv_cum, alpha[k], R[k], I, inv_Lx, inv_Ly);
                     sx[k].add(c.x);
                     sy[k].add(c.y);
                 }
@@ -491,17 +509,19 @@ __global__ void __launch_bounds__(256) k_accum5(Acc5Args a) {
 #pragma unroll
             for (int k = 0; k < 5; ++k) {
                 const long b0 = base + a.N1 + long(k) * a.N2;
-                for (int j = lane; j < a.N2; j += 32) {
-                    const float2 c = mis_term(I.law, xa[k], a.ys[b0 + j], a.fv[b0 + j], w1, w2, I.cum9[s], alpha[k],
-                                              R[k], I);
+#pragma unroll 2
+                for (int j = sub; j < a.N2; j += kAccLanes) {
+                    const float2 y = live ? a.ys[b0 + j] : make_float2(0.f, 0.f);
+                    const float f = live ? a.fv[b0 + j] : 0.f;
+                    const float2 c = mis_term(I.law, xa[k], y, f, w1, w2, cum, inv_cum, alpha[k], R[k], I, inv_Lx, inv_Ly);
                     sx[k].add(c.x);
                     sy[k].add(c.y);
                 }
             }
 #pragma unroll
             for (int k = 0; k < 5; ++k) {
-                group_sum_comp_pair<32>(sx[k].s, sx[k].c);
-                group_sum_comp_pair<32>(sy[k].s, sy[k].c);
+                group_sum_comp_pair<kAccLanes>(sx[k].s, sx[k].c);
+                group_sum_comp_pair<kAccLanes>(sy[k].s, sy[k].c);
                 su[s][k][0] = sx[k].s;
                 cu[s][k][0] = sx[k].c;
                 su[s][k][1] = sy[k].s;
@@ -512,7 +532,7 @@ __global__ void __launch_bounds__(256) k_accum5(Acc5Args a) {
         for (int k = 0; k < 5; ++k)
 #pragma unroll
             for (int d = 0; d < 2; ++d) u[k][d] = comp_diff(su[0][k][d], cu[0][k][d], su[1][k][d], cu[1][k][d]) * inv;
-        if (lane == 0) {
+        if (live && sub == 0) {
             const float vx = u[0][0], vy = u[0][1];
             a.vel[t] = make_float2(vx, vy);
 #pragma unroll
@@ -903,7 +923,7 @@ int issue_pass(vpmc_sim* s, bool advect, bool timed, int* nlaunch) {
         if (def) {
             Acc5Args aa{s->d_mc, s->n_inst, s->pos, s->ys, s->fv, t0, nt, s->N1, s->N2, advect ? 1 : 0, s->vel,
                         s->vel5, pos_out, F_out, s->d_sig, kCoverCap, count_step};
-            VPMC_LAUNCH(k_accum5, blocks_for(nt * 32), 256, 0, st, aa);
+            VPMC_LAUNCH(k_accum5, blocks_for(nt * kAccLanes), 256, 0, st, aa);
         } else if (f64) {
             AccArgs64 aa{s->d_mc, s->n_inst, s->pos, s->ys, s->fv64, s->cum64, t0, nt, s->N1, s->N2, advect ? 1 : 0,
                          s->vel, pos_out, count_step};

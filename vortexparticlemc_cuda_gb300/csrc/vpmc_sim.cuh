@@ -38,14 +38,10 @@ __device__ __forceinline__ int inst_of(const InstMC* I, int n, long t) {
 // SamplingDiskRadius (include/monte_carlo_bs.hpp:73-89), same FP32 steps.
 __host__ __device__ __forceinline__ float disk_radius(float2 d, bool periodic, float Lx, float Ly) {
     if (!periodic) return sqrtf(Lx * Lx + Ly * Ly);
-    float m = 0.f;
-    for (int dx = -1; dx <= 1; ++dx)
-        for (int dy = -1; dy <= 1; ++dy) {
-            const float ix = d.x + dx * Lx, iy = d.y + dy * Ly;
-            const float ex = ix - d.x, ey = iy - d.y;
-            m = fmaxf(m, ex * ex + ey * ey);
-        }
-    return sqrtf(m);
+    // the farthest of the nine images: the larger shift on each axis (FP32 differences)
+    const float xp = (d.x + Lx) - d.x, xm = (d.x - Lx) - d.x, yp = (d.y + Ly) - d.y, ym = (d.y - Ly) - d.y;
+    const float ex = fmaxf(fabsf(xp), fabsf(xm)), ey = fmaxf(fabsf(yp), fabsf(ym));
+    return sqrtf(ex * ex + ey * ey);
 }
 
 struct GenArgs {
@@ -69,9 +65,9 @@ struct GenArgs {
     uint32_t* qcount;
     uint32_t* qsub;               // counts per (bin, sub-cell), or nullptr: per bin in qcount
     uint32_t* qrank;              // with each sample's rank there << 4 | sub-cell, or nullptr
-    float* f32;                   // field values and (adjoint) FP64 values: zeroed where a sample is dropped
+    float* f32;                   // the samples' values, in FP32 or FP64: zeroed where a sample is dropped
     double* f64;
-    int nf64;                     // FP64 values a sample
+    int nval;                     // values a sample (1, or 3 with the gradient)
 };
 
 // One thread per (target, sign, sample): Philox draw, branch-1 CDF / image /

@@ -177,6 +177,14 @@ VPMC_WIDE_FN W3 sqrt3(const W3& x) {
     return norm3(W3{g, c0, c1});
 }
 
+// x added to a sum of three floats, which keeps more digits than an FP64 sum does.
+VPMC_WIDE_FN void add_float(float (&s)[3], float x) {
+    float e, f;
+    two_sum(s[0], x, s[0], e);
+    two_sum(s[1], e, s[1], f);
+    s[2] = add(s[2], f);
+}
+
 // h^3 W(r) / (2 sigma) of the cubic spline at r^2 = r2 < h^2 (h a float, half_h3 =
 // h^3 / 2 as a wide number): with t = h - r,
 //   r > h / 2:   t^3
