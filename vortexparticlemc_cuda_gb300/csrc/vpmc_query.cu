@@ -200,7 +200,9 @@ int vpmc_query_vorticity(vpmc_context* ctx, int N, const float* pos, const float
     }
     const int set_mode = sign > 0 ? SET_POS_ONLY
                                    : (sign < 0 ? SET_NEG_ONLY : (use_signed ? SET_ONE_SIGNED : SET_ONE_ABS));
-    if (!F && double(M) <= kGatherPoints * (2.0 * Lx / h_w) * (2.0 * Ly / h_w)) {
+    // (the gathered form has no staging wait to give up: a limit of 0 polls keeps the
+    // binned one, whose first wait then expires)
+    if (!F && ctx->wait_limit > 0 && double(M) <= kGatherPoints * (2.0 * Lx / h_w) * (2.0 * Ly / h_w)) {
         VPMC_TRY(query_gather(ctx, N, reinterpret_cast<const float2*>(pos), omega, M, reinterpret_cast<const float2*>(pts),
                               set_mode, exclude_center != 0, h_w, Lx, Ly, periodic, out));
         if (sign < 0 && use_signed) VPMC_LAUNCH(k_scale_f32, work_blocks(M), 256, 0, st, out, long(M), -1.0f);
