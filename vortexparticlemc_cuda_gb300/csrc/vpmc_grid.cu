@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(256) k_grid_starts(const uint32_t* __restrict_
 __global__ void k_grid_gather(const uint32_t* __restrict__ perm, const uint32_t* __restrict__ start, long n,
                               uint32_t nbins, const float2* __restrict__ pos, const float* __restrict__ omega,
                               const GridInst* __restrict__ inst, int n_inst, int set_mode,
-                              Cand* __restrict__ cand) {
+                              Cand* __restrict__ cand, float4* __restrict__ cand4) {
     const long nv = start[nbins];
     for (long p = long(blockIdx.x) * blockDim.x + threadIdx.x; p < nv && p < n; p += long(gridDim.x) * blockDim.x) {
         const uint32_t i = perm[p];
@@ -130,7 +130,8 @@ __global__ void k_grid_gather(const uint32_t* __restrict__ perm, const uint32_t*
         // weight 2 sigma |omega| (or 2 sigma omega), FP32 hi part + remainder
         const double wd = double(set_mode == SET_ONE_SIGNED ? w : fabsf(w)) * (80.0 / (7.0 * kPiD * double(G.hw) * G.hw));
         const float wt = float(wd);
-        cand[p] = Cand{q.x, q.x, q.y, q.y, wt, wt, float(wd - double(wt)), 0.f};
+        if (cand) cand[p] = Cand{q.x, q.x, q.y, q.y, wt, wt, float(wd - double(wt)), 0.f};
+        if (cand4) cand4[p] = make_float4(q.x, q.y, wt, 0.f);
     }
 }
 
@@ -511,7 +512,7 @@ __global__ void __launch_bounds__(kPlaceThreads) k_scatter_window(const uint4* _
 __global__ void __launch_bounds__(kAsmThreads, 2) k_scatter_assemble(const uint4* __restrict__ tmp2, long nbins, int wshift,
                                                             const uint32_t* __restrict__ qstart,
                                                             const GridInst* __restrict__ inst, int n_inst,
-                                                            QRec* __restrict__ qrec) {
+                                                            QRec* __restrict__ qrec, uint32_t* __restrict__ sstart) {
     constexpr int kPer = kWinCap / kAsmThreads;     // records per thread of a window that fits
     extern __shared__ __align__(16) QRec buf[];   // kWinCap records
     __shared__ uint32_t cnt[kWinBinsMax];
@@ -520,6 +521,7 @@ __global__ void __launch_bounds__(kAsmThreads, 2) k_scatter_assemble(const uint4
     const long nwin = ((nbins - 1) >> wshift) + 1;
     long w = blockIdx.x;
     if (w >= nwin) return;
+    if (sstart && w == 0 && threadIdx.x == 0) sstart[size_t(nbins) * kSubCells] = qstart[nbins];
     // window w's bounds and (when it fits) its records: loaded one window ahead,
     // so the loads overlap the previous window's write-out
     long b0 = w << wshift, b1 = min(nbins, b0 + (1L << wshift));
@@ -545,10 +547,13 @@ __global__ void __launch_bounds__(kAsmThreads, 2) k_scatter_assemble(const uint4
         }
         for (uint32_t i = threadIdx.x; i < uint32_t(kSubCells) * nb; i += blockDim.x) sub[i] = 0u;
         __syncthreads();
+        // inside each bin the records are ordered by sub-cell, so that consecutive
+        // queries of a bin lie close together (a window of several bins that does not fit
+        // only where boxes need the order: ordering it from global memory costs more
+        // than the closer queries save)
+        const bool order = fits || sstart || nb == 1u;
+        uint32_t kr[kPer];   // bin in the window | sub-cell << 8 | rank within (sub-cell, bin) << 12
         if (fits) {
-            // inside each bin the records are ordered by sub-cell, so that
-            // consecutive queries of a bin lie close together
-            uint32_t kr[kPer];   // bin in the window | sub-cell << 8 | rank within (sub-cell, bin) << 12
 #pragma unroll
             for (int j = 0; j < kPer; ++j) {
                 const uint32_t k = threadIdx.x + uint32_t(j) * uint32_t(kAsmThreads);
@@ -559,24 +564,36 @@ __global__ void __launch_bounds__(kAsmThreads, 2) k_scatter_assemble(const uint4
                 kr[j] = bl | (key << 8) | (atomicAdd(&sub[key * nb + bl], 1u) << 12);
                 r[j] = make_uint4(__float_as_uint(q.x), __float_as_uint(q.y), q.id, q.flags);
             }
-            __syncthreads();
-            // each bin's 16 sub-cell counters -> first slots, by warp 0: two bins
-            // per pass, one counter per lane, a scan inside each 16-lane half
-            if (threadIdx.x < 32) {
-                const uint32_t lane = threadIdx.x, c = lane & 15u;
-                for (uint32_t b = lane >> 4; b < ((nb + 1u) & ~1u); b += 2u) {
-                    const bool live = b < nb;
-                    const uint32_t n = live ? sub[c * nb + b] : 0u;
-                    uint32_t incl = n;
+        } else if (order) {   // a window that does not fit is counted, then placed, from global memory
+            for (uint32_t k = threadIdx.x; k < nw; k += blockDim.x) {
+                const uint4 rr = tmp2[start + k];
+                const uint32_t bl = rr.w - uint32_t(b0);
+                const QRec q = make_qrec(rr, inst, n_inst);
+                atomicAdd(&sub[subcell_key(q.x, q.y, corg[bl]) * nb + bl], 1u);
+            }
+        }
+        __syncthreads();
+        // each bin's 16 sub-cell counters -> first slots, by warp 0: two bins
+        // per pass, one counter per lane, a scan inside each 16-lane half
+        if (threadIdx.x < 32 && order) {
+            const uint32_t lane = threadIdx.x, c = lane & 15u;
+            for (uint32_t b = lane >> 4; b < ((nb + 1u) & ~1u); b += 2u) {
+                const bool live = b < nb;
+                const uint32_t n = live ? sub[c * nb + b] : 0u;
+                uint32_t incl = n;
 #pragma unroll
-                    for (int o = 1; o < 16; o <<= 1) {
-                        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o, 16);
-                        if (c >= uint32_t(o)) incl += y;
-                    }
-                    if (live) sub[c * nb + b] = cnt[b] + incl - n;
+                for (int o = 1; o < 16; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o, 16);
+                    if (c >= uint32_t(o)) incl += y;
+                }
+                if (live) {
+                    sub[c * nb + b] = cnt[b] + incl - n;
+                    if (sstart) sstart[(size_t(b0) + b) * kSubCells + c] = cnt[b] + incl - n;
                 }
             }
-            __syncthreads();
+        }
+        __syncthreads();
+        if (fits) {
 #pragma unroll
             for (int j = 0; j < kPer; ++j) {
                 const uint32_t k = threadIdx.x + uint32_t(j) * uint32_t(kAsmThreads);
@@ -587,8 +604,9 @@ __global__ void __launch_bounds__(kAsmThreads, 2) k_scatter_assemble(const uint4
         } else {
             for (uint32_t k = threadIdx.x; k < nw; k += blockDim.x) {
                 const uint4 rr = tmp2[start + k];
-                const uint32_t slot = atomicAdd(&cnt[rr.w - uint32_t(b0)], 1u);
-                qrec[slot] = make_qrec(rr, inst, n_inst);
+                const uint32_t bl = rr.w - uint32_t(b0);
+                const QRec q = make_qrec(rr, inst, n_inst);
+                qrec[atomicAdd(order ? &sub[subcell_key(q.x, q.y, corg[bl]) * nb + bl] : &cnt[bl], 1u)] = q;
             }
         }
         __syncthreads();
@@ -615,22 +633,77 @@ __global__ void __launch_bounds__(kAsmThreads, 2) k_scatter_assemble(const uint4
     }
 }
 
+// skip: bins of boxed instances get no items here.
 __global__ void k_items_count(const uint32_t* __restrict__ qstart, long nbins, int chunk,
-                              uint32_t* __restrict__ per_bin) {
+                              const GridInst* __restrict__ inst, int n_inst, int skip, uint32_t* __restrict__ per_bin) {
     for (long b = long(blockIdx.x) * blockDim.x + threadIdx.x; b < nbins; b += long(gridDim.x) * blockDim.x) {
-        const uint32_t c = qstart[b + 1] - qstart[b];
+        uint32_t c = qstart[b + 1] - qstart[b];
+        if (skip && inst[inst_of_bin(inst, n_inst, uint32_t(b))].nb) c = 0u;
         per_bin[b] = (c + chunk - 1) / chunk;
+    }
+}
+
+// First slot of each (bin, sub-cell) from the counts and the bins' starts.
+__global__ void k_sub_starts(const uint32_t* __restrict__ qsub, const uint32_t* __restrict__ qstart, long nbins,
+                             uint32_t* __restrict__ sstart) {
+    for (long b = long(blockIdx.x) * blockDim.x + threadIdx.x; b < nbins; b += long(gridDim.x) * blockDim.x) {
+        uint32_t s = qstart[b];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint4 c = reinterpret_cast<const uint4*>(qsub)[4 * b + i];
+            reinterpret_cast<uint4*>(sstart)[4 * b + i] = make_uint4(s, s + c.x, s + c.x + c.y, s + c.x + c.y + c.z);
+            s += c.x + c.y + c.z + c.w;
+        }
+        if (b == nbins - 1) sstart[nbins * kSubCells] = s;
+    }
+}
+
+// Items of the boxes (aligned groups of sub-cells) of boxed instances.
+__global__ void k_box_count(const uint32_t* __restrict__ sstart, long nbins, const GridInst* __restrict__ inst, int n_inst,
+                            uint32_t* __restrict__ per_bin) {
+    for (long b = long(blockIdx.x) * blockDim.x + threadIdx.x; b < nbins; b += long(gridDim.x) * blockDim.x) {
+        const int nb = inst[n_inst == 1 ? 0 : inst_of_bin(inst, n_inst, uint32_t(b))].nb;
+        uint32_t t = 0u;
+        if (nb) {
+            const int per = kSubCells / (nb * nb);
+            for (int s = 0; s < kSubCells; s += per)
+                t += (sstart[b * kSubCells + s + per] - sstart[b * kSubCells + s] + kBoxChunk - 1) / kBoxChunk;
+        }
+        per_bin[b] = t;
+    }
+}
+__global__ void k_box_fill(const uint32_t* __restrict__ sstart, long nbins, const uint32_t* __restrict__ item_start,
+                           const GridInst* __restrict__ inst, int n_inst, Item* __restrict__ items,
+                           uint32_t* __restrict__ n_items, uint32_t* __restrict__ counter, long max_items) {
+    for (long b = long(blockIdx.x) * blockDim.x + threadIdx.x; b < nbins; b += long(gridDim.x) * blockDim.x) {
+        const uint32_t ib = n_inst == 1 ? 0u : uint32_t(inst_of_bin(inst, n_inst, uint32_t(b)));
+        const int nb = inst[ib].nb;
+        if (!nb) continue;
+        const int per = kSubCells / (nb * nb);
+        uint32_t it = item_start[b];
+        for (int s = 0; s < kSubCells; s += per) {
+            const uint32_t q0 = sstart[b * kSubCells + s], c = sstart[b * kSubCells + s + per] - q0;
+            for (uint32_t o = 0; o < c; o += kBoxChunk, ++it)
+                if (it < max_items)
+                    items[it] = Item{uint32_t(b), q0 + o, min(uint32_t(kBoxChunk), c - o) | (uint32_t(s / per) << 16), ib};
+        }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        const uint32_t t = item_start[nbins];
+        *n_items = t < max_items ? t : uint32_t(max_items);
+        *counter = 0;
     }
 }
 
 __global__ void k_items_fill(const uint32_t* __restrict__ qstart, long nbins, int chunk,
                              const uint32_t* __restrict__ item_start, const GridInst* __restrict__ inst,
-                             int n_inst, Item* __restrict__ items, uint32_t* __restrict__ n_items,
+                             int n_inst, int skip, Item* __restrict__ items, uint32_t* __restrict__ n_items,
                              uint32_t* __restrict__ counter, long max_items) {
     for (long b = long(blockIdx.x) * blockDim.x + threadIdx.x; b < nbins; b += long(gridDim.x) * blockDim.x) {
         const uint32_t q0 = qstart[b], c = qstart[b + 1] - q0;
         uint32_t it = item_start[b];
         const uint32_t ib = uint32_t(inst_of_bin(inst, n_inst, uint32_t(b)));
+        if (skip && inst[ib].nb) continue;
         for (uint32_t o = 0; o < c; o += chunk, ++it)
             if (it < max_items) items[it] = Item{uint32_t(b), q0 + o, min(uint32_t(chunk), c - o), ib};
     }
@@ -672,7 +745,7 @@ __device__ __forceinline__ uint32_t scan_1024(uint32_t v, uint32_t* s_warp, uint
 }
 
 __global__ void __launch_bounds__(1024) k_items_small(const uint32_t* __restrict__ qsub, uint32_t* qstart, int nbins,
-                                                      int chunk, const GridInst* __restrict__ inst, int n_inst,
+                                                      int chunk, const GridInst* __restrict__ inst, int n_inst, int skip,
                                                       Item* __restrict__ items, uint32_t* __restrict__ n_items,
                                                       uint32_t* __restrict__ counter, long max_items) {
     __shared__ uint32_t s_warp[32];
@@ -699,10 +772,13 @@ __global__ void __launch_bounds__(1024) k_items_small(const uint32_t* __restrict
         if (threadIdx.x == 0) qstart[nbins] = total;
         __syncthreads();   // the starts are read back by the threads of this CTA
     }
+    auto boxed = [&](int b) { return skip && inst[n_inst > 1 ? inst_of_bin(inst, n_inst, uint32_t(b)) : 0].nb != 0; };
     uint32_t sum = 0u;
-    for (int b = b0; b < b1; ++b) sum += (qstart[b + 1] - qstart[b] + uint32_t(chunk) - 1u) / uint32_t(chunk);
+    for (int b = b0; b < b1; ++b)
+        if (!boxed(b)) sum += (qstart[b + 1] - qstart[b] + uint32_t(chunk) - 1u) / uint32_t(chunk);
     uint32_t it = scan_1024(sum, s_warp, &total);
     for (int b = b0; b < b1; ++b) {
+        if (boxed(b)) continue;
         const uint32_t q0 = qstart[b], c = qstart[b + 1] - q0;
         const uint32_t ib = c && n_inst > 1 ? uint32_t(inst_of_bin(inst, n_inst, uint32_t(b))) : 0u;
         for (uint32_t o = 0; o < c; o += uint32_t(chunk), ++it)
@@ -744,47 +820,6 @@ struct EvalArgs {
     uint32_t wait_limit;      // polls of a staging wait before the kernel gives up
     const double* qweight;    // SCAT modes: the weight of each query (by id)
 };
-
-// Sum over one staged run of candidates for NPR packed query pairs, in
-// bin-local coordinates, every squared distance pre-scaled by kappa = -3/h^2:
-// candidates hold (x, y) relative to the bin centre and kappa c2; queries
-// enter as -2 kappa q and kappa |q|^2, so
-//   s2 = kappa c2 + kappa q2 - 2 kappa c.q = -3 (r/h)^2,   sqrt(|s2|) = sqrt(3) r/h
-//   t  = saturate(1 - sqrt(|s2|)/sqrt(3))                  (= max(1 - r/h, 0))
-//   P += w * min(0.5 + s2 t, t^3)                          (= w W / 2 sigma)
-// because the spline's inner branch 1/2 - 3 q^2 + 3 q^3 is 1/2 - 3 q^2 (1 - q),
-// and beyond the support t = 0 leaves min(1/2, 0) = 0.
-// Per pair of queries: 7 packed FMA-pipe operations + 2 saturating scalar FMAs,
-// 2 square roots on the XU and 2 min on the ALU.  The candidate loop is unrolled
-// eight times (independent chains across candidates, 80 registers; at tg2048
-// 257.7 ms per evaluation against 261.1 unrolled four times, 274.4 twice,
-// 272.5 twelve times, 258.4 sixteen times).
-template <int NPR, int NPMAX>
-__device__ __forceinline__ void packed_run(const Cand* __restrict__ cs, int cnt, const f2x (&QX)[NPMAX],
-                                           const f2x (&QY)[NPMAX], const f2x (&Q2)[NPMAX], f2x (&P)[NPMAX]) {
-    const f2x HALF = pk2(0.5f, 0.5f);
-#pragma unroll 8
-    for (int c = 0; c < cnt; ++c) {
-        const ulonglong2 XY = *reinterpret_cast<const ulonglong2*>(&cs[c].x);
-        const ulonglong2 WC = *reinterpret_cast<const ulonglong2*>(&cs[c].w);   // (w, w), (kappa c2, kappa c2)
-#pragma unroll
-        for (int pr = 0; pr < NPR; ++pr) {
-            const f2x s = add2(WC.y, Q2[pr]);
-            const f2x s2 = fma2(XY.y, QY[pr], fma2(XY.x, QX[pr], s));
-            float ra, rb;
-            up2(s2, ra, rb);
-            // rounding can leave s2 a hair above 0 when c ~ q: take sqrt(|s2|)
-            const float sa = sqrt_approx(fabsf(ra)), sb = sqrt_approx(fabsf(rb));
-            const f2x t = pk2(__saturatef(fmaf(-kInvSqrt3, sa, 1.f)), __saturatef(fmaf(-kInvSqrt3, sb, 1.f)));
-            const f2x in = fma2(s2, t, HALF);
-            const f2x t3 = mul2(mul2(t, t), t);
-            float ia, ib, ta, tb;
-            up2(in, ia, ib);
-            up2(t3, ta, tb);
-            P[pr] = fma2(WC.x, pk2(fminf(ia, ta), fminf(ib, tb)), P[pr]);
-        }
-    }
-}
 
 // The same sum for deformed kernels: s2 from the expanded metric form, its
 // coefficients pre-scaled by kappa (5 packed FMAs instead of 3), the spline as above.
@@ -1790,7 +1825,7 @@ int default_k() { return 2; }
 // ensemble members, h_w 8: 27.0 -> 25.5 (3); 256^2, h_w 4, 16 + 16: 0.52 -> 0.50 (1).
 // The rule looks at one instance alone, so that a member of an ensemble sums as a
 // run of its own does.
-int sample_k(long n, double samples, float Lx, float Ly, float hw) {
+int sample_k(long n, double samples, float Lx, float Ly, float hw, bool boxes) {
     if (n < 1) return default_k();
     const double spacing = std::sqrt(double(Lx) * Ly / double(n));
     int k = int(std::lround(double(hw) / (2.6 * spacing)));
@@ -1798,6 +1833,16 @@ int sample_k(long n, double samples, float Lx, float Ly, float hw) {
     for (; k > 1; --k) {
         const double cells = double(k) * Lx / hw * (double(k) * Ly / hw);
         if (samples >= 150.0 * cells && cells <= double(1L << 22)) break;
+    }
+    // where the pairwise choice has boxes too thin for local expansions, 7 cells may not:
+    // their quadrants (h_w / 14 a side) are the largest boxes the expansions take
+    // (512^2, h_w 16, 32 + 32 samples: a step takes 10.3 ms with 6 cells pair by pair, 5.8 with 7)
+    if (boxes) {
+        auto split = [&](int kk) {
+            const double gx = std::floor(double(kk) * Lx / hw + 1e-9), gy = std::floor(double(kk) * Ly / hw + 1e-9);
+            return gx >= 1.0 && gy >= 1.0 && gx * gy <= double(1L << 22) ? box_split(n, samples, Lx, Ly, hw, int(gx), int(gy)) : 0;
+        };
+        if (!split(k) && split(7)) return 7;
     }
     return k;
 }
@@ -1895,7 +1940,7 @@ int grid_sort(vpmc_context* ctx, GridBufs& g, const float2* pos, const float* om
 }
 
 int grid_build(vpmc_context* ctx, GridBufs& g, const float2* pos, const float* omega, int set_mode,
-               const float4* F) {
+               const float4* F, bool compact) {
     if (F && !g.candf) return VPMC_ERR_INVALID;
     cudaStream_t st = ctx->stream;
     VPMC_TRY(grid_sort(ctx, g, pos, omega, set_mode));
@@ -1906,7 +1951,7 @@ int grid_build(vpmc_context* ctx, GridBufs& g, const float2* pos, const float* o
                     g.inst, g.n_inst, set_mode, g.candf);
     else
         VPMC_LAUNCH(k_grid_gather, blocks_for(g.n), 256, 0, st, vs, g.start, g.n, uint32_t(nsub), pos, omega,
-                    g.inst, g.n_inst, set_mode, g.cand);
+                    g.inst, g.n_inst, set_mode, g.cand, compact ? g.cand4 : nullptr);
     return VPMC_OK;
 }
 
@@ -1929,8 +1974,8 @@ int grid_max_sigma(vpmc_context* ctx, const float4* F, long n, unsigned* d_words
     return VPMC_OK;
 }
 
-void carve_items(Carver& c, long nbins, long max_queries, ItemBufs* it) {
-    it->max_items = max_queries / query_chunk(1) + nbins + 1;
+void carve_items(Carver& c, long nbins, long max_queries, ItemBufs* it, long n_boxes) {
+    it->max_items = max_queries / query_chunk(1) + (n_boxes < 0 ? nbins : n_boxes) + 1;
     it->items = c.take<Item>(size_t(it->max_items));
     it->n_items = c.take<uint32_t>(1);
     it->counter = c.take<uint32_t>(1);
@@ -1939,18 +1984,33 @@ void carve_items(Carver& c, long nbins, long max_queries, ItemBufs* it) {
     it->scan_tmp = c.take<uint32_t>(scan_tmp_elems(nbins + 1) + 1);
 }
 
-int make_items(vpmc_context* ctx, const GridBufs& g, const uint32_t* qstart, ItemBufs& it, int chunk, long queries) {
+namespace {
+int make_items_of(vpmc_context* ctx, const GridBufs& g, const uint32_t* qstart, ItemBufs& it, int chunk, long queries,
+                  int skip) {
     cudaStream_t st = ctx->stream;
     if (items_in_one(g.nbins, queries)) {
         VPMC_LAUNCH(k_items_small, 1, 1024, 0, st, static_cast<const uint32_t*>(nullptr), const_cast<uint32_t*>(qstart),
-                    int(g.nbins), chunk, g.inst, g.n_inst, it.items, it.n_items, it.counter, it.max_items);
+                    int(g.nbins), chunk, g.inst, g.n_inst, skip, it.items, it.n_items, it.counter, it.max_items);
         return VPMC_OK;
     }
-    VPMC_LAUNCH(k_items_count, blocks_for(g.nbins), 256, 0, st, qstart, g.nbins, chunk, it.per_bin);
+    VPMC_LAUNCH(k_items_count, blocks_for(g.nbins), 256, 0, st, qstart, g.nbins, chunk, g.inst, g.n_inst, skip, it.per_bin);
     VPMC_TRY(exclusive_scan(ctx, it.per_bin, it.item_start, g.nbins, it.scan_tmp, true));
     VPMC_LAUNCH(k_items_fill, blocks_for(g.nbins), 256, 0, st, qstart, g.nbins, chunk, it.item_start, g.inst,
-                g.n_inst, it.items, it.n_items, it.counter, it.max_items);
+                g.n_inst, skip, it.items, it.n_items, it.counter, it.max_items);
     return VPMC_OK;
+}
+int make_box_items(vpmc_context* ctx, const GridBufs& g, const uint32_t* sstart, ItemBufs& it) {
+    cudaStream_t st = ctx->stream;
+    VPMC_LAUNCH(k_box_count, blocks_for(g.nbins), 256, 0, st, sstart, g.nbins, g.inst, g.n_inst, it.per_bin);
+    VPMC_TRY(exclusive_scan(ctx, it.per_bin, it.item_start, g.nbins, it.scan_tmp, true));
+    VPMC_LAUNCH(k_box_fill, blocks_for(g.nbins), 256, 0, st, sstart, g.nbins, it.item_start, g.inst, g.n_inst, it.items,
+                it.n_items, it.counter, it.max_items);
+    return VPMC_OK;
+}
+}  // namespace
+
+int make_items(vpmc_context* ctx, const GridBufs& g, const uint32_t* qstart, ItemBufs& it, int chunk, long queries) {
+    return make_items_of(ctx, g, qstart, it, chunk, queries, 0);
 }
 
 // Samples are placed directly up to this many a chunk (the records in L2), in
@@ -1960,7 +2020,7 @@ constexpr long kDirectSamples = 1L << 21;
 // Up to this many bins (32 MB of counters) the generator counts per (bin, sub-cell).
 constexpr long kSubBins = 1L << 19;
 
-void carve_queries(Carver& c, long nbins, long max_points, QueryBufs* q, bool samples) {
+void carve_queries(Carver& c, long nbins, long max_points, QueryBufs* q, bool samples, bool boxes) {
     const size_t m = size_t(max_points < 1 ? 1 : max_points);
     const bool sub = samples && nbins <= kSubBins, direct = sub && max_points <= kDirectSamples;
     const bool staged = samples && !direct;
@@ -1976,6 +2036,7 @@ void carve_queries(Carver& c, long nbins, long max_points, QueryBufs* q, bool sa
     q->clear = counts;
     q->n_clear = n_sub + n_fill + (sub ? 0 : n_count);
     q->qstart = c.take<uint32_t>(size_t(nbins + 1));
+    q->sstart = boxes ? c.take<uint32_t>(size_t(nbins) * kSubCells + 1) : nullptr;
     q->qfill = samples ? nullptr : c.take<uint32_t>(size_t(nbins + 1));
     q->qrank = direct ? c.take<uint32_t>(m) : nullptr;
     q->qrec = c.take<QRec>(m);
@@ -2000,20 +2061,24 @@ int clear_counts(vpmc_context* ctx, QueryBufs& q) {
 }
 
 int place_samples(vpmc_context* ctx, const GridBufs& g, QueryBufs& q, const float2* pts, long M, ItemBufs& it,
-                  int chunk) {
+                  int chunk, ItemBufs* boxes) {
     cudaStream_t st = ctx->stream;
+    const int skip = boxes ? 1 : 0;
+    if (boxes && !q.sstart) return VPMC_ERR_INVALID;
     if (q.qrank && items_in_one(g.nbins, M)) {
-        VPMC_LAUNCH(k_items_small, 1, 1024, 0, st, q.qsub, q.qstart, int(g.nbins), chunk, g.inst, g.n_inst, it.items,
+        VPMC_LAUNCH(k_items_small, 1, 1024, 0, st, q.qsub, q.qstart, int(g.nbins), chunk, g.inst, g.n_inst, skip, it.items,
                     it.n_items, it.counter, it.max_items);
     } else {
         if (q.qsub) VPMC_LAUNCH(k_bin_totals, blocks_for(g.nbins), 256, 0, st, q.qsub, g.nbins, q.qcount);
         VPMC_TRY(exclusive_scan(ctx, q.qcount, q.qstart, g.nbins, q.scan_tmp, true));
-        VPMC_TRY(make_items(ctx, g, q.qstart, it, chunk, M));
+        VPMC_TRY(make_items_of(ctx, g, q.qstart, it, chunk, M, skip));
     }
     if (q.qrank) {
         VPMC_LAUNCH(k_place_direct, blocks_for(M), 256, 0, st, pts, M, g.inst, g.n_inst, q.qbin, q.qrank, q.qstart, q.qsub,
                     q.qrec);
-        return VPMC_OK;
+        if (!boxes) return VPMC_OK;
+        VPMC_LAUNCH(k_sub_starts, blocks_for(g.nbins), 256, 0, st, q.qsub, q.qstart, g.nbins, q.sstart);
+        return make_box_items(ctx, g, q.sstart, *boxes);
     }
     int shift = 0;
     while (((g.nbins - 1) >> shift) + 1 > kTargetSuper) ++shift;
@@ -2038,8 +2103,8 @@ int place_samples(vpmc_context* ctx, const GridBufs& g, QueryBufs& q, const floa
     VPMC_LAUNCH(k_scatter_window, tgrid, kPlaceThreads, tile_smem, st, q.tmp, q.qstart + g.nbins, M, wshift, q.qstart,
                 q.win_fill, q.tmp2);
     VPMC_LAUNCH(k_scatter_assemble, int(std::max<long>(1, std::min<long>(nwin, 2L * ctx->sm_count))), kAsmThreads, win_smem,
-                st, q.tmp2, g.nbins, wshift, q.qstart, g.inst, g.n_inst, q.qrec);
-    return VPMC_OK;
+                st, q.tmp2, g.nbins, wshift, q.qstart, g.inst, g.n_inst, q.qrec, boxes ? q.sstart : nullptr);
+    return boxes ? make_box_items(ctx, g, q.sstart, *boxes) : int(VPMC_OK);
 }
 
 int bin_points(vpmc_context* ctx, const GridBufs& g, QueryBufs& q, const float2* pts, long M, int set, int field9) {

@@ -35,6 +35,7 @@ struct GridInst {
     int p_begin, p_end;     // particle range of the instance
     float half_h3[3];       // h_w^3 / 2 as a sum of three floats (vpmc_wide.cuh)
     double inv_h3;          // 1 / h_w^3
+    int nb;                 // boxes per cell and axis that local expansions sum (vpmc_eval_box.cu), 0: none
 };
 
 // Candidate record (32 bytes): coordinates and weight duplicated so that one
@@ -66,7 +67,7 @@ struct QRec {
 struct Item {
     uint32_t bin;
     uint32_t qbeg;
-    uint32_t qcnt;
+    uint32_t qcnt;   // (box items: count | box << 16)
     uint32_t inst;
 };
 
@@ -109,6 +110,47 @@ __device__ __forceinline__ float sqrt_approx(float x) {
     float r;
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
+}
+
+// Sum over one staged run of candidates for NPR packed query pairs, in
+// bin-local coordinates, every squared distance pre-scaled by kappa = -3/h^2:
+// candidates hold (x, y) relative to the bin centre and kappa c2; queries
+// enter as -2 kappa q and kappa |q|^2, so
+//   s2 = kappa c2 + kappa q2 - 2 kappa c.q = -3 (r/h)^2,   sqrt(|s2|) = sqrt(3) r/h
+//   t  = saturate(1 - sqrt(|s2|)/sqrt(3))                  (= max(1 - r/h, 0))
+//   P += w * min(0.5 + s2 t, t^3)                          (= w W / 2 sigma)
+// because the spline's inner branch 1/2 - 3 q^2 + 3 q^3 is 1/2 - 3 q^2 (1 - q),
+// and beyond the support t = 0 leaves min(1/2, 0) = 0.
+// Per pair of queries: 7 packed FMA-pipe operations + 2 saturating scalar FMAs,
+// 2 square roots on the XU and 2 min on the ALU.  The candidate loop is unrolled
+// eight times (independent chains across candidates, 80 registers; at tg2048
+// 257.7 ms per evaluation against 261.1 unrolled four times, 274.4 twice,
+// 272.5 twelve times, 258.4 sixteen times).
+template <int NPR, int NPMAX, int UNROLL = 8>
+__device__ __forceinline__ void packed_run(const Cand* __restrict__ cs, int cnt, const f2x (&QX)[NPMAX],
+                                           const f2x (&QY)[NPMAX], const f2x (&Q2)[NPMAX], f2x (&P)[NPMAX]) {
+    const f2x HALF = pk2(0.5f, 0.5f);
+#pragma unroll UNROLL
+    for (int c = 0; c < cnt; ++c) {
+        const ulonglong2 XY = *reinterpret_cast<const ulonglong2*>(&cs[c].x);
+        const ulonglong2 WC = *reinterpret_cast<const ulonglong2*>(&cs[c].w);   // (w, w), (kappa c2, kappa c2)
+#pragma unroll
+        for (int pr = 0; pr < NPR; ++pr) {
+            const f2x s = add2(WC.y, Q2[pr]);
+            const f2x s2 = fma2(XY.y, QY[pr], fma2(XY.x, QX[pr], s));
+            float ra, rb;
+            up2(s2, ra, rb);
+            // rounding can leave s2 a hair above 0 when c ~ q: take sqrt(|s2|)
+            const float sa = sqrt_approx(fabsf(ra)), sb = sqrt_approx(fabsf(rb));
+            const f2x t = pk2(__saturatef(fmaf(-kInvSqrt3, sa, 1.f)), __saturatef(fmaf(-kInvSqrt3, sb, 1.f)));
+            const f2x in = fma2(s2, t, HALF);
+            const f2x t3 = mul2(mul2(t, t), t);
+            float ia, ib, ta, tb;
+            up2(in, ia, ib);
+            up2(t3, ta, tb);
+            P[pr] = fma2(WC.x, pk2(fminf(ia, ta), fminf(ib, tb)), P[pr]);
+        }
+    }
 }
 
 // One column of a bin's walk (lane = 0 .. 2k of a warp; column ox = lane - k
@@ -227,8 +269,8 @@ struct InstDesc {
 long grid_plan(const InstDesc* in, int n, int k, int nsets, GridInst* out);
 int default_k();
 // Walk cells per h_w for an instance of n particles that evaluates `samples` points
-// of each sign set a pass.
-int sample_k(long n, double samples, float Lx, float Ly, float hw);
+// of each sign set a pass (boxes: whether local expansions may sum them).
+int sample_k(long n, double samples, float Lx, float Ly, float hw, bool boxes = false);
 
 // Device-side working set of one grid (caller owns the memory).
 struct GridBufs {
@@ -242,6 +284,7 @@ struct GridBufs {
     uint32_t* cstart = nullptr; // nbins + 1: candidate range of a whole bin (= start when rows == 1)
     Cand* cand = nullptr;       // n
     CandF* candf = nullptr;     // n (deformed kernels only)
+    float4* cand4 = nullptr;    // n compact records {x, y, weight, 0} (boxes only)
     uint32_t* perm = nullptr;   // n: sorted slot -> particle (points into rs buffers)
     RadixScratch rs{};
 };
@@ -252,10 +295,10 @@ void carve_grid(Carver& c, long n, long nbins, int n_inst, GridBufs* g, bool def
 // omega (SET_SIGN_SPLIT scales |omega| by 2 sigma, SET_ONE_SIGNED by
 // 2 sigma too).  Writes g.cand / g.start / g.perm; with F (per particle,
 // row-major {F11, F12, F21, F22}) it writes the deformed records g.candf.
-// grid_sort: keys, sort and ranges alone.
+// compact: the float4 records g.cand4 as well.  grid_sort: keys, sort and ranges alone.
 int grid_sort(vpmc_context* ctx, GridBufs& g, const float2* pos, const float* omega, int set_mode);
 int grid_build(vpmc_context* ctx, GridBufs& g, const float2* pos, const float* omega, int set_mode,
-               const float4* F = nullptr);
+               const float4* F = nullptr, bool compact = false);
 // Overwrite candidate weights from a vector in sorted order: cand[p].z/.w =
 // hi/lo FP32 split of scale * x[p] (FP64 in, for the SpMV).
 int grid_set_weights_sorted(vpmc_context* ctx, GridBufs& g, const double* x_sorted, double scale);
@@ -270,7 +313,8 @@ struct ItemBufs {
     uint32_t* scan_tmp = nullptr;
     long max_items = 0;
 };
-void carve_items(Carver& c, long nbins, long max_queries, ItemBufs* it);
+// n_boxes: items are made of that many boxes (-1: of bins).
+void carve_items(Carver& c, long nbins, long max_queries, ItemBufs* it, long n_boxes = -1);
 // chunk = queries per item = 256 * queries-per-thread of the eval launch.
 int make_items(vpmc_context* ctx, const GridBufs& g, const uint32_t* qstart, ItemBufs& it, int chunk, long queries);
 int query_chunk(int qpt);
@@ -284,6 +328,7 @@ struct QueryBufs {
     uint32_t* qfill = nullptr;   // nbins
     uint32_t* qrank = nullptr;   // direct placement: rank in (bin, sub-cell) << 4 | sub-cell, per point
     uint32_t* qsub = nullptr;    // points per (bin, sub-cell)
+    uint32_t* sstart = nullptr;  // first slot of each (bin, sub-cell), nbins 16 + 1 (boxes)
     QRec* qrec = nullptr;        // max points
     uint4* tmp = nullptr;        // max points (staged placement: super-bins)
     uint4* tmp2 = nullptr;       // max points (staged placement: slot windows)
@@ -294,7 +339,8 @@ struct QueryBufs {
     uint32_t* scan_tmp = nullptr;
 };
 // samples: binned samples of the MIS step (place_samples) instead of points.
-void carve_queries(Carver& c, long nbins, long max_points, QueryBufs* q, bool samples = false);
+// boxes: the starts of each bin's sub-cells too.
+void carve_queries(Carver& c, long nbins, long max_points, QueryBufs* q, bool samples = false, bool boxes = false);
 // Bin arbitrary points (one instance `inst_of` lookup per point by index range
 // `point_inst` == nullptr -> instance 0).  set = candidate set to query.
 int bin_points(vpmc_context* ctx, const GridBufs& g, QueryBufs& q, const float2* pts, long M, int set,
@@ -308,19 +354,35 @@ int scatter_points(vpmc_context* ctx, const GridBufs& g, QueryBufs& q, const flo
 // q.qsub is carved, per (bin, sub-cell), there with each sample's rank where
 // q.qrank is carved (direct placement).
 int clear_counts(vpmc_context* ctx, QueryBufs& q);
+// boxes (when the plan has any): the items of the boxed instances' boxes go there and
+// not into `it`.
 int place_samples(vpmc_context* ctx, const GridBufs& g, QueryBufs& q, const float2* pts, long M, ItemBufs& it,
-                  int chunk);
+                  int chunk, ItemBufs* boxes = nullptr);
+
+constexpr int kSubCells = 16;
 
 #ifdef __CUDACC__
-// Sub-cell of a query (wrapped point p in the cell of its bin): 4 x 4
-// sub-cells in serpentine order (rows of sub-cells, alternate rows reversed),
-// so that any run of consecutive keys covers a compact part of the cell.
-// c = {cx, cy, gx / Lx, gy / Ly} of the bin's cell.
-constexpr int kSubCells = 16;
+// Sub-cell of a query (wrapped point p in the cell of its bin): 4 x 4 sub-cells along
+// a Hilbert curve, so that any run of consecutive keys covers a compact part of the
+// cell and each aligned four are a 2 x 2 box.  c = {cx, cy, gx / Lx, gy / Ly} of the
+// bin's cell.  (No operation that a compiler may contract: every kernel that forms
+// the key of a point forms the same one.)
 __device__ __forceinline__ uint32_t subcell_key(float px, float py, float4 c) {
-    const int ix = min(max(int((px * c.z - c.x) * 4.f), 0), 3);
-    const int iy = min(max(int((py * c.w - c.y) * 4.f), 0), 3);
-    return uint32_t(iy * 4 + ((iy & 1) ? 3 - ix : ix));
+    const int ix = min(max(int(__fmul_rn(__fmaf_rn(px, c.z, -c.x), 4.f)), 0), 3);
+    const int iy = min(max(int(__fmul_rn(__fmaf_rn(py, c.w, -c.y), 4.f)), 0), 3);
+    // keys of (iy, ix), iy = 0 first, ix = 0 lowest: 0 1 14 15 | 3 2 13 12 | 4 7 8 11 | 5 6 9 10
+    constexpr unsigned long long kHilbert = 0xa965b874cd23fe10ull;
+    return uint32_t(kHilbert >> (4 * (iy * 4 + ix))) & 15u;
+}
+// (x, y) of box `box` among nb x nb (nb = 4: sub-cells, 2: quadrants, 1: the cell).
+__device__ __forceinline__ uint2 box_coords(uint32_t box, int nb) {
+    if (nb == 4) {
+        // x and y of each Hilbert key, two bits each: 00 10 11 01 02 03 13 12 22 23 33 32 31 21 20 30 (x y)
+        constexpr uint32_t kX = 0xebfa5014u, kY = 0x05bebe50u;
+        return make_uint2((kX >> (2u * box)) & 3u, (kY >> (2u * box)) & 3u);
+    }
+    if (nb == 2) return make_uint2(box >> 1, (box ^ (box >> 1)) & 1u);
+    return make_uint2(0u, 0u);
 }
 #endif
 
@@ -354,5 +416,31 @@ struct EvalTcArgs {
     uint32_t wait_limit;
 };
 int launch_eval_tc(vpmc_context* ctx, const EvalTcArgs& a, bool field9);
+
+// The FIELD / FIELD9 evaluation of boxed instances by local expansions (vpmc_eval_box.cu).
+constexpr int kBoxChunk = 192;        // samples an item
+constexpr float kBoxSide = 0.075f;    // largest box side, in h_w
+constexpr double kBoxSamples = 32.0;  // samples a box gathers at least (on average)
+constexpr double kBoxReach = 80.0;    // particles within h_w at least (on average)
+struct EvalBoxArgs {
+    const GridInst* inst;
+    const uint32_t* cstart;
+    int rows;
+    const float4* cand;
+    const QRec* qrec;
+    const Item* items;
+    const uint32_t* n_items;
+    uint32_t* counter;
+    float* out;
+    unsigned* flags;
+    uint32_t wait_limit;   // 0: give up as the pairwise kernel's first wait does
+};
+int launch_eval_box(vpmc_context* ctx, const EvalBoxArgs& a, bool field9);
+// Boxes per cell and axis for an instance of n particles with `samples` points a sign
+// set and pass (0: pair by pair).  512^2 particles, evaluation of a step by boxes and
+// pair by pair: 84 samples a box 4.2 and 8.5 ms, 63: 3.5 and 6.6, 42: 4.5 and 5.3 (and
+// 0.82 and 1.26 for 256^2), 21: 3.9 and 2.8; 113 particles within h_w 9.9 and 12.9, 50
+// particles 11.7 and 8.7.
+int box_split(long n, double samples, float Lx, float Ly, float hw, int gx, int gy);
 
 }  // namespace vpmc

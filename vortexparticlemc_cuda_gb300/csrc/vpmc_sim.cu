@@ -796,14 +796,26 @@ int upload_mc(vpmc_sim* s) {
 int alloc_work(vpmc_sim* s) {
     vpmc_context* ctx = s->ctx;
     std::vector<InstDesc> d(s->n_inst);
+    // instances that sample densely enough are summed by boxes (plain FP32 kernels, the
+    // default 4 queries a thread)
+    const bool can_box = s->precision == 32 && !s->deform && s->qpt == 4;
     for (int i = 0; i < s->n_inst; ++i)
         d[i] = InstDesc{s->prm[i].Lx, s->prm[i].Ly, s->mc[i].hw, s->prm[i].periodic, int(s->begin[i]),
                         int(s->begin[i] + s->counts[i]), s->deform ? s->cover : 1.f,
                         sample_k(s->counts[i], std::min(double(s->counts[i]) * samples_per(s), double(1L << 29)),
-                                 s->prm[i].Lx, s->prm[i].Ly, s->mc[i].hw)};
+                                 s->prm[i].Lx, s->prm[i].Ly, s->mc[i].hw, can_box)};
     s->plan.resize(s->n_inst);
     const long nb = grid_plan(d.data(), s->n_inst, s->k_walk, 2, s->plan.data());
     if (nb < 0) return int(-nb);
+    s->any_box = s->any_pair = false;
+    long n_boxes = 0;
+    for (int i = 0; i < s->n_inst; ++i) {
+        GridInst& g = s->plan[i];
+        if (can_box)
+            g.nb = box_split(s->counts[i], std::min(double(s->counts[i]) * samples_per(s), double(1L << 29)), g.Lx, g.Ly, g.hw, g.gx, g.gy);
+        (g.nb ? s->any_box : s->any_pair) = true;
+        n_boxes += 2L * g.gx * g.gy * g.nb * g.nb;
+    }
     const long Q2 = 2L * samples_per(s);
     long per_chunk = s->max_samples / Q2;
     if (per_chunk < 1) per_chunk = 1;
@@ -816,8 +828,10 @@ int alloc_work(vpmc_sim* s) {
     for (auto& e : s->chunk_ev) VPMC_CUDA(cudaEventCreate(&e));
     auto carve_all = [&](Carver& c) {
         carve_grid(c, s->N, nb, s->n_inst, &s->g, s->deform != 0, s->rows);
+        s->g.cand4 = s->any_box ? c.take<float4>(size_t(s->N)) : nullptr;
         carve_items(c, nb, ns, &s->it);
-        carve_queries(c, nb, ns, &s->q, true);
+        if (s->any_box) carve_items(c, nb, ns, &s->itb, n_boxes);
+        carve_queries(c, nb, ns, &s->q, true, s->any_box);
         s->ys = c.take<float2>(size_t(ns));
         s->ys_t0 = -1;
         s->ys_nt = 0;
@@ -892,7 +906,7 @@ int issue_pass(vpmc_sim* s, bool advect, bool timed, int* nlaunch) {
     const bool in_place = !def || s->t_end - s->t_begin <= s->chunk_targets;
     float2* const pos_out = in_place ? s->pos : s->pos_next;
     float4* const F_out = in_place ? s->F : s->F_next;
-    VPMC_TRY(grid_build(ctx, s->g, s->pos, s->omega, SET_SIGN_SPLIT, def ? s->F : nullptr));
+    VPMC_TRY(grid_build(ctx, s->g, s->pos, s->omega, SET_SIGN_SPLIT, def ? s->F : nullptr, s->any_box));
     if (def && advect) VPMC_CUDA(cudaMemsetAsync(s->d_sig, 0, 2 * sizeof(unsigned), st));
     const long Q = samples_per(s);
     if (!def) VPMC_LAUNCH(k_sub_pos, blocks_for(2 * s->N), 256, 0, st, s->d_mc, s->n_inst, s->sub, s->pos, 2 * s->N,
@@ -907,7 +921,7 @@ int issue_pass(vpmc_sim* s, bool advect, bool timed, int* nlaunch) {
                    s->d_step, t0, nt, s->N1, s->N2, def ? 5 : 1, nullptr, s->ys, s->q.qbin, s->q.qcount,
                    s->q.qsub, s->q.qrank, f64 ? nullptr : s->fv, f64 ? s->fv64 : nullptr, 1};
         VPMC_TRY(launch_gen(st, ga));
-        VPMC_TRY(place_samples(ctx, s->g, s->q, s->ys, ns, s->it, query_chunk(f64 ? 4 : s->qpt)));
+        VPMC_TRY(place_samples(ctx, s->g, s->q, s->ys, ns, s->it, query_chunk(f64 ? 4 : s->qpt), s->any_box ? &s->itb : nullptr));
         EvalLaunch L;
         const bool unb = s->mc[0].law == VPMC_LAW_UNBIASED;
         L.mode = f64 ? (unb ? EVAL_FIELD9_64 : EVAL_FIELD64)
@@ -917,7 +931,10 @@ int issue_pass(vpmc_sim* s, bool advect, bool timed, int* nlaunch) {
         L.out_f64 = s->fv64;
         const size_t ci = size_t((t0 - s->t_begin) / s->chunk_targets);
         if (timed) VPMC_CUDA(cudaEventRecordWithFlags(s->chunk_ev[2 * ci], st, ev_flags));
-        VPMC_TRY(launch_eval(ctx, s->g, s->q.qrec, s->it, L));
+        if (s->any_pair) VPMC_TRY(launch_eval(ctx, s->g, s->q.qrec, s->it, L));
+        if (s->any_box)
+            VPMC_TRY(launch_eval_box(ctx, EvalBoxArgs{s->g.inst, s->g.start, s->g.rows, s->g.cand4, s->q.qrec, s->itb.items,
+                                                      s->itb.n_items, s->itb.counter, s->fv, ctx->d_flags, ctx->wait_limit}, unb));
         if (timed) VPMC_CUDA(cudaEventRecordWithFlags(s->chunk_ev[2 * ci + 1], st, ev_flags));
         unsigned long long* const count_step = advect && t0 + nt >= s->t_end ? s->d_step : nullptr;
         if (def) {

@@ -121,6 +121,8 @@ struct vpmc_sim {
     std::vector<GridInst> plan;
     GridBufs g;
     ItemBufs it;
+    ItemBufs itb;                      // items of boxed instances
+    bool any_box = false, any_pair = true;   // some instance's samples are summed by boxes / pair by pair
     QueryBufs q;
     float2* ys = nullptr;
     long ys_t0 = -1, ys_nt = 0;        // targets whose samples ys holds (last chunk of the last pass)
