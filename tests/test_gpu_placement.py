@@ -36,3 +36,29 @@ def test_shards_agree_with_the_whole_run(cuda, nx, law):
     whole = run([(0, n)])
     assert torch.equal(whole, run([(0, 1), (1, 700), (700, n)]))
     assert not torch.equal(whole, pos)
+
+
+# bins of 260, 576 and 1,040 samples on average (the three sizes of the window assembly),
+# spread evenly and clustered, where most of the samples lie in windows that overflow.
+# The whole run is staged, its shards are placed directly.
+@pytest.mark.parametrize("hwr,walk", [(4, 2), (3, 1), (4, 1)])
+@pytest.mark.parametrize("clustered", [False, True])
+def test_windows_of_every_size(cuda, hwr, walk, clustered):
+    from vortexparticlemc_cuda_gb300 import phash as P
+    nx = 129
+    n = nx * nx
+    rng = np.random.default_rng(hwr + walk)
+    p = rng.random((n, 2))
+    if clustered:
+        p[: n * 4 // 5] = (0.02 * rng.normal(size=(n * 4 // 5, 2))) % 1.0
+    pos = torch.from_numpy(p.astype(np.float32)).cuda()
+    om = torch.from_numpy(rng.normal(size=n).astype(np.float32)).cuda()
+    sim = P.Simulation(P.SimParam(dt=1e-3, Nx=nx, hwr=hwr, N1=32, N2=32, seed=5), [n])
+    sim.set_tuning(walk, 4)
+    sim.set_particles(pos, om)
+    sim.prepare()
+    whole = sim.velocity(2)
+    for a, b in [(0, 5000), (5000, n)]:
+        sim.set_target_range(a, b)
+        assert torch.equal(whole[a:b], sim.velocity(2)[a:b])
+    sim.close()

@@ -306,9 +306,8 @@ constexpr int kPlaceTile = 8;                                // records per thre
 constexpr int kTileRecs = kPlaceThreads * kPlaceTile;        // 4096 records = 64 KB staged per tile
 constexpr int kTargetSuper = 512;                            // super-bins per grid
 constexpr int kWinMax = 2048;                                // windows one tile may sort in shared memory
-constexpr int kWinCap = 4096;                                // records a window assembles in shared memory
-constexpr int kAsmThreads = 512;                             // window assembly: 2 CTAs per SM
-constexpr int kWinBinsMax = 256;                             // bins per window at most
+constexpr int kAsmPer = 8;                                   // records per thread of a window that fits
+constexpr int kWinBinsMax = 64;                             // bins per window at most
 
 // Exclusive prefix sum of v[0..n) in place (shared memory, n small), block
 // of kPlaceThreads; returns the total.
@@ -407,19 +406,22 @@ __global__ void __launch_bounds__(kPlaceThreads) k_scatter_coarse(const float2* 
     }
 }
 
-// Query record of a placed sample: wrapped point and image flags.
-__device__ __forceinline__ QRec make_qrec(uint4 r, const GridInst* __restrict__ inst, int n_inst) {
-    const GridInst& G = inst[n_inst == 1 ? 0 : inst_of_bin(inst, n_inst, r.w)];
+// Query record of a placed sample: wrapped point and image flags (Lx, Ly: the
+// domain of its instance, (0, 0) where it is not periodic).
+__device__ __forceinline__ QRec make_qrec(uint4 r, float2 L) {
     float2 p = make_float2(__uint_as_float(r.x), __uint_as_float(r.y));
     uint32_t fl = (2u) | (2u << 3);
-    if (G.periodic) {
-        const float kx = floorf(p.x / G.Lx), ky = floorf(p.y / G.Ly);
-        p.x = p.x - kx * G.Lx;
-        p.y = p.y - ky * G.Ly;
+    if (L.x > 0.f) {
+        const float kx = floorf(p.x / L.x), ky = floorf(p.y / L.y);
+        p.x = p.x - kx * L.x;
+        p.y = p.y - ky * L.y;
         const int ikx = min(max(int(kx), -2), 2), iky = min(max(int(ky), -2), 2);
         fl = uint32_t(ikx + 2) | (uint32_t(iky + 2) << 3);
     }
     return QRec{p.x, p.y, r.z, fl};
+}
+__device__ __forceinline__ float2 wrap_lengths(const GridInst& G) {
+    return G.periodic ? make_float2(G.Lx, G.Ly) : make_float2(0.f, 0.f);
 }
 
 // Pass 2: the same per tile of the super-bin-grouped records, by window
@@ -507,17 +509,27 @@ __global__ void __launch_bounds__(kPlaceThreads) k_scatter_window(const uint4* _
 
 // Pass 3: one window per CTA: every record gets its slot from shared-memory
 // counters started at qstart of its bin, the window is built in shared memory
-// and written out as one contiguous block (an over-full window stores
-// directly).
-__global__ void __launch_bounds__(kAsmThreads, 2) k_scatter_assemble(const uint4* __restrict__ tmp2, long nbins, int wshift,
+// and written out as one contiguous block (an over-full window is counted and
+// placed from global memory, 8 records a thread in flight).  The chain of a window
+// (load, rank, scan, place, store, and a barrier after each) bounds it, so many small
+// CTAs share an SM: 128 threads where the bins hold up to 512 records, 256 up to
+// 1,024, else 512.  What a record needs of its instance is looked up once a bin.
+// 67 M samples in 668 a bin: 797 us with 512 threads, 610 with 256; 195 M samples of
+// 24 instances around vortices: 3.09 ms with 512 threads and
+// over-full windows in any order, 2.14 with 128 and all windows ordered (which takes
+// 8 % from the evaluation after it).  Bulk copies of the windows in and out, one or
+// two windows ahead, measured the same as these loads.
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_scatter_assemble(const uint4* __restrict__ tmp2, long nbins, int wshift,
                                                             const uint32_t* __restrict__ qstart,
                                                             const GridInst* __restrict__ inst, int n_inst,
                                                             QRec* __restrict__ qrec, uint32_t* __restrict__ sstart) {
-    constexpr int kPer = kWinCap / kAsmThreads;     // records per thread of a window that fits
-    extern __shared__ __align__(16) QRec buf[];   // kWinCap records
+    constexpr int kCap = THREADS * kAsmPer;
+    extern __shared__ __align__(16) QRec buf[];   // kCap records
     __shared__ uint32_t cnt[kWinBinsMax];
     __shared__ uint32_t sub[kSubCells * kWinBinsMax];   // per (sub-cell, bin of the window): count, then first slot
     __shared__ float4 corg[kWinBinsMax];                 // per bin of the window: its cell, for subcell_key
+    __shared__ float2 wrap[kWinBinsMax];                 // and its instance's periodic lengths
     const long nwin = ((nbins - 1) >> wshift) + 1;
     long w = blockIdx.x;
     if (w >= nwin) return;
@@ -526,58 +538,62 @@ __global__ void __launch_bounds__(kAsmThreads, 2) k_scatter_assemble(const uint4
     // so the loads overlap the previous window's write-out
     long b0 = w << wshift, b1 = min(nbins, b0 + (1L << wshift));
     uint32_t start = qstart[b0], nw = qstart[b1] - start;
-    uint4 r[kPer];
+    uint4 r[kAsmPer];
     auto load_records = [&](uint32_t st, uint32_t n) {
-        if (n > uint32_t(kWinCap)) return;
 #pragma unroll
-        for (int j = 0; j < kPer; ++j) {
-            const uint32_t k = threadIdx.x + uint32_t(j) * uint32_t(kAsmThreads);
-            r[j] = k < n ? tmp2[st + k] : make_uint4(0u, 0u, 0u, 0u);
+        for (int j = 0; j < kAsmPer; ++j) {
+            const uint32_t k = threadIdx.x + uint32_t(j) * uint32_t(THREADS);
+            if (k < n) r[j] = tmp2[st + k];
         }
     };
-    load_records(start, nw);
+    auto load_window = [&](uint32_t st, uint32_t n) {
+        if (n <= uint32_t(kCap)) load_records(st, n);
+    };
+    load_window(start, nw);
     for (;;) {
-        const bool fits = nw <= uint32_t(kWinCap);
+        const bool fits = nw <= uint32_t(kCap);
         const uint32_t nb = uint32_t(b1 - b0);
-        for (long b = b0 + threadIdx.x; b < b1; b += blockDim.x) {
+        for (long b = b0 + threadIdx.x; b < b1; b += THREADS) {
             cnt[b - b0] = qstart[b];
             const GridInst& G = inst[n_inst == 1 ? 0 : inst_of_bin(inst, n_inst, uint32_t(b))];
             const uint32_t cell = (uint32_t(b) - uint32_t(G.bin_base)) % uint32_t(G.gx * G.gy);
             corg[b - b0] = make_float4(float(int(cell) / G.gy), float(int(cell) % G.gy), G.inv_sx, G.inv_sy);
+            wrap[b - b0] = wrap_lengths(G);
         }
-        for (uint32_t i = threadIdx.x; i < uint32_t(kSubCells) * nb; i += blockDim.x) sub[i] = 0u;
+        for (uint32_t i = threadIdx.x; i < uint32_t(kSubCells) * nb; i += THREADS) sub[i] = 0u;
         __syncthreads();
         // inside each bin the records are ordered by sub-cell, so that consecutive
-        // queries of a bin lie close together (a window of several bins that does not fit
-        // only where boxes need the order: ordering it from global memory costs more
-        // than the closer queries save)
-        const bool order = fits || sstart || nb == 1u;
-        uint32_t kr[kPer];   // bin in the window | sub-cell << 8 | rank within (sub-cell, bin) << 12
+        // queries of a bin lie close together
+        uint32_t kr[kAsmPer];   // bin in the window | sub-cell << 8 | rank within (sub-cell, bin) << 12
         if (fits) {
 #pragma unroll
-            for (int j = 0; j < kPer; ++j) {
-                const uint32_t k = threadIdx.x + uint32_t(j) * uint32_t(kAsmThreads);
+            for (int j = 0; j < kAsmPer; ++j) {
+                const uint32_t k = threadIdx.x + uint32_t(j) * uint32_t(THREADS);
                 if (k >= nw) break;
                 const uint32_t bl = r[j].w - uint32_t(b0);
-                const QRec q = make_qrec(r[j], inst, n_inst);
+                const QRec q = make_qrec(r[j], wrap[bl]);
                 const uint32_t key = subcell_key(q.x, q.y, corg[bl]);
                 kr[j] = bl | (key << 8) | (atomicAdd(&sub[key * nb + bl], 1u) << 12);
                 r[j] = make_uint4(__float_as_uint(q.x), __float_as_uint(q.y), q.id, q.flags);
             }
-        } else if (order) {   // a window that does not fit is counted, then placed, from global memory
-            for (uint32_t k = threadIdx.x; k < nw; k += blockDim.x) {
-                const uint4 rr = tmp2[start + k];
-                const uint32_t bl = rr.w - uint32_t(b0);
-                const QRec q = make_qrec(rr, inst, n_inst);
-                atomicAdd(&sub[subcell_key(q.x, q.y, corg[bl]) * nb + bl], 1u);
+        } else {   // a window that does not fit is counted, then placed, from global memory
+            for (uint32_t k0 = 0; k0 < nw; k0 += uint32_t(kCap)) {
+                load_records(start + k0, nw - k0);
+#pragma unroll
+                for (int j = 0; j < kAsmPer; ++j) {
+                    if (k0 + threadIdx.x + uint32_t(j) * uint32_t(THREADS) >= nw) break;
+                    const uint32_t bl = r[j].w - uint32_t(b0);
+                    const QRec q = make_qrec(r[j], wrap[bl]);
+                    atomicAdd(&sub[subcell_key(q.x, q.y, corg[bl]) * nb + bl], 1u);
+                }
             }
         }
         __syncthreads();
-        // each bin's 16 sub-cell counters -> first slots, by warp 0: two bins
+        // each bin's 16 sub-cell counters -> first slots: a warp takes two bins
         // per pass, one counter per lane, a scan inside each 16-lane half
-        if (threadIdx.x < 32 && order) {
-            const uint32_t lane = threadIdx.x, c = lane & 15u;
-            for (uint32_t b = lane >> 4; b < ((nb + 1u) & ~1u); b += 2u) {
+        {
+            const uint32_t lane = threadIdx.x & 31u, c = lane & 15u;
+            for (uint32_t b = (threadIdx.x >> 5) * 2u + (lane >> 4); b < ((nb + 1u) & ~1u); b += THREADS / 16) {
                 const bool live = b < nb;
                 const uint32_t n = live ? sub[c * nb + b] : 0u;
                 uint32_t incl = n;
@@ -595,18 +611,22 @@ __global__ void __launch_bounds__(kAsmThreads, 2) k_scatter_assemble(const uint4
         __syncthreads();
         if (fits) {
 #pragma unroll
-            for (int j = 0; j < kPer; ++j) {
-                const uint32_t k = threadIdx.x + uint32_t(j) * uint32_t(kAsmThreads);
+            for (int j = 0; j < kAsmPer; ++j) {
+                const uint32_t k = threadIdx.x + uint32_t(j) * uint32_t(THREADS);
                 if (k >= nw) break;
                 const uint32_t slot = sub[((kr[j] >> 8) & 15u) * nb + (kr[j] & 255u)] + (kr[j] >> 12);
                 buf[slot - start] = QRec{__uint_as_float(r[j].x), __uint_as_float(r[j].y), r[j].z, r[j].w};
             }
         } else {
-            for (uint32_t k = threadIdx.x; k < nw; k += blockDim.x) {
-                const uint4 rr = tmp2[start + k];
-                const uint32_t bl = rr.w - uint32_t(b0);
-                const QRec q = make_qrec(rr, inst, n_inst);
-                qrec[atomicAdd(order ? &sub[subcell_key(q.x, q.y, corg[bl]) * nb + bl] : &cnt[bl], 1u)] = q;
+            for (uint32_t k0 = 0; k0 < nw; k0 += uint32_t(kCap)) {
+                load_records(start + k0, nw - k0);
+#pragma unroll
+                for (int j = 0; j < kAsmPer; ++j) {
+                    if (k0 + threadIdx.x + uint32_t(j) * uint32_t(THREADS) >= nw) break;
+                    const uint32_t bl = r[j].w - uint32_t(b0);
+                    const QRec q = make_qrec(r[j], wrap[bl]);
+                    qrec[atomicAdd(&sub[subcell_key(q.x, q.y, corg[bl]) * nb + bl], 1u)] = q;
+                }
             }
         }
         __syncthreads();
@@ -619,10 +639,10 @@ __global__ void __launch_bounds__(kAsmThreads, 2) k_scatter_assemble(const uint4
             nb1 = min(nbins, nb0 + (1L << wshift));
             nstart = qstart[nb0];
             nnw = qstart[nb1] - nstart;
-            load_records(nstart, nnw);
+            load_window(nstart, nnw);
         }
         if (fits)
-            for (uint32_t k = threadIdx.x; k < nw; k += blockDim.x) qrec[start + k] = buf[k];
+            for (uint32_t k = threadIdx.x; k < nw; k += THREADS) qrec[start + k] = buf[k];
         __syncthreads();
         if (wn >= nwin) break;
         w = wn;
@@ -2083,17 +2103,28 @@ int place_samples(vpmc_context* ctx, const GridBufs& g, QueryBufs& q, const floa
     int shift = 0;
     while (((g.nbins - 1) >> shift) + 1 > kTargetSuper) ++shift;
     const int nsuper = int(((g.nbins - 1) >> shift) + 1);
-    // windows of 2^W bins holding about half the assembly capacity on average
+    // windows of 2^W bins holding about half the assembly capacity on average, of the
+    // smallest capacity that holds twice a bin and whose windows the second pass can
+    // count (1.07 G samples in 1.6 M bins, windows of one bin, 3,136 a super-bin: that
+    // pass reserves record by record, 18.8 ms; of two bins, 1,568: 8.8 ms)
     const double per_bin = double(M) / double(std::max<long>(g.nbins, 1));
-    int wshift = 0;
-    while ((1 << (wshift + 1)) <= kWinBinsMax && per_bin * double(2L << wshift) <= 0.5 * kWinCap) ++wshift;
+    int asm_threads = 64, win_cap = 0, wshift = 0;
+    do {
+        asm_threads *= 2;
+        win_cap = asm_threads * kAsmPer;
+        wshift = 0;
+        while ((1 << (wshift + 1)) <= kWinBinsMax && per_bin * double(2L << wshift) <= 0.5 * win_cap) ++wshift;
+    } while (asm_threads < 512 && (per_bin > 0.5 * win_cap || (1L << std::max(shift - wshift, 0)) > kWinMax));
     const long nwin = ((g.nbins - 1) >> wshift) + 1;
     static bool configured[64] = {};
-    const size_t tile_smem = sizeof(uint4) * size_t(kTileRecs), win_smem = sizeof(QRec) * size_t(kWinCap);
+    const size_t tile_smem = sizeof(uint4) * size_t(kTileRecs), win_smem = sizeof(QRec) * size_t(win_cap);
     if (ctx->device < 64 && !configured[ctx->device]) {
         VPMC_CUDA(cudaFuncSetAttribute(k_scatter_coarse, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tile_smem)));
         VPMC_CUDA(cudaFuncSetAttribute(k_scatter_window, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tile_smem)));
-        VPMC_CUDA(cudaFuncSetAttribute(k_scatter_assemble, cudaFuncAttributeMaxDynamicSharedMemorySize, int(win_smem)));
+        VPMC_CUDA(cudaFuncSetAttribute(k_scatter_assemble<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       int(sizeof(QRec)) * 256 * kAsmPer));
+        VPMC_CUDA(cudaFuncSetAttribute(k_scatter_assemble<512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       int(sizeof(QRec)) * 512 * kAsmPer));
         configured[ctx->device] = true;
     }
     const long tiles = (M + kTileRecs - 1) / kTileRecs;
@@ -2102,8 +2133,9 @@ int place_samples(vpmc_context* ctx, const GridBufs& g, QueryBufs& q, const floa
                 q.super_fill, q.tmp);
     VPMC_LAUNCH(k_scatter_window, tgrid, kPlaceThreads, tile_smem, st, q.tmp, q.qstart + g.nbins, M, wshift, q.qstart,
                 q.win_fill, q.tmp2);
-    VPMC_LAUNCH(k_scatter_assemble, int(std::max<long>(1, std::min<long>(nwin, 2L * ctx->sm_count))), kAsmThreads, win_smem,
-                st, q.tmp2, g.nbins, wshift, q.qstart, g.inst, g.n_inst, q.qrec, boxes ? q.sstart : nullptr);
+    auto* const assemble = asm_threads == 128 ? k_scatter_assemble<128> : asm_threads == 256 ? k_scatter_assemble<256> : k_scatter_assemble<512>;
+    VPMC_LAUNCH(assemble, int(std::max<long>(1, std::min<long>(nwin, (1024L / asm_threads) * ctx->sm_count))), asm_threads,
+                win_smem, st, q.tmp2, g.nbins, wshift, q.qstart, g.inst, g.n_inst, q.qrec, boxes ? q.sstart : nullptr);
     return boxes ? make_box_items(ctx, g, q.sstart, *boxes) : int(VPMC_OK);
 }
 
