@@ -166,135 +166,142 @@ __device__ __forceinline__ float2 aux_point(float2 x, int a, float dx) {
 // A few thousand bins make the counts collide (thousands of samples a bin: the
 // atomics of one address go one by one): 8.4 M samples in 8,192 bins took 219 us
 // counted per bin, 114 us per (bin, sub-cell).
+// 2^lane_bits threads take a target's samples in turn, so that the target's instance,
+// its fields and the disk's radius are found once a target: 24 instances, 195 M samples
+// 2.83 -> 2.29 ms; one instance of 512^2, 67 M samples 857 -> 799 us (without the CDF,
+// position and counter sectors it would be half of that: L2 is 75 % busy with them),
+// 2048^2 14.3 ms before and after.
 template <int COUNT>
 __global__ void __launch_bounds__(256) k_gen(GenArgs a) {
     const int Q = a.N1 + a.naux * a.N2;
-    const uint32_t Q2 = uint32_t(2 * Q);
-    const uint32_t total = uint32_t(a.nt) * Q2;   // samples of one chunk (< 2^31)
+    const uint32_t Q2 = uint32_t(2 * Q), lanes = 1u << a.lane_bits;
     const unsigned long long step = *a.step;
-    // sample sid = (target tl, sign s, sample j): decomposed once, then advanced
-    // by the grid stride without dividing again
-    const uint32_t stride = gridDim.x * blockDim.x;
-    const uint32_t dtl = stride / Q2, drem = stride - dtl * Q2;
-    uint32_t sid = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t tl = sid / Q2, rem = sid - tl * Q2;
-    for (; sid < total; sid += stride) {
-        const int s = rem >= uint32_t(Q) ? 1 : 0, j = int(rem) - s * Q;
+    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = (gridDim.x * blockDim.x) >> a.lane_bits;
+    for (uint32_t tl = tid >> a.lane_bits; tl < uint32_t(a.nt); tl += stride) {
         const long t = a.t0 + long(tl);
-        tl += dtl;
-        rem += drem;
-        if (rem >= Q2) { rem -= Q2; ++tl; }
         const int ii = inst_of(a.mc, a.n_inst, t);
         const InstMC& I = a.mc[ii];
         const GridInst& G = a.gi[ii];
         const float2 x = a.pos[t];
-        // counter = (sample | sign, instance-local target, step): an ensemble
-        // member draws exactly what a standalone run with its seed draws
-        const U4 r = philox4x32_10(U4{uint32_t(j) | (uint32_t(s) << 31), uint32_t(t - I.p_begin), uint32_t(step),
-                                      uint32_t(step >> 32)},
-                                   I.key0, I.key1);
-        float2 y = x;
-        bool valid = true;
-        int src = -1;
-        if (j < a.N1) {
-            const int n = I.cnt[s];
-            if (n == 0) {
-                valid = false;
+        for (uint32_t rem = tid & (lanes - 1u); rem < Q2; rem += lanes) {
+            const uint32_t sid = tl * Q2 + rem;   // < 2^31
+            const int s = rem >= uint32_t(Q) ? 1 : 0, j = int(rem) - s * Q;
+            // counter = (sample | sign, instance-local target, step): an ensemble
+            // member draws exactly what a standalone run with its seed draws
+            const U4 r = philox4x32_10(U4{uint32_t(j) | (uint32_t(s) << 31), uint32_t(t - I.p_begin), uint32_t(step),
+                                          uint32_t(step >> 32)},
+                                       I.key0, I.key1);
+            float2 y = x;
+            bool valid = true;
+            int src = -1;
+            if (j < a.N1) {
+                const int n = I.cnt[s];
+                if (n == 0) {
+                    valid = false;
+                } else {
+                    const int idx = sample_cdf(a.cdf + I.off[s], a.guide + I.goff[s], n, r.x);
+                    int p = -1;
+                    if (a.pos_sub) {
+                        y = a.pos_sub[I.off[s] + idx];
+                    } else {
+                        p = a.sub[I.off[s] + idx] + I.p_begin;   // subsets hold instance-local indices
+                        src = p;
+                        y = a.pos[p];
+                    }
+                    if (I.periodic) {
+                        const int m9 = min(int(u01(r.y) * 9.f), 8);
+                        y.x += float(m9 / 3 - 1) * I.Lx;
+                        y.y += float(m9 % 3 - 1) * I.Ly;
+                    }
+                    float rr;
+                    const float ur = u01(r.z);
+                    if (I.law == VPMC_LAW_REFERENCE) {
+                        // sample_kernel_radius (include/monte_carlo_bs.cuh:78-88): the
+                        // table already holds h_w and is scaled by h_w once more
+                        const float f = ur * (kIcdfRef - 1);
+                        const int i0 = int(f), i1 = min(i0 + 1, kIcdfRef - 1);
+                        const float tt = f - i0;
+                        rr = (I.icdf[i0] * (1.f - tt) + I.icdf[i1] * tt) * I.hw;
+                    } else {
+                        const float f = ur * kJitTab;
+                        const int i0 = min(int(f), kJitTab - 1);
+                        const float tt = f - i0;
+                        const float2 jt = a.jit[i0];   // (table[i0], table[i0 + 1])
+                        rr = (jt.x * (1.f - tt) + jt.y * tt) * I.hw;
+                    }
+                    float sn, cs;
+                    sincospif(2.f * u01(r.w), &sn, &cs);   // angle 2 pi u
+                    const float jx = rr * cs, jy = rr * sn;
+                    if (a.F) {
+                        // mul_mat2(F, r) (include/monte_carlo_bs.cuh:99-103)
+                        const float4 f = a.F[p];
+                        y.x += f.x * jx + f.y * jy;
+                        y.y += f.z * jx + f.w * jy;
+                    } else {
+                        y.x += jx;
+                        y.y += jy;
+                    }
+                }
             } else {
-                const int idx = sample_cdf(a.cdf + I.off[s], a.guide + I.goff[s], n, r.x);
-                int p = -1;
-                if (a.pos_sub) {
-                    y = a.pos_sub[I.off[s] + idx];
-                } else {
-                    p = a.sub[I.off[s] + idx] + I.p_begin;   // subsets hold instance-local indices
-                    src = p;
-                    y = a.pos[p];
-                }
-                if (I.periodic) {
-                    const int m9 = min(int(u01(r.y) * 9.f), 8);
-                    y.x += float(m9 / 3 - 1) * I.Lx;
-                    y.y += float(m9 % 3 - 1) * I.Ly;
-                }
-                float rr;
-                const float ur = u01(r.z);
-                if (I.law == VPMC_LAW_REFERENCE) {
-                    // sample_kernel_radius (include/monte_carlo_bs.cuh:78-88): the
-                    // table already holds h_w and is scaled by h_w once more
-                    const float f = ur * (kIcdfRef - 1);
-                    const int i0 = int(f), i1 = min(i0 + 1, kIcdfRef - 1);
-                    const float tt = f - i0;
-                    rr = (I.icdf[i0] * (1.f - tt) + I.icdf[i1] * tt) * I.hw;
-                } else {
-                    const float f = ur * kJitTab;
-                    const int i0 = min(int(f), kJitTab - 1);
-                    const float tt = f - i0;
-                    const float2 jt = a.jit[i0];   // (table[i0], table[i0 + 1])
-                    rr = (jt.x * (1.f - tt) + jt.y * tt) * I.hw;
-                }
+                const int ax = a.naux > 1 ? (j - a.N1) / a.N2 : 0;
+                const float2 xa = aux_point(x, ax, I.dx);
+                const float R = disk_radius(xa, I.periodic != 0, I.Lx, I.Ly);
+                const float ur = u01(r.y);
+                const float rr = I.law == VPMC_LAW_REFERENCE ? R * sqrtf(ur) : R * ur;
                 float sn, cs;
-                sincospif(2.f * u01(r.w), &sn, &cs);   // angle 2 pi u
-                const float jx = rr * cs, jy = rr * sn;
-                if (a.F) {
-                    // mul_mat2(F, r) (include/monte_carlo_bs.cuh:99-103)
-                    const float4 f = a.F[p];
-                    y.x += f.x * jx + f.y * jy;
-                    y.y += f.z * jx + f.w * jy;
+                sincospif(2.f * u01(r.x), &sn, &cs);   // angle 2 pi u
+                y.x = xa.x + rr * cs;
+                y.y = xa.y + rr * sn;
+            }
+            uint32_t b = kNoBin;
+            if (valid) {
+                float px = y.x, py = y.y;
+                bool ok = true;
+                if (I.periodic) {
+                    const float kx = floorf(px / I.Lx), ky = floorf(py / I.Ly);
+                    if (I.law == VPMC_LAW_UNBIASED && (fabsf(kx) > 2.f || fabsf(ky) > 2.f)) ok = false;
+                    px -= kx * I.Lx;
+                    py -= ky * I.Ly;
                 } else {
-                    y.x += jx;
-                    y.y += jy;
+                    ok = !(px < 0.f || px > I.Lx || py < 0.f || py > I.Ly);
+                }
+                if (ok) {
+                    const int cx = min(max(floor_int(px * G.inv_sx), 0), G.gx - 1);
+                    const int cy = min(max(floor_int(py * G.inv_sy), 0), G.gy - 1);
+                    b = uint32_t(G.bin_base) + uint32_t(s) * uint32_t(G.gx * G.gy) + uint32_t(cx * G.gy + cy);
+                    if constexpr (COUNT == 0) {
+                        atomicAdd(&a.qcount[b], 1u);
+                    } else {
+                        const uint32_t sub = subcell_key(px, py, make_float4(float(cx), float(cy), G.inv_sx, G.inv_sy));
+                        uint32_t* c = &a.qsub[size_t(b) * kSubCells + sub];
+                        if constexpr (COUNT == 1) atomicAdd(c, 1u);
+                        else a.qrank[sid] = (atomicAdd(c, 1u) << 4) | sub;
+                    }
                 }
             }
-        } else {
-            const int ax = a.naux > 1 ? (j - a.N1) / a.N2 : 0;
-            const float2 xa = aux_point(x, ax, I.dx);
-            const float R = disk_radius(xa, I.periodic != 0, I.Lx, I.Ly);
-            const float ur = u01(r.y);
-            const float rr = I.law == VPMC_LAW_REFERENCE ? R * sqrtf(ur) : R * ur;
-            float sn, cs;
-            sincospif(2.f * u01(r.x), &sn, &cs);   // angle 2 pi u
-            y.x = xa.x + rr * cs;
-            y.y = xa.y + rr * sn;
-        }
-        uint32_t b = kNoBin;
-        if (valid) {
-            float px = y.x, py = y.y;
-            bool ok = true;
-            if (I.periodic) {
-                const float kx = floorf(px / I.Lx), ky = floorf(py / I.Ly);
-                if (I.law == VPMC_LAW_UNBIASED && (fabsf(kx) > 2.f || fabsf(ky) > 2.f)) ok = false;
-                px -= kx * I.Lx;
-                py -= ky * I.Ly;
-            } else {
-                ok = !(px < 0.f || px > I.Lx || py < 0.f || py > I.Ly);
-            }
-            if (ok) {
-                const int cx = min(max(floor_int(px * G.inv_sx), 0), G.gx - 1);
-                const int cy = min(max(floor_int(py * G.inv_sy), 0), G.gy - 1);
-                b = uint32_t(G.bin_base) + uint32_t(s) * uint32_t(G.gx * G.gy) + uint32_t(cx * G.gy + cy);
-                if constexpr (COUNT == 0) {
-                    atomicAdd(&a.qcount[b], 1u);
-                } else {
-                    const uint32_t sub = subcell_key(px, py, make_float4(float(cx), float(cy), G.inv_sx, G.inv_sy));
-                    uint32_t* c = &a.qsub[size_t(b) * kSubCells + sub];
-                    if constexpr (COUNT == 1) atomicAdd(c, 1u);
-                    else a.qrank[sid] = (atomicAdd(c, 1u) << 4) | sub;
+            if (b == kNoBin) {   // no query will write its value
+                for (int v = 0; v < a.nval; ++v) {
+                    if (a.f32) a.f32[size_t(sid) * a.nval + v] = 0.f;
+                    if (a.f64) a.f64[size_t(sid) * a.nval + v] = 0.0;
                 }
             }
+            a.ys[sid] = y;
+            a.qbin[sid] = b;
+            if (a.src) a.src[sid] = src;
         }
-        if (b == kNoBin) {   // no query will write its value
-            for (int v = 0; v < a.nval; ++v) {
-                if (a.f32) a.f32[size_t(sid) * a.nval + v] = 0.f;
-                if (a.f64) a.f64[size_t(sid) * a.nval + v] = 0.0;
-            }
-        }
-        a.ys[sid] = y;
-        a.qbin[sid] = b;
-        if (a.src) a.src[sid] = src;
     }
 }
 
-int launch_gen(cudaStream_t st, const GenArgs& a) {
-    const int grid = blocks_for(a.nt * 2 * (a.N1 + long(a.naux) * a.N2));
+int launch_gen(cudaStream_t st, const GenArgs& args) {
+    GenArgs a = args;
+    const long q2 = 2 * (a.N1 + long(a.naux) * a.N2);
+    // 32 threads a target, fewer where more than an eighth of them would idle at the
+    // end, more where the targets alone do not fill the device
+    a.lane_bits = 5;
+    while (a.lane_bits > 0 && (-q2 & ((1L << a.lane_bits) - 1)) * 8 > q2) --a.lane_bits;
+    if (a.lane_bits == 5)
+        while (a.nt << a.lane_bits < (1L << 19) && (1L << a.lane_bits) < q2) ++a.lane_bits;
+    const int grid = blocks_for(a.nt << a.lane_bits);
     if (!a.qsub) VPMC_LAUNCH(k_gen<0>, grid, 256, 0, st, a);
     else if (!a.qrank) VPMC_LAUNCH(k_gen<1>, grid, 256, 0, st, a);
     else VPMC_LAUNCH(k_gen<2>, grid, 256, 0, st, a);

@@ -68,6 +68,7 @@ struct GenArgs {
     float* f32;                   // the samples' values, in FP32 or FP64: zeroed where a sample is dropped
     double* f64;
     int nval;                     // values a sample (1, or 3 with the gradient)
+    int lane_bits = 0;            // 2^lane_bits threads share a target (set by launch_gen)
 };
 
 // One thread per (target, sign, sample): Philox draw, branch-1 CDF / image /
