@@ -54,3 +54,12 @@ def test_query_on_small_grids(cuda, n, m, sign):
     k = 40 / (7 * math.pi * hw * hw) * torch.where(q <= 0.5, 6 * (q ** 3 - q * q) + 1, 2 * t ** 3)
     want, scale = k @ w, float((k @ w.abs()).max())
     assert float((got.double() - want).abs().max()) <= 1e-5 * max(scale, 1e-30)
+
+
+# 4,096 cells are the most that sort in one counting pass (tiles of 512 to 16,384 members)
+@pytest.mark.parametrize("n,rx,ry,sub", [(16385, 64, 64, False), (17000, 1, 1, True), (20000, 2, 1, False), (33000, 1, 3, False),
+                                         (40000, 3, 5, True), (60000, 3, 11, False), (70000, 5, 205, True),
+                                         (77824, 64, 64, True), (77825, 63, 65, False), (200001, 64, 64, False),
+                                         (200001, 17, 241, True), (2500001, 50, 81, False), (3000000, 64, 64, True)])
+def test_counting_pass_is_a_stable_counting_sort(cuda, n, rx, ry, sub):
+    test_hash_is_a_stable_counting_sort(cuda, n, rx, ry, sub)

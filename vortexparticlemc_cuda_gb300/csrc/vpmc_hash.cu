@@ -1,12 +1,15 @@
 // vpmc_hash.cu -- the reference-shaped spatial hash (FillCells / CountingSort)
 // and the sign subsets with their FP64 |omega| CDFs.
 //
-// Hash: one key kernel (cell of sub[i]), a stable radix sort of (cell, local index)
-// pairs, whose values are vp_sort, and each cell's first entry among the sorted
-// cells (cell_acc); FillCells alone counts the cells and scans the counts.  The result equals the reference's sequential counting
+// Hash: up to kTileCells cells in one counting pass over tiles (one CTA does a whole
+// small hash), else one key kernel (cell of sub[i]), a stable radix sort of (cell,
+// local index) pairs, whose values are vp_sort, and each cell's first entry among the
+// sorted cells (cell_acc); FillCells alone counts the cells and scans the counts.  The
+// result equals the reference's sequential counting
 // sort (src/cpu/hash.cpp:36-48) bit for bit: members of a cell ascend by local
 // index.  The reference's CUDA scatter (src/cuda/hash.cu:27-39) uses atomicSub
 // and is order-nondeterministic; this one is deterministic.
+#include <algorithm>
 #include <vector>
 
 #include "vpmc_blocksort.cuh"
@@ -95,6 +98,122 @@ __global__ void k_cell_starts(const uint32_t* __restrict__ keys, int N, int ncel
     if (c >= ncell) return;
     cell_acc[c] = int(lower_bound_key(keys, uint32_t(N), uint32_t(c)));
     if (cell_num) cell_num[c] = 0;
+}
+
+// A hash of up to kTileCells cells sorts in one counting pass.  Its members are cut
+// into tiles, one CTA each: k_cells_count writes the cells and each tile's counts per
+// cell, k_cell_columns turns the counts into prefixes over the tiles and the cells'
+// totals (whose scan is cell_acc), and k_cells_place ranks each tile's members in index
+// order and stores them.  2.1 M members of 4,096 cells: the two radix passes and their
+// scans took 95 us of kernels (152 us the call), these 52 us (98 us): reading the
+// members through sub 13 us, ranking by ballots and 4-byte stores 30 us.  50,000 members
+// 96 -> 79 us a call, 17,000 on 17^2 cells 73 and 75.
+constexpr int kTileCells = 4096;
+constexpr long kTileMaxN = 1L << 23;      // at most 512 tiles
+constexpr int kTileMax = 16384;           // members a tile
+constexpr int kPlaceThreads = 512, kPlaceWarps = kPlaceThreads / 32;
+constexpr size_t place_smem(int ncell, int tile) {   // counts per (warp, cell), first slots, ranks
+    return size_t(kPlaceWarps) * 2 * size_t((ncell + 1) & ~1) + 4 * size_t(ncell) + 2 * size_t(tile);
+}
+
+__global__ void __launch_bounds__(1024) k_cells_count(int rshx, int rshy, float inv_hx, float inv_hy,
+                                                      const int* __restrict__ sub, const float2* __restrict__ pos,
+                                                      long N, int tile, int* __restrict__ vp_cell,
+                                                      uint32_t* __restrict__ counts) {
+    __shared__ uint32_t hist[kTileCells];
+    const int ncell = rshx * rshy;
+    for (int c = threadIdx.x; c < ncell; c += 1024) hist[c] = 0u;
+    __syncthreads();
+    const long t0 = long(blockIdx.x) * tile, t1 = min(N, t0 + tile);
+#pragma unroll 4
+    for (long i = t0 + threadIdx.x; i < t1; i += 1024) {
+        const float2 p = pos[sub ? sub[i] : int(i)];
+        const int ix = min(max(floor_int(p.x * inv_hx), 0), rshx - 1);
+        const int iy = min(max(floor_int(p.y * inv_hy), 0), rshy - 1);
+        const int c = ix * rshy + iy;
+        vp_cell[i] = c;
+        atomicAdd(&hist[c], 1u);
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < ncell; c += 1024) counts[size_t(blockIdx.x) * ncell + c] = hist[c];
+}
+
+// 32 cells a CTA, a cell a lane; each warp a run of tiles.
+__global__ void __launch_bounds__(1024) k_cell_columns(uint32_t* __restrict__ counts, int ntiles, int ncell,
+                                                       uint32_t* __restrict__ total, int* __restrict__ cell_num) {
+    __shared__ uint32_t part[32][33];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
+    const int per = (ntiles + 31) / 32, a = min(ntiles, w * per), b = min(ntiles, a + per);
+    uint32_t sum = 0u;
+    if (c < ncell)
+        for (int t = a; t < b; ++t) sum += counts[size_t(t) * ncell + c];
+    part[w][lane] = sum;
+    __syncthreads();
+    if (c >= ncell) return;
+    uint32_t run = 0u;
+    for (int q = 0; q < w; ++q) run += part[q][lane];
+    for (int t = a; t < b; ++t) {
+        const uint32_t v = counts[size_t(t) * ncell + c];
+        counts[size_t(t) * ncell + c] = run;
+        run += v;
+    }
+    if (w == 31) {
+        total[c] = run;
+        if (cell_num) cell_num[c] = 0;
+    }
+}
+
+__global__ void __launch_bounds__(kPlaceThreads) k_cells_place(const int* __restrict__ vp_cell, long N, int tile, int ncell,
+                                                               int bits, const uint32_t* __restrict__ counts,
+                                                               const int* __restrict__ cell_acc,
+                                                               int* __restrict__ vp_sort) {
+    extern __shared__ __align__(16) uint32_t s_place[];
+    const int half = (ncell + 1) >> 1;                                // words of 16-bit counters a warp
+    uint32_t* const wcnt = s_place;                                   // [warp][half]
+    uint32_t* const first = wcnt + kPlaceWarps * half;                // [ncell]
+    uint16_t* const rank = reinterpret_cast<uint16_t*>(first + ncell);   // [tile]
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i < kPlaceWarps * half; i += kPlaceThreads) wcnt[i] = 0u;
+    for (int c = threadIdx.x; c < ncell; c += kPlaceThreads)
+        first[c] = uint32_t(cell_acc[c]) + counts[size_t(blockIdx.x) * ncell + c];
+    __syncthreads();
+    // each warp ranks a contiguous part of the tile, 32 members at a time
+    const long t0 = long(blockIdx.x) * tile;
+    const int n = int(min(long(tile), N - t0)), part = tile / kPlaceWarps, e0 = w * part, e1 = min(n, e0 + part);
+    uint16_t* const mine = reinterpret_cast<uint16_t*>(wcnt + w * half);
+    const unsigned lt = (1u << lane) - 1u;
+    uint32_t next = e0 + lane < e1 ? uint32_t(vp_cell[t0 + e0 + lane]) : 0u;
+#pragma unroll 1
+    for (int e = e0; e < e1; e += 32) {
+        const bool valid = e + lane < e1;
+        const uint32_t c = next;
+        if (e + 32 + lane < e1) next = uint32_t(vp_cell[t0 + e + 32 + lane]);
+        const uint32_t peers = digit_peers(c, valid, bits), before = __popc(peers & lt);
+        const uint32_t base = valid ? mine[c] : 0u;
+        __syncwarp();
+        if (valid) {
+            if (before == 0u) mine[c] = uint16_t(base + __popc(peers));
+            rank[e + lane] = uint16_t(base + before);
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    // the warps' counts -> the members of the cell in the warps before (two cells a word)
+    for (int i = threadIdx.x; i < half; i += kPlaceThreads) {
+        uint32_t run = 0u;
+#pragma unroll
+        for (int q = 0; q < kPlaceWarps; ++q) {
+            const uint32_t v = wcnt[q * half + i];
+            wcnt[q * half + i] = run;
+            run += v;
+        }
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int e = e0 + lane; e < e1; e += 32) {
+        const uint32_t c = uint32_t(vp_cell[t0 + e]);
+        vp_sort[first[c] + mine[c] + rank[e]] = int(t0 + e);
+    }
 }
 
 __global__ void k_max_key(const int* __restrict__ keys, long n, int* __restrict__ out) {
@@ -385,6 +504,33 @@ int vpmc_hash_build(vpmc_context* ctx, int rshx, int rshy, float Lx, float Ly, i
     if (N == 0) {
         if (cell_num) VPMC_CUDA(cudaMemsetAsync(cell_num, 0, sizeof(int) * size_t(ncell), st));
         VPMC_CUDA(cudaMemsetAsync(cell_acc, 0, sizeof(int) * size_t(ncell), st));
+    } else if (ncell <= kTileCells && N <= kTileMaxN) {
+        // tiles of at least 512 members, a multiple of it, one an SM where they fit
+        const long per = (N + ctx->sm_count - 1) / ctx->sm_count;
+        const int tile = int(std::min<long>(kTileMax, std::max<long>(1, (per + kPlaceThreads - 1) / kPlaceThreads) * kPlaceThreads));
+        const int ntiles = int((N + tile - 1) / tile);
+        Carver dry;
+        dry.take<uint32_t>(size_t(ntiles) * ncell);
+        dry.take<uint32_t>(size_t(ncell));
+        dry.take<uint32_t>(scan_tmp_elems(ncell) + 1);
+        char* base = nullptr;
+        VPMC_TRY(scratch(ctx, SLOT_HASH, dry.off, &base));
+        Carver c{base, 0};
+        uint32_t* const counts = c.take<uint32_t>(size_t(ntiles) * ncell);
+        uint32_t* const total = c.take<uint32_t>(size_t(ncell));
+        uint32_t* const tmp = c.take<uint32_t>(scan_tmp_elems(ncell) + 1);
+        static bool configured[64] = {};
+        if (ctx->device < 64 && !configured[ctx->device]) {
+            VPMC_CUDA(cudaFuncSetAttribute(k_cells_place, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           int(place_smem(kTileCells, kTileMax))));
+            configured[ctx->device] = true;
+        }
+        VPMC_LAUNCH(k_cells_count, ntiles, 1024, 0, st, rshx, rshy, rshx / Lx, rshy / Ly, sub,
+                    reinterpret_cast<const float2*>(pos), long(N), tile, vp_cell, counts);
+        VPMC_LAUNCH(k_cell_columns, (ncell + 31) / 32, 1024, 0, st, counts, ntiles, ncell, total, cell_num);
+        VPMC_TRY(exclusive_scan(ctx, total, reinterpret_cast<uint32_t*>(cell_acc), ncell, tmp, false));
+        VPMC_LAUNCH(k_cells_place, ntiles, kPlaceThreads, place_smem(ncell, tile), st, vp_cell, long(N), tile, ncell,
+                    bits_for(uint64_t(ncell)), counts, cell_acc, vp_sort);
     } else {
         VPMC_LAUNCH(k_cells, blocks_for(N), kHashThreads, 0, st, rshx, rshy, rshx / Lx, rshy / Ly, sub,
                     reinterpret_cast<const float2*>(pos), long(N), vp_cell);
