@@ -60,3 +60,13 @@ def test_forms(cuda, n, m, hw, L, periodic, sign, signed, exclude):
     scale = float(w.abs().max()) * 40 / (7 * math.pi * hw * hw)
     got = torch.where(torch.isnan(got), torch.full_like(got, 1e30), got)
     assert bool(((got - want).abs() <= tol * (torch.nan_to_num(size) + scale)).all())
+
+
+# 2^17 points are the most that are gathered whatever their bins hold, with 2^27 pairs at
+# most in reach: 2,600 particles within h_w = 0.25 and 52,429 points are 2^27
+@pytest.mark.parametrize("n,m,hw,L", [(700, 131072, 0.1, (1.0, 1.0)), (700, 131073, 0.1, (1.0, 1.0)),
+                                      (13038, 52000, 0.25, (1.0, 1.0)), (13038, 53000, 0.25, (1.0, 1.0))])
+@pytest.mark.parametrize("periodic", [True, False])
+@pytest.mark.parametrize("sign,signed,exclude", [(1, False, False), (0, True, True)])
+def test_most_that_is_gathered(cuda, n, m, hw, L, periodic, sign, signed, exclude):
+    test_forms(cuda, n, m, hw, L, periodic, sign, signed, exclude)

@@ -17,10 +17,19 @@ __global__ void k_scale_f32(float* __restrict__ a, long n, float s) {
 // reach of it).  Lanes over the points of a bin (k_eval) leave most lanes idle when
 // a bin holds a few points; here a point costs about 0.6 instructions a visited
 // particle against 0.2 for a full bin of 128 points, so up to kGatherPoints points
-// a bin are gathered.  Needs no binning of the points.  20,011 points in 262,144
+// a bin are gathered, and up to kGatherMost with at most kGatherPairs particles in reach
+// of them in all: so few points leave the device idle when they are binned (h_w 16
+// spacings, the call: 50,000 points in 200^2 particles 316 us binned, 167 gathered;
+// 150,000 in 422^2 332 and 302, 250,000 395 and 405).  Needs no binning of the points.  20,011 points in 262,144
 // particles, h_w = 16 spacings: 224 us binned (half-support cells), 36 us gathered; the
 // whole call 401 -> 143 us.
 constexpr double kGatherPoints = 40.0;
+constexpr long kGatherMost = 1L << 17;
+constexpr double kGatherPairs = double(1L << 27);
+// Binned points take cells a quarter as full as a simulation's samples do (37 points):
+// 476,719 points in 422^2 particles, h_w 16 spacings: 557 -> 424 us, 700,000 in 300^2,
+// h_w 8: 445 -> 338 us.
+constexpr double kBinShare = 4.0;
 constexpr int kGatherRows = 4;   // sub-rows a cell
 constexpr int kQueryRows = 16;   // the same for binned points
 
@@ -202,7 +211,10 @@ int vpmc_query_vorticity(vpmc_context* ctx, int N, const float* pos, const float
                                    : (sign < 0 ? SET_NEG_ONLY : (use_signed ? SET_ONE_SIGNED : SET_ONE_ABS));
     // (the gathered form has no staging wait to give up: a limit of 0 polls keeps the
     // binned one, whose first wait then expires)
-    if (!F && ctx->wait_limit > 0 && double(M) <= kGatherPoints * (2.0 * Lx / h_w) * (2.0 * Ly / h_w)) {
+    const double reach = 3.14159265 * double(N) * h_w * h_w / (double(Lx) * Ly);   // particles within h_w
+    const bool few = double(M) <= kGatherPoints * (2.0 * Lx / h_w) * (2.0 * Ly / h_w) ||
+                     (M <= kGatherMost && double(M) * reach <= kGatherPairs);
+    if (!F && ctx->wait_limit > 0 && few) {
         VPMC_TRY(query_gather(ctx, N, reinterpret_cast<const float2*>(pos), omega, M, reinterpret_cast<const float2*>(pts),
                               set_mode, exclude_center != 0, h_w, Lx, Ly, periodic, out));
         if (sign < 0 && use_signed) VPMC_LAUNCH(k_scale_f32, work_blocks(M), 256, 0, st, out, long(M), -1.0f);
@@ -210,7 +222,7 @@ int vpmc_query_vorticity(vpmc_context* ctx, int N, const float* pos, const float
     }
     Work w;
     // smaller cells and sub-rows trim the walk, as in a simulation's passes
-    VPMC_TRY(setup_work(ctx, SLOT_QUERY, N, h_w, Lx, Ly, periodic, M, 0, &w, F ? 0 : sample_k(N, M, Lx, Ly, h_w), cover,
+    VPMC_TRY(setup_work(ctx, SLOT_QUERY, N, h_w, Lx, Ly, periodic, M, 0, &w, F ? 0 : sample_k(N, kBinShare * M, Lx, Ly, h_w), cover,
                         F != nullptr, kQueryRows));
     VPMC_TRY(grid_build(ctx, w.g, reinterpret_cast<const float2*>(pos), omega, set_mode,
                         reinterpret_cast<const float4*>(F)));
