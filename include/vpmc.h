@@ -181,9 +181,10 @@ int vpmc_query_vorticity(vpmc_context* ctx, int N, const float* pos, const float
                          int use_signed, int exclude_center, float h_w, float Lx,
                          float Ly, int periodic, float* out);
 
-/* The same query with every pair and the sum in FP64 (the plain FP64 GPU path
- * of the query: the FP32 strengths, split exactly into two floats, times the
- * spline evaluated in FP64); isotropic kernels only, no exclude_center.
+/* The same query with every pair and the sum at FP64 accuracy or better (the
+ * FP32 strengths, split exactly into two floats, times the spline; values are
+ * unevaluated sums of three floats, or FP64 where the weights' range or h_w do
+ * not fit those); isotropic kernels only, no exclude_center.
  * out: M doubles (device).  No reference counterpart (an FP64 comparison
  * path for queryVorticityAbs, include/vorticity_query.cuh:15-79). */
 int vpmc_query_vorticity_f64(vpmc_context* ctx, int N, const float* pos, const float* omega,
@@ -429,10 +430,11 @@ int vpmc_sim_set_step(vpmc_sim* sim, uint64_t step);
 uint64_t vpmc_sim_get_step(vpmc_sim* sim);
 
 /* Arithmetic of the MIS step: 32 (default: FP32 pair arithmetic with
- * compensated sums) or 64 (the plain FP64 path of the same estimator: field
- * values, MIS terms, sums and the Euler update in FP64; sample points are
- * drawn as in FP32 mode).  The FP64 path is the baseline the FP32 path is
- * measured against; on GB300 FP64 runs at a small fraction of the FP32 rate. */
+ * compensated sums; densely sampled instances by local expansions) or 64 (the
+ * plain FP64 path of the same estimator: field values at FP64 accuracy or
+ * better in three-float arithmetic, MIS terms, sums and the Euler update in
+ * FP64; sample points are drawn as in FP32 mode).  The FP64 path is the
+ * baseline the FP32 path is measured against. */
 int vpmc_sim_set_precision(vpmc_sim* sim, int bits);
 
 /* Neighbour-walk tuning: cells per h_w (1 <= k <= 8; the walk covers the
