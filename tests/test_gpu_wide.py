@@ -61,3 +61,23 @@ def test_error_is_below_fp64_arithmetic(cuda):
     v = np.where(q <= 0.5, Q(0.5) - 3 * q * q * t, t * t * t) * (w0.astype(Q) + w1.astype(Q))[None]
     want = v.sum(1)
     assert (np.abs(got - want) <= 3 * 2.0 ** -53 * want).all()
+
+
+def test_items_of_either_size(cuda):
+    """A member whose items hold 64 samples alone and 128 in a large ensemble: the same velocities, bit for bit."""
+    from vortexparticlemc_cuda_gb300 import phash as P
+    rng = np.random.default_rng(8)
+    sizes = [64, 300]                     # 1 M and 24 M samples, on either side of 2^24
+    prm = [P.SimParam(dt=1e-3, Nx=s, hwr=3, N1=64, N2=64, seed=s) for s in sizes]
+    parts = [(rng.random((s * s, 2)).astype(np.float32), (rng.normal(size=s * s) / (s * s)).astype(np.float32)) for s in sizes]
+
+    def velocity(which):
+        sim = P.Simulation([prm[i] for i in which], [sizes[i] ** 2 for i in which])
+        sim.set_precision(64)
+        sim.set_particles(*(to_dev(np.concatenate([parts[i][j] for i in which]), cuda) for j in (0, 1)))
+        sim.prepare()
+        v = sim.velocity(3)
+        sim.close()
+        return v
+
+    assert torch.equal(velocity([0, 1])[:64 * 64], velocity([0]))

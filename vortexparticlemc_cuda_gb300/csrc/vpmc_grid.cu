@@ -1994,8 +1994,8 @@ int grid_max_sigma(vpmc_context* ctx, const float4* F, long n, unsigned* d_words
     return VPMC_OK;
 }
 
-void carve_items(Carver& c, long nbins, long max_queries, ItemBufs* it, long n_boxes) {
-    it->max_items = max_queries / query_chunk(1) + (n_boxes < 0 ? nbins : n_boxes) + 1;
+void carve_items(Carver& c, long nbins, long max_queries, ItemBufs* it, long n_boxes, int chunk) {
+    it->max_items = max_queries / chunk + (n_boxes < 0 ? nbins : n_boxes) + 1;
     it->items = c.take<Item>(size_t(it->max_items));
     it->n_items = c.take<uint32_t>(1);
     it->counter = c.take<uint32_t>(1);

@@ -313,8 +313,8 @@ struct ItemBufs {
     uint32_t* scan_tmp = nullptr;
     long max_items = 0;
 };
-// n_boxes: items are made of that many boxes (-1: of bins).
-void carve_items(Carver& c, long nbins, long max_queries, ItemBufs* it, long n_boxes = -1);
+// n_boxes: items are made of that many boxes (-1: of bins); chunk: queries an item (at least).
+void carve_items(Carver& c, long nbins, long max_queries, ItemBufs* it, long n_boxes = -1, int chunk = 128);
 // chunk = queries per item = 256 * queries-per-thread of the eval launch.
 int make_items(vpmc_context* ctx, const GridBufs& g, const uint32_t* qstart, ItemBufs& it, int chunk, long queries);
 int query_chunk(int qpt);

@@ -830,13 +830,18 @@ int alloc_work(vpmc_sim* s) {
     s->chunk_targets = per_chunk;
     const long ns = per_chunk * Q2;
     const size_t nchunks = size_t((s->N + per_chunk - 1) / per_chunk);
+    // FP64 field values: half-full items up to 2^24 samples, where whole ones leave part
+    // of the device idle at the end (64^2 particles 576 -> 492 us a step, 128^2 3.31 -> 3.11
+    // ms, 256^2 11.04 -> 10.92; 512^2, 33 M samples: 41.5 and 41.7 ms; FP32 values lose at
+    // every size, 64^2 155 and 161 us, 256^2 1.20 and 1.31 ms)
+    s->chunk64 = ns <= (1L << 24) ? 64 : query_chunk(4);
     for (auto e : s->chunk_ev) cudaEventDestroy(e);
     s->chunk_ev.assign(2 * nchunks, nullptr);
     for (auto& e : s->chunk_ev) VPMC_CUDA(cudaEventCreate(&e));
     auto carve_all = [&](Carver& c) {
         carve_grid(c, s->N, nb, s->n_inst, &s->g, s->deform != 0, s->rows);
         s->g.cand4 = s->any_box ? c.take<float4>(size_t(s->N)) : nullptr;
-        carve_items(c, nb, ns, &s->it);
+        carve_items(c, nb, ns, &s->it, -1, s->precision == 64 ? s->chunk64 : 128);
         if (s->any_box) carve_items(c, nb, ns, &s->itb, n_boxes);
         carve_queries(c, nb, ns, &s->q, true, s->any_box);
         s->ys = c.take<float2>(size_t(ns));
@@ -928,7 +933,7 @@ int issue_pass(vpmc_sim* s, bool advect, bool timed, int* nlaunch) {
                    s->d_step, t0, nt, s->N1, s->N2, def ? 5 : 1, nullptr, s->ys, s->q.qbin, s->q.qcount,
                    s->q.qsub, s->q.qrank, f64 ? nullptr : s->fv, f64 ? s->fv64 : nullptr, 1};
         VPMC_TRY(launch_gen(st, ga));
-        VPMC_TRY(place_samples(ctx, s->g, s->q, s->ys, ns, s->it, query_chunk(f64 ? 4 : s->qpt), s->any_box ? &s->itb : nullptr));
+        VPMC_TRY(place_samples(ctx, s->g, s->q, s->ys, ns, s->it, f64 ? s->chunk64 : query_chunk(s->qpt), s->any_box ? &s->itb : nullptr));
         EvalLaunch L;
         const bool unb = s->mc[0].law == VPMC_LAW_UNBIASED;
         L.mode = f64 ? (unb ? EVAL_FIELD9_64 : EVAL_FIELD64)

@@ -101,6 +101,7 @@ struct vpmc_sim {
     int N1 = 0, N2 = 0;
     uint64_t step = 0;
     int k_walk = 0, qpt = 4;
+    int chunk64 = 128;                     // queries an item of FP64 field values
     int rows = 32;                     // candidate sub-rows per cell of the evaluation grid
     bool prepared = false;
     // device state
