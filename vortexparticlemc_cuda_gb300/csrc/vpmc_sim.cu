@@ -584,9 +584,11 @@ __global__ void __launch_bounds__(256) k_accum5(Acc5Args a) {
 }
 
 // The plain FP64 path of the same estimator: field values, MIS terms, sums
-// and the Euler update in FP64 (sample points are drawn as in FP32 mode).
-__device__ __forceinline__ double2 mis_term64(int law, float2 xf, float2 yf, double f, double w1, double w2,
-                                              double cum, double alpha, double R, const InstMC& I) {
+// and the Euler update in FP64 (sample points are drawn as in FP32 mode).  The FP64
+// pipe bounds it: the term is one quotient, f cum r / ((w1 f r + w2 alpha cum) 2 pi r^2),
+// instead of three (256^2, 32 + 32 samples: 1.20 -> 1.02 ms).  w2a: w2 alpha.
+__device__ __forceinline__ double2 mis_term64(int law, float2 xf, float2 yf, double f, double w1, double w2a,
+                                              double cum, double R, const InstMC& I) {
     if (!(f > 0.0)) return make_double2(0.0, 0.0);
     const double rx = double(xf.x) - double(yf.x), ry = double(xf.y) - double(yf.y);
     if (law == VPMC_LAW_REFERENCE) {
@@ -596,16 +598,13 @@ __device__ __forceinline__ double2 mis_term64(int law, float2 xf, float2 yf, dou
             wy = ry - round(ry / I.Ly) * I.Ly;
         }
         const double rn = fmax(sqrt(wx * wx + wy * wy), 1e-6);
-        const double inv_r2 = 1.0 / (rx * rx + ry * ry + 1e-8);
-        const double denom = w1 * f / cum + w2 * alpha / rn;
-        const double sc = f / denom * inv_r2 / (2.0 * kPiD);
+        const double sc = f * cum * rn / ((w1 * f * rn + w2a * cum) * (2.0 * kPiD * (rx * rx + ry * ry + 1e-8)));
         return make_double2(-ry * sc, rx * sc);
     }
     const double r2 = rx * rx + ry * ry;
     if (!(r2 > 0.0)) return make_double2(0.0, 0.0);
     const double rn = sqrt(r2);
-    const double p2 = rn < R ? alpha / rn : 0.0;
-    const double sc = f / ((w1 * f / cum + w2 * p2) * (2.0 * kPiD * r2));
+    const double sc = f * cum * rn / ((w1 * f * rn + (rn < R ? w2a * cum : 0.0)) * (2.0 * kPiD * r2));
     return make_double2(-ry * sc, rx * sc);
 }
 
@@ -637,14 +636,13 @@ __global__ void __launch_bounds__(256) k_accum64(AccArgs64 a) {
         const InstMC& I = a.mc[ii];
         const float2 x = a.pos[t];
         const double R = sqrt(double(I.Lx) * I.Lx + double(I.Ly) * I.Ly);
-        const double alpha = 1.0 / (2.0 * kPiD * R);
+        const double w2a = w2 / (2.0 * kPiD * R);
         double u[2][2];
         for (int s = 0; s < 2; ++s) {
             double sx = 0.0, sy = 0.0;
             const long base = (tl * 2 + s) * Q;
             for (int j = lane; j < Q; j += 32) {
-                const double2 c = mis_term64(I.law, x, a.ys[base + j], a.fv[base + j], w1, w2, a.cum64[2 * ii + s],
-                                             alpha, R, I);
+                const double2 c = mis_term64(I.law, x, a.ys[base + j], a.fv[base + j], w1, w2a, a.cum64[2 * ii + s], R, I);
                 sx += c.x;
                 sy += c.y;
             }
