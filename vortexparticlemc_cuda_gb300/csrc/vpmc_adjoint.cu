@@ -34,15 +34,17 @@ using namespace sim;
 // as precise as the forward's FP32 term; the caller accumulates in FP64).
 // The factor 1 - (w1 f / cum) / D of df/f is written as the disk term's share
 // w2 p2 / D, which equals it and has no cancellation when branch 1 dominates.
+// With E = w1 f r + w2a cum = D cum r the term needs the reciprocals of E and r^2
+// alone (w2a: w2 alpha, icum: 1 / cum) instead of eight quotients.
 template <typename R_>
-__device__ __forceinline__ void mis_term_adj(int law, float2 xf, float2 yf, R_ f, R_ w1, R_ w2, R_ cum, R_ alpha,
+__device__ __forceinline__ void mis_term_adj(int law, float2 xf, float2 yf, R_ f, R_ w1, R_ w2a, R_ cum, R_ icum,
                                              R_ R, const InstMC& I, R_ vx, R_ vy, R_& gxx, R_& gxy, R_& df, R_& dc,
                                              R_& cval) {
     gxx = gxy = df = dc = cval = R_(0);
     if (!(f > R_(0))) return;
     const R_ rx = R_(xf.x) - R_(yf.x), ry = R_(xf.y) - R_(yf.y);
     const R_ P = vy * rx - vx * ry;   // v . perp(r)
-    const R_ two_pi = R_(2.0 * kPiD);
+    const R_ i2pi = R_(0.5 / kPiD);
     if (law == VPMC_LAW_REFERENCE) {
         R_ wx = rx, wy = ry;
         if (I.periodic) {
@@ -50,34 +52,32 @@ __device__ __forceinline__ void mis_term_adj(int law, float2 xf, float2 yf, R_ f
             wy = ry - round(ry / R_(I.Ly)) * R_(I.Ly);
         }
         const R_ wn = sqrt(wx * wx + wy * wy);
-        const R_ rn = fmax(wn, R_(1e-6));
+        const R_ rn = fmax(wn, R_(1e-6)), irn = R_(1) / rn;
         const R_ inv = R_(1) / (rx * rx + ry * ry + R_(1e-8));
-        const R_ K = inv / two_pi;
-        const R_ b2 = w2 * alpha / rn;   // the disk term of the denominator
-        const R_ denom = w1 * f / cum + b2;
-        const R_ sc = f / denom;
-        const R_ drx = wn > R_(1e-6) ? wx / wn : R_(0), dry = wn > R_(1e-6) ? wy / wn : R_(0);   // d rn / d r
-        const R_ g = sc / denom * (b2 / rn);                                                       // d sc / d rn
+        const R_ K = inv * i2pi;
+        const R_ own = w1 * f * rn, disk = w2a * cum, iE = R_(1) / (own + disk);
+        const R_ share = disk * iE, iD = cum * rn * iE;   // the disk term's share of the denominator, its reciprocal
+        const R_ sc = f * iD;
+        const R_ g = wn > R_(1e-6) ? sc * share * irn * irn : R_(0);   // d sc / d rn, over rn
         cval = sc * K * P;
-        gxx = sc * K * vy - R_(2) * rx * inv * K * sc * P + K * P * g * drx;
-        gxy = -sc * K * vx - R_(2) * ry * inv * K * sc * P + K * P * g * dry;
-        df = K * P * (b2 / denom) / denom;
-        dc = K * P * sc * (w1 * f / (cum * cum * denom));
+        gxx = sc * K * vy - R_(2) * rx * inv * K * sc * P + K * P * g * wx;
+        gxy = -sc * K * vx - R_(2) * ry * inv * K * sc * P + K * P * g * wy;
+        df = K * P * share * iD;
+        dc = K * P * sc * (own * iE * icum);
         return;
     }
     const R_ r2 = rx * rx + ry * ry;
     if (!(r2 > R_(0))) return;
-    const R_ rn = sqrt(r2);
-    const bool in = rn < R;
-    const R_ p2 = in ? alpha / rn : R_(0);
-    const R_ D = w1 * f / cum + w2 * p2;
-    const R_ sc = f / (D * two_pi * r2);
-    const R_ ex = (in ? -w2 * alpha / (rn * r2) : R_(0)) / D + R_(2) / r2;   // -(d sc / d r) / (sc r)
+    const R_ rn = sqrt(r2), ir2 = R_(1) / r2;
+    const R_ own = w1 * f * rn, disk = rn < R ? w2a * cum : R_(0), iE = R_(1) / (own + disk);
+    const R_ share = disk * iE, A = cum * rn * iE * (ir2 * i2pi);
+    const R_ sc = f * A;
+    const R_ ex = (R_(2) - share) * ir2;   // -(d sc / d r) / (sc r)
     cval = sc * P;
     gxx = sc * vy - P * sc * ex * rx;
     gxy = -sc * vx - P * sc * ex * ry;
-    df = P * (w2 * p2 / D) / (two_pi * r2 * D);
-    dc = P * sc * (w1 * f / (cum * cum * D));
+    df = P * share * A;
+    dc = P * sc * (own * iE * icum);
 }
 
 __device__ __forceinline__ double warp_sum_d(double v) {
@@ -120,8 +120,11 @@ struct AdjSum<true> {
     __device__ __forceinline__ double value() const { return (double(s[0]) + double(s[1])) + double(s[2]); }
 };
 
-// One warp per target: the MIS-term derivatives of all its samples, each in
-// FP32 (F32: the FP32 path) or FP64, the sums as AdjSum, every atomic in FP64.
+// One warp per target at a time: the MIS-term derivatives of all its samples, each in
+// FP32 (F32: the FP32 path) or FP64, the sums as AdjSum, every atomic in FP64.  The
+// FP64 pipe bounds it, so a warp keeps an instance's constants and Omega sums over
+// all its targets (256^2, 32 + 32 samples: 512 -> 230 us a step, with one sum, atomic,
+// root and quotient a target before).
 template <bool F32>
 __global__ void __launch_bounds__(256) k_adj_terms(AdjArgs a) {
     using R_ = typename std::conditional<F32, float, double>::type;
@@ -133,25 +136,50 @@ __global__ void __launch_bounds__(256) k_adj_terms(AdjArgs a) {
     const R_* fg;
     if constexpr (F32) fg = a.fg32;
     else fg = a.fg;
+    // what the warp's targets of one instance share: its constants and its sums
+    int cur = -1;
+    R_ rad = R_(0), w2a = R_(0), cum[2] = {R_(0), R_(0)}, icum[2] = {R_(0), R_(0)};
+    AdjSum<F32> dca[2], csa[2];
+    auto flush = [&]() {
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            const double dcs = warp_sum_d(dca[s].value());
+            if (lane == 0 && dcs != 0.0) atomicAdd(&a.dcum[2 * cur + s], dcs);
+            if (a.gsc) {
+                const double css = warp_sum_d(csa[s].value());
+                if (lane == 0 && css != 0.0) atomicAdd(&a.csum[2 * cur + s], css);
+            }
+            dca[s] = csa[s] = AdjSum<F32>();
+        }
+    };
     for (long tl = warp; tl < a.nt; tl += nwarps) {
         const long t = a.t0 + tl;
         const int ii = inst_of(a.mc, a.n_inst, t);
         const InstMC& I = a.mc[ii];
+        if (ii != cur) {
+            if (cur >= 0) flush();
+            cur = ii;
+            const double R = sqrt(double(I.Lx) * I.Lx + double(I.Ly) * I.Ly);   // as the FP64 path
+            rad = R_(R);
+            w2a = R_(w2 / (2.0 * kPiD * R));
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                cum[s] = R_(a.cum64[2 * ii + s]);
+                icum[s] = R_(1.0 / a.cum64[2 * ii + s]);
+            }
+        }
         const float2 x = a.pos[t];
-        const double R = sqrt(double(I.Lx) * I.Lx + double(I.Ly) * I.Ly);   // as the FP64 path
-        const double alpha = 1.0 / (2.0 * kPiD * R);
         const double mux = double(I.dt) * a.lam_next[2 * t], muy = double(I.dt) * a.lam_next[2 * t + 1];
         AdjSum<F32> ltx, lty;
+#pragma unroll
         for (int s = 0; s < 2; ++s) {
             const double sg = (s == 0 ? inv : -inv);
             const R_ vx = R_(mux * sg), vy = R_(muy * sg);
-            const R_ cum = R_(a.cum64[2 * ii + s]);
             const long base = (tl * 2 + s) * Q;
-            AdjSum<F32> dca, csa;
             for (int j = lane; j < Q; j += 32) {
                 const long sid = base + j;
                 R_ gxx, gxy, df, dc, cv;
-                mis_term_adj<R_>(I.law, x, a.ys[sid], fg[3 * sid], R_(w1), R_(w2), cum, R_(alpha), R_(R), I, vx, vy, gxx,
+                mis_term_adj<R_>(I.law, x, a.ys[sid], fg[3 * sid], R_(w1), w2a, cum[s], icum[s], rad, I, vx, vy, gxx,
                                  gxy, df, dc, cv);
                 const R_ fx = df * fg[3 * sid + 1], fy = df * fg[3 * sid + 2];   // dc/dy = -dc/dx|_f + dc/df grad f
                 ltx.add(gxx);
@@ -170,17 +198,11 @@ __global__ void __launch_bounds__(256) k_adj_terms(AdjArgs a) {
                     }
                     if (a.gsc && p >= 0 && cv != R_(0)) {
                         atomicAdd(&a.gsc[p], double(cv));
-                        csa.add(cv);
+                        csa[s].add(cv);
                     }
                 }
                 a.as[sid] = double(df);
-                dca.add(dc);
-            }
-            const double dcs = warp_sum_d(dca.value());
-            if (lane == 0 && dcs != 0.0) atomicAdd(&a.dcum[2 * ii + s], dcs);
-            if (a.gsc) {
-                const double css = warp_sum_d(csa.value());
-                if (lane == 0 && css != 0.0) atomicAdd(&a.csum[2 * ii + s], css);
+                dca[s].add(dc);
             }
         }
         const double lx = warp_sum_d(ltx.value()), ly = warp_sum_d(lty.value());
@@ -189,6 +211,7 @@ __global__ void __launch_bounds__(256) k_adj_terms(AdjArgs a) {
             atomicAdd(&a.lam[2 * t + 1], ly);
         }
     }
+    if (cur >= 0) flush();
 }
 
 // The transposed sums (by grid slot) onto the particles: dL/domega through the
@@ -302,8 +325,13 @@ int adjoint_step(vpmc_sim* s, AdjBufs& A, const double* lam_in, double* lam_out,
         VPMC_TRY(launch_eval(ctx, s->g, s->q.qrec, s->it, L));
         AdjArgs aa{s->d_mc, s->n_inst, s->pos, s->ys, A.fg, fg32, A.src, s->cum64, t0, nt, s->N1, s->N2, lam_in, lam_out,
                    A.as, A.dcum, score ? A.gsc : nullptr, A.csum};
-        if (f32) VPMC_LAUNCH(k_adj_terms<true>, blocks_for(nt * 32), 256, 0, st, aa);
-        else VPMC_LAUNCH(k_adj_terms<false>, blocks_for(nt * 32), 256, 0, st, aa);
+        // resident CTAs only: each warp keeps its sums over several targets
+        int per_sm = 0;
+        VPMC_CUDA(f32 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adj_terms<true>, 256, 0)
+                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adj_terms<false>, 256, 0));
+        const int terms_grid = std::min(blocks_for(nt * 32), ctx->sm_count * std::max(per_sm, 1));
+        if (f32) VPMC_LAUNCH(k_adj_terms<true>, terms_grid, 256, 0, st, aa);
+        else VPMC_LAUNCH(k_adj_terms<false>, terms_grid, 256, 0, st, aa);
         // transposed sums from the sample side: the same items, each sample
         // weighted by its dc/df, every in-support (sample, particle) pair adding
         // a_s W and a_s dW/dx_p to the particle's slot
