@@ -586,7 +586,8 @@ __global__ void __launch_bounds__(256) k_accum5(Acc5Args a) {
 // The plain FP64 path of the same estimator: field values, MIS terms, sums
 // and the Euler update in FP64 (sample points are drawn as in FP32 mode).  The FP64
 // pipe bounds it: the term is one quotient, f cum r / ((w1 f r + w2 alpha cum) 2 pi r^2),
-// instead of three (256^2, 32 + 32 samples: 1.20 -> 1.02 ms).  w2a: w2 alpha.
+// instead of three, and a
+// target's sums, quotients and update share their instructions (256^2, 32 + 32 samples: 1.20 -> 0.69 ms).  w2a: w2 alpha.
 __device__ __forceinline__ double2 mis_term64(int law, float2 xf, float2 yf, double f, double w1, double w2a,
                                               double cum, double R, const InstMC& I) {
     if (!(f > 0.0)) return make_double2(0.0, 0.0);
@@ -630,50 +631,55 @@ __global__ void __launch_bounds__(256) k_accum64(AccArgs64 a) {
     const long nwarps = (long(gridDim.x) * blockDim.x) >> 5;
     const int Q = a.N1 + a.N2;
     const double w1 = double(a.N1) / Q, w2 = double(a.N2) / Q;
+    // an instance's constants, kept over the warp's targets
+    int cur = -1;
+    double R = 0.0, w2a = 0.0, cum[2] = {0.0, 0.0};
     for (long tl = warp; tl < a.nt; tl += nwarps) {
         const long t = a.t0 + tl;
         const int ii = inst_of(a.mc, a.n_inst, t);
         const InstMC& I = a.mc[ii];
+        if (ii != cur) {
+            cur = ii;
+            R = sqrt(double(I.Lx) * I.Lx + double(I.Ly) * I.Ly);
+            w2a = w2 / (2.0 * kPiD * R);
+            cum[0] = a.cum64[2 * ii];
+            cum[1] = a.cum64[2 * ii + 1];
+        }
         const float2 x = a.pos[t];
-        const double R = sqrt(double(I.Lx) * I.Lx + double(I.Ly) * I.Ly);
-        const double w2a = w2 / (2.0 * kPiD * R);
         double u[2][2];
+#pragma unroll
         for (int s = 0; s < 2; ++s) {
             double sx = 0.0, sy = 0.0;
             const long base = (tl * 2 + s) * Q;
             for (int j = lane; j < Q; j += 32) {
-                const double2 c = mis_term64(I.law, x, a.ys[base + j], a.fv[base + j], w1, w2a, a.cum64[2 * ii + s], R, I);
+                const double2 c = mis_term64(I.law, x, a.ys[base + j], a.fv[base + j], w1, w2a, cum[s], R, I);
                 sx += c.x;
                 sy += c.y;
             }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {   // fixed butterfly, identical on every lane
-                const double ox = __shfl_xor_sync(0xffffffffu, sx, o), oy = __shfl_xor_sync(0xffffffffu, sy, o);
-                const bool lo = (lane & o) == 0;
-                sx = lo ? sx + ox : ox + sx;
-                sy = lo ? sy + oy : oy + sy;
-            }
-            u[s][0] = sx / Q;
-            u[s][1] = sy / Q;
+            u[s][0] = sx;
+            u[s][1] = sy;
         }
-        if (lane == 0) {
-            const double vx = u[0][0] - u[1][0], vy = u[0][1] - u[1][1];
-            a.vel[t] = make_float2(float(vx), float(vy));
+        // the four sums by one butterfly: lanes of bit 16 take a sign each, of bit 8 a
+        // component, so a sum costs an addition and a half; then each lane divides its
+        // own and lanes 0 and 8 update a coordinate each
+        const bool neg = lane & 16, hy = lane & 8;
+        const double ax = neg ? u[0][0] : u[1][0], ay = neg ? u[0][1] : u[1][1];
+        const double sx = (neg ? u[1][0] : u[0][0]) + __shfl_xor_sync(0xffffffffu, ax, 16);
+        const double sy = (neg ? u[1][1] : u[0][1]) + __shfl_xor_sync(0xffffffffu, ay, 16);
+        double v = (hy ? sy : sx) + __shfl_xor_sync(0xffffffffu, hy ? sx : sy, 8);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        v /= Q;
+        v -= __shfl_xor_sync(0xffffffffu, v, 16);   // lanes below 16: u+ - u-
+        if (lane == 0 || lane == 8) {
+            reinterpret_cast<float*>(a.vel)[2 * t + (hy ? 1 : 0)] = float(v);
             if (a.advect) {
-                double nx = double(x.x) + double(I.dt) * vx, ny = double(x.y) + double(I.dt) * vy;
-                float ox, oy;
-                if (I.periodic) {
-                    nx -= floor(nx / double(I.Lx)) * double(I.Lx);
-                    ny -= floor(ny / double(I.Ly)) * double(I.Ly);
-                    ox = float(nx);
-                    oy = float(ny);
-                    if (ox >= I.Lx) ox = 0.f;
-                    if (oy >= I.Ly) oy = 0.f;
-                } else {
-                    ox = float(nx);
-                    oy = float(ny);
-                }
-                a.pos_out[t] = make_float2(ox, oy);
+                const float L = hy ? I.Ly : I.Lx;
+                double nx = double(hy ? x.y : x.x) + double(I.dt) * v;
+                if (I.periodic) nx -= floor(nx / double(L)) * double(L);
+                float ox = float(nx);
+                if (I.periodic && ox >= L) ox = 0.f;
+                reinterpret_cast<float*>(a.pos_out)[2 * t + (hy ? 1 : 0)] = ox;
             }
         }
     }
@@ -954,7 +960,9 @@ int issue_pass(vpmc_sim* s, bool advect, bool timed, int* nlaunch) {
         } else if (f64) {
             AccArgs64 aa{s->d_mc, s->n_inst, s->pos, s->ys, s->fv64, s->cum64, t0, nt, s->N1, s->N2, advect ? 1 : 0,
                          s->vel, pos_out, count_step};
-            VPMC_LAUNCH(k_accum64, blocks_for(nt * 32), 256, 0, st, aa);
+            int per_sm = 0;   // resident CTAs only: a warp keeps an instance's constants
+            VPMC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_accum64, 256, 0));
+            VPMC_LAUNCH(k_accum64, std::min(blocks_for(nt * 32), ctx->sm_count * std::max(per_sm, 1)), 256, 0, st, aa);
         } else {
             AccArgs aa{s->d_mc, s->n_inst, s->pos, s->ys, s->fv, t0, nt, s->N1, s->N2, advect ? 1 : 0, s->vel,
                        pos_out, count_step};
