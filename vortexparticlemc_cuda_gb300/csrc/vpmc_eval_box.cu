@@ -244,8 +244,11 @@ __global__ void __launch_bounds__(kBoxThreads, 24) k_eval_box(EvalBoxArgs a) {
                     s_list[n_list + __popc(pm & lt)] = Cand{lx, lx, ly, ly, c.z, c.z, c2, c2};
                 }
                 n_list += __popc(pm);
-                if (__any_sync(0xffffffffu, reach && !pair)) {
-                    const float w = reach && !pair ? c.z : 0.f;
+                // only the lanes that expand: in the others 1 / c may be infinite (a candidate a
+                // rounding off the box centre) or r no number (one outside an open domain by
+                // 1e19 h), and a weight of 0 would make NaN of it
+                if (reach && !pair) {
+                    const float w = c.z;
                     const bool outer = r > 0.5f;
                     // coefficients of q, q^3 and q^2, times w
                     const float e1 = outer ? -3.f * w : 0.f, e3 = outer ? -w : 3.f * w, k2 = outer ? 3.f * w : -3.f * w;
@@ -357,7 +360,7 @@ __global__ void __launch_bounds__(kBoxThreads, 24) k_eval_box(EvalBoxArgs a) {
             up2(ACC[p], v[0], v[1]);
 #pragma unroll
             for (int s = 0; s < 2; ++s)
-                if (uint32_t(p * 64 + s * 32 + lane) < cnt) a.out[qid[2 * p + s]] = fmaxf(v[s], 0.f);
+                if (uint32_t(p * 64 + s * 32 + lane) < cnt) a.out[qid[2 * p + s]] = v[s] < 0.f ? 0.f : v[s];   // a NaN stays one
         }
         item = __shfl_sync(0xffffffffu, next, 0);
     }
