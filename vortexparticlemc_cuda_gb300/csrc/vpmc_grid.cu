@@ -1869,36 +1869,73 @@ int sample_k(long n, double samples, float Lx, float Ly, float hw, bool boxes) {
 
 int query_chunk(int qpt) { return (qpt == 8 ? 8 : qpt == 6 ? 6 : 4) * kEvalThreads; }   // qpt 1 (tensor cores): 128
 
+namespace {
+// Cells of a plan: the first of kk = k, k - 1, ..., 1 a h_w whose walk does not meet itself
+// (no cells: the domain is too small for any).
+struct Cells {
+    int k = 0, gx = 0, gy = 0;
+};
+Cells plan_cells(const InstDesc& d, double reach, int k) {
+    Cells c;
+    for (c.k = k; c.k >= 1; --c.k) {
+        c.gx = int(std::floor(double(c.k) * double(d.Lx) / reach + 1e-9));
+        c.gy = int(std::floor(double(c.k) * double(d.Ly) / reach + 1e-9));
+        if (!d.periodic || (c.gx >= 2 * c.k + 1 && c.gy >= 2 * c.k + 1)) break;
+    }
+    if (c.k < 1 || c.gx < 1 || c.gy < 1) return Cells{};
+    return c;
+}
+constexpr long kMaxCells = 1L << 24;
+constexpr long kMaxBins = 1L << 31;
+}  // namespace
+
+// The library's own choice of cells decides how fast a sum is, never whether a domain is
+// accepted: that is the default walk's doing, whose cells are taken wherever the chosen
+// ones do not fit (a period of 2.5 to 3 h_w, or an open domain between 0.5 and 1 h_w
+// wide, has room for two cells a h_w and not for one).
 long grid_plan(const InstDesc* in, int n, int k, int nsets, GridInst* out) {
     if (k > kMaxK) k = kMaxK;
-    long base = 0;
+    std::vector<Cells> cells(static_cast<size_t>(n));
+    long bins = 0;
     for (int i = 0; i < n; ++i) {
         const InstDesc& d = in[i];
-        const int k_i = k > 0 ? k : d.k > 0 ? std::min(d.k, kMaxK) : default_k();
         if (!(d.hw > 0.f) || !(d.Lx > 0.f) || !(d.Ly > 0.f)) return -VPMC_ERR_INVALID;
         if (!(d.cover >= 1.f)) return -VPMC_ERR_INVALID;
         const double reach = double(d.hw) * double(d.cover);   // physical support radius to cover
-        int kk = k_i, gx = 0, gy = 0;
-        for (; kk >= 1; --kk) {
-            gx = int(std::floor(double(kk) * double(d.Lx) / reach + 1e-9));
-            gy = int(std::floor(double(kk) * double(d.Ly) / reach + 1e-9));
-            if (!d.periodic || (gx >= 2 * kk + 1 && gy >= 2 * kk + 1)) break;
+        cells[size_t(i)] = plan_cells(d, reach, k > 0 ? k : default_k());
+        const Cells& c = cells[size_t(i)];
+        if (c.k < 1) return -VPMC_ERR_GEOMETRY;
+        if (long(c.gx) * c.gy > kMaxCells) return -VPMC_ERR_CAPACITY;
+        bins += long(nsets) * c.gx * c.gy;
+        if (bins >= kMaxBins) return -VPMC_ERR_CAPACITY;
+    }
+    if (k <= 0)
+        for (int i = 0; i < n; ++i) {
+            if (in[i].k < 1) continue;
+            Cells& c = cells[size_t(i)];
+            const Cells own = plan_cells(in[i], double(in[i].hw) * double(in[i].cover), std::min(in[i].k, kMaxK));
+            const long more = long(nsets) * (long(own.gx) * own.gy - long(c.gx) * c.gy);
+            if (own.k < 1 || long(own.gx) * own.gy > kMaxCells || bins + more >= kMaxBins) continue;
+            c = own;
+            bins += more;
         }
-        if (kk < 1 || gx < 1 || gy < 1) return -VPMC_ERR_GEOMETRY;
-        if (long(gx) * gy > (1L << 24)) return -VPMC_ERR_CAPACITY;
+    long base = 0;
+    for (int i = 0; i < n; ++i) {
+        const InstDesc& d = in[i];
+        const Cells& c = cells[size_t(i)];
         GridInst g{};
         g.Lx = d.Lx;
         g.Ly = d.Ly;
-        g.gx = gx;
-        g.gy = gy;
-        g.inv_sx = float(gx) / d.Lx;
-        g.inv_sy = float(gy) / d.Ly;
-        g.k = kk;
+        g.gx = c.gx;
+        g.gy = c.gy;
+        g.inv_sx = float(c.gx) / d.Lx;
+        g.inv_sy = float(c.gy) / d.Ly;
+        g.k = c.k;
         g.bin_base = int(base);
         g.nsets = nsets;
         g.periodic = d.periodic;
         g.hw = d.hw;
-        g.reach = float(reach);
+        g.reach = float(double(d.hw) * double(d.cover));
         const double h = d.hw;
         g.inv_hw = float(1.0 / h);
         g.A = float(3.0 / (h * h * h));
@@ -1908,14 +1945,13 @@ long grid_plan(const InstDesc* in, int n, int k, int nsets, GridInst* out) {
         g.p_end = d.p_end;
         // h^3 / 2 exactly (72 bits) as three floats: h^2 is exact in FP64, its product
         // with h as a value and an error
-        const double h2 = h * h, c = h2 * h * 0.5, ce = std::fma(h2, h * 0.5, -c);
-        g.half_h3[0] = float(c);
-        g.half_h3[1] = float((c - double(g.half_h3[0])) + ce);
-        g.half_h3[2] = float(((c - double(g.half_h3[0])) - double(g.half_h3[1])) + ce);
+        const double h2 = h * h, hh = h2 * h * 0.5, he = std::fma(h2, h * 0.5, -hh);
+        g.half_h3[0] = float(hh);
+        g.half_h3[1] = float((hh - double(g.half_h3[0])) + he);
+        g.half_h3[2] = float(((hh - double(g.half_h3[0])) - double(g.half_h3[1])) + he);
         g.inv_h3 = 1.0 / (h * h * h);
         out[i] = g;
-        base += long(nsets) * gx * gy;
-        if (base >= (1L << 31)) return -VPMC_ERR_CAPACITY;
+        base += long(nsets) * c.gx * c.gy;
     }
     return base;
 }

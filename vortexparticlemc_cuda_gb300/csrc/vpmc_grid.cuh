@@ -265,7 +265,7 @@ struct InstDesc {
 
 // Plan the grid: fills `out` (n entries) and returns the bin count, or a
 // negative vpmc_status on geometry errors.  k <= 0 selects each instance's own
-// choice.
+// choice; a domain is then accepted exactly where the default walk accepts it.
 long grid_plan(const InstDesc* in, int n, int k, int nsets, GridInst* out);
 int default_k();
 // Walk cells per h_w for an instance of n particles that evaluates `samples` points
