@@ -32,7 +32,8 @@ def velocity(n, walk, F=None, **kw):
 @pytest.mark.parametrize("n,kw", [(64, dict(Nx=8, hwr=3, N1=16, N2=16)), (256, dict(Nx=16, hwr=6, N1=2, N2=2)),
                                   (100, dict(Nx=10, hwr=3.5, N1=64, N2=64)), (121, dict(Nx=11, hwr=4, N1=16, N2=16)),
                                   (4, dict(Nx=2, hwr=3, N1=16, N2=16, periodic=False)),
-                                  (1, dict(Nx=2, hwr=4, N1=16, N2=16, periodic=False))])
+                                  (1, dict(Nx=2, hwr=4, N1=16, N2=16, periodic=False)),
+                                  (1600, dict(Nx=40, hwr=16, N1=1, N2=0))])   # 2.5 h_w, the FP32 h_w a rounding longer
 @pytest.mark.parametrize("law", [0, 1])
 def test_accepted(cuda, n, kw, law):
     got, k = velocity(n, 0, law=law, **kw)

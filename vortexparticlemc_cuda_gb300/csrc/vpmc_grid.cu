@@ -1870,20 +1870,24 @@ int sample_k(long n, double samples, float Lx, float Ly, float hw, bool boxes) {
 int query_chunk(int qpt) { return (qpt == 8 ? 8 : qpt == 6 ? 6 : 4) * kEvalThreads; }   // qpt 1 (tensor cores): 128
 
 namespace {
-// Cells of a plan: the first of kk = k, k - 1, ..., 1 a h_w whose walk does not meet itself
-// (no cells: the domain is too small for any).
+// Cells of a plan: the first of k, k - 1, ..., 1 a h_w whose walk does not meet itself (no
+// cells: the domain is too small for any).  Where none fits, once more with h_w 2^-22
+// shorter: h_w = (Lx / Nx) hwr carries up to two FP32 roundings, and a period of 2.5 h_w
+// is not refused for them (pairs in the sliver have no FP32 weight).
 struct Cells {
     int k = 0, gx = 0, gy = 0;
 };
 Cells plan_cells(const InstDesc& d, double reach, int k) {
-    Cells c;
-    for (c.k = k; c.k >= 1; --c.k) {
-        c.gx = int(std::floor(double(c.k) * double(d.Lx) / reach + 1e-9));
-        c.gy = int(std::floor(double(c.k) * double(d.Ly) / reach + 1e-9));
-        if (!d.periodic || (c.gx >= 2 * c.k + 1 && c.gy >= 2 * c.k + 1)) break;
+    for (const double r : {reach, reach * (1.0 - 0x1p-22)}) {
+        Cells c;
+        for (c.k = k; c.k >= 1; --c.k) {
+            c.gx = int(std::floor(double(c.k) * double(d.Lx) / r + 1e-9));
+            c.gy = int(std::floor(double(c.k) * double(d.Ly) / r + 1e-9));
+            if (!d.periodic || (c.gx >= 2 * c.k + 1 && c.gy >= 2 * c.k + 1)) break;
+        }
+        if (c.k >= 1 && c.gx >= 1 && c.gy >= 1) return c;
     }
-    if (c.k < 1 || c.gx < 1 || c.gy < 1) return Cells{};
-    return c;
+    return Cells{};
 }
 constexpr long kMaxCells = 1L << 24;
 constexpr long kMaxBins = 1L << 31;
