@@ -416,7 +416,13 @@ int vpmc_sim_freeze_sampling(vpmc_sim* sim, int on);
  * target's samples depend only on its instance, its instance-local index and
  * the step (the Philox counter), so a shard's velocities and positions are
  * bit-identical to the whole run's as long as all positions agree: a sharded
- * run on several GPUs all-gathers the updated positions after each step.
+ * run on several GPUs all-gathers the updated positions after each step.  Both
+ * must sum on the same grid: with a walk given to vpmc_sim_set_tuning they
+ * always do; with the library's choice (0) unless the shard draws fewer than
+ * 32 samples of a sign in a box of the local expansions, or 64 in a bin, on
+ * average, where it takes the grid that suits its own samples and agrees with
+ * the whole run to FP32 rounding.  (Setting a range may therefore re-plan and
+ * grow the working set, as vpmc_sim_set_tuning does.)
  * Particles outside the range keep their positions and velocities.  Not with
  * deformation mode or the adjoint (VPMC_ERR_UNSUPPORTED).  Default: [0, N).
  * No reference counterpart (the reference runs on one GPU). */

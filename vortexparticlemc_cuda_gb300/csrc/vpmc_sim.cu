@@ -803,27 +803,65 @@ int upload_mc(vpmc_sim* s) {
     return VPMC_OK;
 }
 
+// The evaluation grid of every instance: cells, and boxes where densely sampled instances
+// are summed by them (plain FP32 kernels, the default 4 queries a thread).  Returns the bin
+// count or a negative status.
+//
+// Cells and boxes are chosen by the samples of a whole run, so that a shard of one sums as
+// the run does, bit for bit.  Where the walk is the library's choice, that holds for as
+// long as it pays with the samples the shard draws: with fewer than kBoxSamples a box, or
+// kShardSamples a bin, it chooses by its own, never fewer cells than the default walk
+// unless the run has fewer.  A pass over 1 / 8 of 1024^2 targets, h_w 16 spacings, 64 + 64
+// samples: 26.1 ms with the run's boxes (7 samples each), 11.4 with its own cells; 1 / 16:
+// 24.6 and 6.4; 1 / 16 of the same with h_w 8, 32 + 32: 2.16 ms with the run's cells (28 a
+// bin), 1.80 with its own, 1 / 8 (57 a bin) 3.03 and 2.85, 1 / 4 (114) 4.91 and 4.85.
+constexpr double kShardSamples = 64.0;
+long plan_instances(const vpmc_sim* s, std::vector<GridInst>& plan) {
+    const bool can_box = s->precision == 32 && !s->deform && s->qpt == 4;
+    const double per = double(samples_per(s)), most = double(1L << 29);   // a sign set's samples in a pass
+    std::vector<InstDesc> d(s->n_inst);
+    std::vector<double> drawn(s->n_inst), by(s->n_inst);
+    for (int i = 0; i < s->n_inst; ++i) {
+        const long b = s->begin[i], e = b + s->counts[i];
+        const long own = std::max(0L, std::min(e, s->t_end) - std::max(b, s->t_begin));
+        drawn[i] = std::min(double(own) * per, most);
+        by[i] = std::min(double(s->counts[i]) * per, most);
+        d[i] = InstDesc{s->prm[i].Lx, s->prm[i].Ly, s->mc[i].hw, s->prm[i].periodic, int(b), int(e),
+                        s->deform ? s->cover : 1.f,
+                        sample_k(s->counts[i], by[i], s->prm[i].Lx, s->prm[i].Ly, s->mc[i].hw, can_box)};
+    }
+    auto boxes = [&](const GridInst& g, int i) {
+        return can_box ? box_split(s->counts[i], by[i], g.Lx, g.Ly, g.hw, g.gx, g.gy) : 0;
+    };
+    plan.resize(s->n_inst);
+    long nb = grid_plan(d.data(), s->n_inst, s->k_walk, 2, plan.data());
+    if (nb < 0) return nb;
+    bool again = false;
+    for (int i = 0; i < s->n_inst; ++i) {
+        GridInst& g = plan[i];
+        g.nb = boxes(g, i);
+        const double bins = double(g.gx) * g.gy;
+        if (s->k_walk || drawn[i] <= 0.0 || drawn[i] >= bins * (g.nb ? kBoxSamples * g.nb * g.nb : kShardSamples) ||
+            drawn[i] >= by[i])
+            continue;
+        by[i] = drawn[i];
+        d[i].k = std::max(sample_k(s->counts[i], by[i], g.Lx, g.Ly, g.hw, can_box), std::min(d[i].k, default_k()));
+        again = true;
+    }
+    if (!again) return nb;
+    nb = grid_plan(d.data(), s->n_inst, s->k_walk, 2, plan.data());
+    for (int i = 0; nb >= 0 && i < s->n_inst; ++i) plan[i].nb = boxes(plan[i], i);
+    return nb;
+}
+
 // Working set sized for the largest chunk (samples <= max_samples).
 int alloc_work(vpmc_sim* s) {
     vpmc_context* ctx = s->ctx;
-    std::vector<InstDesc> d(s->n_inst);
-    // instances that sample densely enough are summed by boxes (plain FP32 kernels, the
-    // default 4 queries a thread)
-    const bool can_box = s->precision == 32 && !s->deform && s->qpt == 4;
-    for (int i = 0; i < s->n_inst; ++i)
-        d[i] = InstDesc{s->prm[i].Lx, s->prm[i].Ly, s->mc[i].hw, s->prm[i].periodic, int(s->begin[i]),
-                        int(s->begin[i] + s->counts[i]), s->deform ? s->cover : 1.f,
-                        sample_k(s->counts[i], std::min(double(s->counts[i]) * samples_per(s), double(1L << 29)),
-                                 s->prm[i].Lx, s->prm[i].Ly, s->mc[i].hw, can_box)};
-    s->plan.resize(s->n_inst);
-    const long nb = grid_plan(d.data(), s->n_inst, s->k_walk, 2, s->plan.data());
+    const long nb = plan_instances(s, s->plan);
     if (nb < 0) return int(-nb);
     s->any_box = s->any_pair = false;
     long n_boxes = 0;
-    for (int i = 0; i < s->n_inst; ++i) {
-        GridInst& g = s->plan[i];
-        if (can_box)
-            g.nb = box_split(s->counts[i], std::min(double(s->counts[i]) * samples_per(s), double(1L << 29)), g.Lx, g.Ly, g.hw, g.gx, g.gy);
+    for (const GridInst& g : s->plan) {
         (g.nb ? s->any_box : s->any_pair) = true;
         n_boxes += 2L * g.gx * g.gy * g.nb * g.nb;
     }
@@ -1375,12 +1413,29 @@ int vpmc_sim_set_precision(vpmc_sim* s, int bits) {
 int vpmc_sim_set_target_range(vpmc_sim* s, long long begin, long long end) {
     if (!s || begin < 0 || end > s->N || begin >= end) return VPMC_ERR_INVALID;
     if (s->deform && (begin != 0 || end != s->N)) return VPMC_ERR_UNSUPPORTED;
+    const long old_begin = s->t_begin, old_end = s->t_end;
     s->t_begin = long(begin);
     s->t_end = long(end);
     s->ys_t0 = -1;
     s->ys_nt = 0;
     drop_graphs(s);   // the captured passes cover the old range (the chunk events cover all N)
-    return VPMC_OK;
+    // another grid where the range's samples ask for one (plan_instances)
+    std::vector<GridInst> plan;
+    const long nb = plan_instances(s, plan);
+    const bool same = nb >= 0 && std::equal(plan.begin(), plan.end(), s->plan.begin(), s->plan.end(),
+                                            [](const GridInst& a, const GridInst& b) {
+                                                return a.k == b.k && a.gx == b.gx && a.gy == b.gy && a.nb == b.nb;
+                                            });
+    if (same) return VPMC_OK;
+    VPMC_CUDA(cudaSetDevice(s->ctx->device));
+    const int rc = nb < 0 ? int(-nb) : alloc_work(s);
+    if (rc != VPMC_OK) {
+        s->t_begin = old_begin;
+        s->t_end = old_end;
+        (void)alloc_work(s);
+        return rc;
+    }
+    return vpmc_context_sync(s->ctx);
 }
 
 int vpmc_sim_get_target_range(vpmc_sim* s, long long* begin, long long* end) {

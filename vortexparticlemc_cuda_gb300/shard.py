@@ -8,7 +8,11 @@ after each step the ranks all-gather the shards' updated positions, so every
 replica holds all positions again before the next step.  That all-gather is
 the path's one exchange (8 bytes per particle per step).  A sample's Philox
 counter is keyed by its target's instance-local index and the step, so a
-sharded run gives, bit for bit, the positions of the one-GPU run.
+sharded run gives, bit for bit, the positions of the one-GPU run in the same
+explicit tuning.  With the library's own choice of walk it does as long as a
+rank's samples are dense enough for the whole run's grid (32 of a sign in each
+box of the local expansions, 64 in each bin); a thinner shard takes the grid
+that suits its samples and agrees to FP32 rounding.
 
 Ensembles: instances are independent, so they are split over ranks by
 particle count with no collective at all.
