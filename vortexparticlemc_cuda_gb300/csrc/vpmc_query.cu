@@ -152,9 +152,9 @@ int query_gather(vpmc_context* ctx, long N, const float2* pos, const float* omeg
     const double density = double(N) / (double(Lx) * Ly);
     const int k = int(std::min(3.0, std::max(1.0, 2.0 * double(hw) * hw * density / 48.0)));
     InstDesc d{Lx, Ly, hw, periodic, 0, int(N)};
+    d.k = double(k) * Lx / hw * k * Ly / hw <= double(1L << 22) ? k : 1;
     GridInst plan;
-    long nb = grid_plan(&d, 1, 0, 1, &plan);   // what the default walk refuses is refused
-    if (nb > 0) nb = grid_plan(&d, 1, std::min(k, double(k) * Lx / hw * k * Ly / hw <= double(1L << 22) ? k : 1), 1, &plan);
+    const long nb = grid_plan(&d, 1, 0, 1, &plan);
     if (nb < 0) return int(-nb);
     GridBufs g;
     float4* rec = nullptr;

@@ -22,10 +22,11 @@ inline int work_blocks(long n) {
     return int(b);
 }
 
+// k: walk cells per h_w the caller would like (0: the default walk's).
 inline int setup_work(vpmc_context* ctx, int slot, long N, float hw, float Lx, float Ly, int periodic, long M, int nvec,
                       Work* w, int k = 0, float cover = 1.f, bool deformed = false, int rows = 1) {
-    InstDesc d{Lx, Ly, hw, periodic, 0, int(N), cover};
-    const long nb = grid_plan(&d, 1, k, 1, &w->plan);
+    InstDesc d{Lx, Ly, hw, periodic, 0, int(N), cover, k};
+    const long nb = grid_plan(&d, 1, 0, 1, &w->plan);
     if (nb < 0) return int(-nb);
     const long nq = M > N ? M : N;
     auto carve_all = [&](Carver& c) {
