@@ -85,6 +85,10 @@ uint64_t vpmc_kernel_launch_count(void);
  * latency), then the kernel lets the copy in flight land, stops, and the call
  * returns VPMC_ERR_TIMEOUT with the context still usable.  0 makes every such
  * wait give up at once: a way to exercise that error path without a fault.
+ * Every call that sums on the evaluation grid is bounded so (queries, RBF
+ * products and fits, simulation passes and adjoints); where it would take a
+ * form without such waits (gathered queries, fits with a kept matrix), a limit
+ * of 0 selects the staged form, and boxed passes end with the status.
  * No reference counterpart (its only device check is an unused trap,
  * src/utilities.cu:99-103). */
 #define VPMC_WAIT_LIMIT_DEFAULT (1u << 26)

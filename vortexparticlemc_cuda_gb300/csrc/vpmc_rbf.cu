@@ -533,7 +533,9 @@ int begin(vpmc_context* ctx, Solver& s, int N, const float* pos, const float* b,
     // particles spread evenly have N pi h^2 / (Lx Ly) neighbours: a matrix far
     // from fitting by that is not counted
     const double even = double(N) * std::min(1.0, kPiD * h_w * h_w / (double(Lx) * Ly));
-    if (double(N) * even * 12.0 <= 2.0 * double(kMaxMatrixBytes)) {
+    // (a kept matrix has no staging wait to give up: a limit of 0 polls takes the products
+    // that form the values, whose first wait then expires)
+    if (ctx->wait_limit > 0 && double(N) * even * 12.0 <= 2.0 * double(kMaxMatrixBytes)) {
         VPMC_LAUNCH(k_rbf_rows<false>, grid, kThreads, 0, st, w.g.inst, w.g.cstart, w.g.cand, long(N), A, ctx->d_flags);
         unsigned long long total = 0;
         VPMC_CUDA(cudaMemcpyAsync(&total, A.cursor, sizeof(total), cudaMemcpyDeviceToHost, st));
