@@ -1463,10 +1463,13 @@ int vpmc_sim_set_tuning(vpmc_sim* s, int k_walk, int qpt) {
 // Autotuner: time one full velocity pass (gen + bin + eval + accumulate) for
 // each candidate (cells per h_w, queries per thread) and keep the fastest.
 // Results are cached in-process by (hwr, samples per target, particles per
-// h_w^2 of instance 0), so a second simulation of the same shape reuses them.
+// h_w^2 of instance 0, precision, share of the targets that a pass takes), so a
+// second simulation of the same shape reuses them: what FP64 values or a shard's
+// thinner bins are fastest with is not what a whole FP32 run is (which may take
+// local expansions).
 namespace {
 std::mutex g_tune_mu;
-std::map<std::tuple<int, int, int>, std::pair<int, int>> g_tune_cache;
+std::map<std::tuple<int, int, int, int, int>, std::pair<int, int>> g_tune_cache;
 }  // namespace
 
 int vpmc_sim_autotune(vpmc_sim* s, int* k_out, int* qpt_out, float* best_ms) {
@@ -1476,7 +1479,8 @@ int vpmc_sim_autotune(vpmc_sim* s, int* k_out, int* qpt_out, float* best_ms) {
     const vpmc_sim_params& p = s->prm[0];
     const double density = double(s->counts[0]) / (double(p.Lx) * p.Ly) * double(s->mc[0].hw) * s->mc[0].hw;
     const auto key = std::make_tuple(int(std::lround(p.hwr * 16 * (s->deform ? s->cover : 1.f))),
-                                     int(samples_per(s)) * (s->deform ? -1 : 1), int(std::lround(density)));
+                                     int(samples_per(s)) * (s->deform ? -1 : 1), int(std::lround(density)),
+                                     s->precision, int(std::lround(256.0 * double(s->t_end - s->t_begin) / double(s->N))));
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         auto it = g_tune_cache.find(key);
