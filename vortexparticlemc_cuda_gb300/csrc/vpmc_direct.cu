@@ -411,8 +411,9 @@ __global__ void __launch_bounds__(kDT, 2) k_direct_wide(const float2* __restrict
 // the rounding of the FP32 differences is most of it, with either reciprocal).
 // 40,000 targets x 40,000 sources: 3,217 -> 697 us, 29.8 TFLOP/s at 13 flop a pair.
 // A tile with a source (or a block with a target) many periods away (2^20, or
-// 256 where the product with 1/L is rounded) or with a strength that could
-// overflow against e2 takes the general arithmetic.
+// 256 where the product with 1/L is rounded), without periods 2^61 away (beyond,
+// r2 may pass 2^126, whose reciprocal the estimate flushes to 0), or with a
+// strength that could overflow against e2 takes the general arithmetic.
 constexpr int kPT = 128;          // threads
 constexpr int kPTargets = 4;      // targets a thread
 constexpr int kPTile = 64;        // sources a tile
@@ -456,7 +457,8 @@ __global__ void __launch_bounds__(kPT) k_plummer_f32(const float2* __restrict__ 
     const long s0 = c * chunk, s1 = min(N, s0 + chunk);
     const long m0 = long(blockIdx.x) * (kPT * kPTargets) + threadIdx.x;
     const float e2 = param * param, inv2pi = 1.f / (2.f * kPiF), iLx = 1.f / Lx, iLy = 1.f / Ly;
-    constexpr float kFar = kExact ? 1048576.f : 256.f;   // periods
+    constexpr float kFar = !kPeriodic ? 0x1p61f : kExact ? 1048576.f : 256.f;   // periods, or lengths without them
+    const float ux = kPeriodic ? iLx : 1.f, uy = kPeriodic ? iLy : 1.f;
     const float wmax = 3.0e38f * fminf(e2, 1.f);
     float2 x[kPTargets];
     int self[kPTargets];
@@ -466,7 +468,7 @@ __global__ void __launch_bounds__(kPT) k_plummer_f32(const float2* __restrict__ 
         const long m = m0 + long(j) * kPT;
         self[j] = m < M ? tidx[m] : -1;
         x[j] = m < M ? pos[self[j]] : make_float2(0.f, 0.f);
-        if (kPeriodic) far |= !(fabsf(x[j].x) * iLx < kFar && fabsf(x[j].y) * iLy < kFar);
+        far |= !(fabsf(x[j].x) * ux < kFar && fabsf(x[j].y) * uy < kFar);
     }
     f2x X[2], Y[2], U[2], V[2];
 #pragma unroll
@@ -485,7 +487,7 @@ __global__ void __launch_bounds__(kPT) k_plummer_f32(const float2* __restrict__ 
             const float w = om[t0 + threadIdx.x] * inv2pi;
             src[threadIdx.x] = PSrc{-p.x, -p.x, -p.y, -p.y, w, w, 0.f, 0.f};
             general |= !(fabsf(w) <= wmax);
-            if (kPeriodic) general |= !(fabsf(p.x) * iLx < kFar && fabsf(p.y) * iLy < kFar);
+            general |= !(fabsf(p.x) * ux < kFar && fabsf(p.y) * uy < kFar);
         }
         f2x tu[2] = {ZERO, ZERO}, tv[2] = {ZERO, ZERO};
         if (!__syncthreads_or(general)) {
@@ -639,10 +641,12 @@ extern "C" int vpmc_direct_velocity_f32(vpmc_context* ctx, int kernel, int N, co
     if (kernel == VPMC_DIRECT_MOLLIFIED && !(param > 0.f)) return VPMC_ERR_INVALID;
     VPMC_CUDA(cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->stream;
-    // the packed Plummer kernel wants r2 + e2 in the reciprocal's normal range
-    // (e2 bounds it below); a smaller or huge core keeps the IEEE quotients
+    // the packed Plummer kernel wants r2 + e2 in the reciprocal's normal range (e2
+    // bounds it below, the period above); a smaller or huge core and a huge period
+    // keep the IEEE quotients
     const float e2 = param * param;
-    const bool packed = kernel == VPMC_DIRECT_PLUMMER && e2 >= 1e-30f && e2 <= 1e30f;
+    const bool packed = kernel == VPMC_DIRECT_PLUMMER && e2 >= 1e-30f && e2 <= 1e30f &&
+                        !(periodic && std::max(Lx, Ly) > 0x1p61f);
     const long per_block = packed ? long(kPT) * kPTargets : long(kDT);
     const long tile = packed ? kPTile : kTileSrc;
     const long tblocks = (long(M) + per_block - 1) / per_block;
