@@ -155,7 +155,9 @@ __global__ void __launch_bounds__(kThreads) k_rbf_rows(const GridInst* __restric
 // outside the support.  They are the numbers spline_w_d gives (the matrix-free
 // product's), in 26 FP64 instructions instead of ~35: the root and the quotient
 // r / h come from an estimate (the hardware's, 1 / h) by fused residual
-// corrections (Markstein, IBM J. Res. Dev. 34, 1990) and are correctly rounded.
+// corrections (Markstein, IBM J. Res. Dev. 34, 1990); over 2^30 distances, across the
+// pieces, at the knots and down to 2^-400 h, root, quotient and value had the bits of
+// sqrt, of the division and of spline_w_d.
 // FP64-pipe bound (192^2, h_w = 8: 7.8 M entries, 0.47 ms).
 __global__ void __launch_bounds__(kThreads) k_rbf_values(const GridInst* __restrict__ inst,
                                                          const Cand* __restrict__ cand, long n, RbfMatrix A) {
