@@ -326,7 +326,12 @@ struct AccArgs {
     float2* vel;
     float2* pos_out;              // may be pos: a target reads only its own
     unsigned long long* step;     // stepped by this launch, or nullptr
+    const unsigned* flags;        // FLAG_TIMEOUT: the field values were not all written
 };
+
+// The samples a sum may read: none after an evaluation that gave up (the particles then
+// stay where they are, and the call returns the timeout).
+__device__ __forceinline__ int sampled(const unsigned* flags, int n) { return (*flags & FLAG_TIMEOUT) ? 0 : n; }
 
 // mis_contrib_dev (src/cuda/monte_carlo_bs.cu:35-51) for the reference law;
 // the balance-heuristic estimator with the true sampling densities for the
@@ -378,7 +383,7 @@ __global__ void __launch_bounds__(256) k_accum(AccArgs a) {
     constexpr int kPerWarp = 32 / kAccLanes;
     const long warp = (long(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const long nwarps = (long(gridDim.x) * blockDim.x) >> 5;
-    const int Q = a.N1 + a.N2;
+    const int Q = a.N1 + a.N2, nq = sampled(a.flags, Q);
     const float w1 = float(a.N1) / float(Q), w2 = float(a.N2) / float(Q);
     const float inv = 1.f / float(Q);
     // the loop runs the same trips in every lane of a warp (the group sums shuffle)
@@ -395,7 +400,7 @@ __global__ void __launch_bounds__(256) k_accum(AccArgs a) {
             KSum sx, sy;
             const long base = (tl * 2 + s) * Q;
             const float cum = I.cum9[s], inv_cum = 1.f / cum;
-            for (int j0 = sub; j0 < Q; j0 += 4 * kAccLanes) {
+            for (int j0 = sub; j0 < nq; j0 += 4 * kAccLanes) {
                 float2 y[4];
                 float f[4];
 #pragma unroll
@@ -469,6 +474,7 @@ struct Acc5Args {
     unsigned* sig;         // [0] = max sigma_max(F_out) (float bits), [1] = targets with sigma_max > cap
     float cap;
     unsigned long long* step;
+    const unsigned* flags;
 };
 
 __global__ void __launch_bounds__(256) k_accum5(Acc5Args a) {
@@ -477,7 +483,7 @@ __global__ void __launch_bounds__(256) k_accum5(Acc5Args a) {
     constexpr int kPerWarp = 32 / kAccLanes;
     const long warp = (long(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const long nwarps = (long(gridDim.x) * blockDim.x) >> 5;
-    const int Q = a.N1 + 5 * a.N2;
+    const int Q = a.N1 + 5 * a.N2, n1 = sampled(a.flags, a.N1), n2 = sampled(a.flags, a.N2);
     const float w1 = float(a.N1) / float(a.N1 + a.N2), w2 = float(a.N2) / float(a.N1 + a.N2);
     const float inv = 1.f / float(a.N1 + a.N2);
     // the loop runs the same trips in every lane of a warp (the group sums shuffle)
@@ -503,7 +509,7 @@ __global__ void __launch_bounds__(256) k_accum5(Acc5Args a) {
             const long base = (tl * 2 + s) * Q;
             const float cum = I.cum9[s], inv_cum = 1.f / cum;
 #pragma unroll 2
-            for (int j = sub; j < a.N1; j += kAccLanes) {
+            for (int j = sub; j < n1; j += kAccLanes) {
                 const float2 y = live ? a.ys[base + j] : make_float2(0.f, 0.f);
                 const float f = live ? a.fv[base + j] : 0.f;
 #pragma unroll
@@ -517,7 +523,7 @@ __global__ void __launch_bounds__(256) k_accum5(Acc5Args a) {
             for (int k = 0; k < 5; ++k) {
                 const long b0 = base + a.N1 + long(k) * a.N2;
 #pragma unroll 2
-                for (int j = sub; j < a.N2; j += kAccLanes) {
+                for (int j = sub; j < n2; j += kAccLanes) {
                     const float2 y = live ? a.ys[b0 + j] : make_float2(0.f, 0.f);
                     const float f = live ? a.fv[b0 + j] : 0.f;
                     const float2 c = mis_term(I.law, xa[k], y, f, w1, w2, cum, inv_cum, alpha[k], R[k], I, inv_Lx, inv_Ly);
@@ -622,6 +628,7 @@ struct AccArgs64 {
     float2* vel;
     float2* pos_out;
     unsigned long long* step;
+    const unsigned* flags;
 };
 
 __global__ void __launch_bounds__(256) k_accum64(AccArgs64 a) {
@@ -629,7 +636,7 @@ __global__ void __launch_bounds__(256) k_accum64(AccArgs64 a) {
     const int lane = threadIdx.x & 31;
     const long warp = (long(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const long nwarps = (long(gridDim.x) * blockDim.x) >> 5;
-    const int Q = a.N1 + a.N2;
+    const int Q = a.N1 + a.N2, nq = sampled(a.flags, Q);
     const double w1 = double(a.N1) / Q, w2 = double(a.N2) / Q;
     // an instance's constants, kept over the warp's targets
     int cur = -1;
@@ -651,7 +658,7 @@ __global__ void __launch_bounds__(256) k_accum64(AccArgs64 a) {
         for (int s = 0; s < 2; ++s) {
             double sx = 0.0, sy = 0.0;
             const long base = (tl * 2 + s) * Q;
-            for (int j = lane; j < Q; j += 32) {
+            for (int j = lane; j < nq; j += 32) {
                 const double2 c = mis_term64(I.law, x, a.ys[base + j], a.fv[base + j], w1, w2a, cum[s], R, I);
                 sx += c.x;
                 sy += c.y;
@@ -993,17 +1000,17 @@ int issue_pass(vpmc_sim* s, bool advect, bool timed, int* nlaunch) {
         unsigned long long* const count_step = advect && t0 + nt >= s->t_end ? s->d_step : nullptr;
         if (def) {
             Acc5Args aa{s->d_mc, s->n_inst, s->pos, s->ys, s->fv, t0, nt, s->N1, s->N2, advect ? 1 : 0, s->vel,
-                        s->vel5, pos_out, F_out, s->d_sig, kCoverCap, count_step};
+                        s->vel5, pos_out, F_out, s->d_sig, kCoverCap, count_step, ctx->d_flags};
             VPMC_LAUNCH(k_accum5, blocks_for(nt * kAccLanes), 256, 0, st, aa);
         } else if (f64) {
             AccArgs64 aa{s->d_mc, s->n_inst, s->pos, s->ys, s->fv64, s->cum64, t0, nt, s->N1, s->N2, advect ? 1 : 0,
-                         s->vel, pos_out, count_step};
+                         s->vel, pos_out, count_step, ctx->d_flags};
             int per_sm = 0;   // resident CTAs only: a warp keeps an instance's constants
             VPMC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_accum64, 256, 0));
             VPMC_LAUNCH(k_accum64, std::min(blocks_for(nt * 32), ctx->sm_count * std::max(per_sm, 1)), 256, 0, st, aa);
         } else {
             AccArgs aa{s->d_mc, s->n_inst, s->pos, s->ys, s->fv, t0, nt, s->N1, s->N2, advect ? 1 : 0, s->vel,
-                       pos_out, count_step};
+                       pos_out, count_step, ctx->d_flags};
             VPMC_LAUNCH(k_accum, blocks_for(nt * kAccLanes), 256, 0, st, aa);
         }
     }
