@@ -208,7 +208,13 @@ int vpmc_rbf_matvec(vpmc_context* ctx, int N, const float* pos, const float* x, 
  * iterations.  Dot products and norms are FP64.  omega_out (device) receives
  * w.  info (HOST, may be NULL) receives {iterations, recursive |r|/|b|,
  * true |b - A w|/|b| recomputed with the FP64 SpMV}.  Returns
- * VPMC_ERR_NOT_CONVERGED (with omega_out written) when max_iter is reached. */
+ * VPMC_ERR_NOT_CONVERGED (with omega_out written) when max_iter is reached.
+ * Device memory, this solver and MINRES: the matrix's in-support entries are
+ * kept for the solve at 12 bytes each where they take at most 4 GB (the
+ * allocation adds a quarter, so up to 5 GB); with more, or where that much
+ * cannot be allocated, every product forms them again.  An allocation above
+ * 512 MB is given back at the end, a smaller one stays in the context's
+ * scratch for the next solve. */
 int vpmc_cg_rbf(vpmc_context* ctx, int N, const float* pos, const float* b,
                 float* omega_out, float h_w, float Lx, float Ly, int periodic,
                 double tol, int max_iter, double* info);
@@ -396,10 +402,12 @@ int vpmc_sim_vorticity_grid(vpmc_sim* sim, int inst, int res_x, int res_y, int s
  *     in the recorded final state.  The trajectory is the forward's (its
  *     precision); the adjoint's field values and gradients at the samples,
  *     its transposed sums and its MIS-term derivatives take their terms in
- *     the forward's precision (for the FP32 path: FP32 pairs summed into
- *     FP64 per candidate run, the transposed sums compensated in FP32 per
- *     work item, FP32 MIS-term derivatives); every accumulation across
- *     runs, items and samples is FP64.
+ *     the forward's precision (for the FP32 path: FP32 pairs, their run sums
+ *     added as three floats, which keep more digits than FP64, and a sample's
+ *     value and gradient rounded once to FP32; the transposed sums compensated
+ *     in FP32 per work item; FP32 MIS-term derivatives, a warp's sums of them
+ *     as three floats); every accumulation across warps and work items, and
+ *     all of the FP64 path's, is FP64.
  *     flags: VPMC_ADJ_SCORE adds the score-function term of the discrete
  *     branch-1 draw (P(I = J) = |omega_J| / Omega), which makes dL/domega an
  *     unbiased estimate of the gradient of the expected trajectory; without
@@ -425,8 +433,10 @@ int vpmc_sim_freeze_sampling(vpmc_sim* sim, int on);
  * always do; with the library's choice (0) unless the shard draws fewer than
  * 32 samples of a sign in a box of the local expansions, or 64 in a bin, on
  * average, where it takes the grid that suits its own samples and agrees with
- * the whole run to FP32 rounding.  (Setting a range may therefore re-plan and
- * grow the working set, as vpmc_sim_set_tuning does.)
+ * the whole run to FP32 rounding.  (An explicit walk with 4 queries a thread
+ * keeps the run's expansions although a thin shard is slower with them; 6 and
+ * 8 queries sum pair by pair at any range.)  Setting a range may re-plan and
+ * grow the working set, as vpmc_sim_set_tuning does.
  * Particles outside the range keep their positions and velocities.  Not with
  * deformation mode or the adjoint (VPMC_ERR_UNSUPPORTED).  Default: [0, N).
  * No reference counterpart (the reference runs on one GPU). */

@@ -2,7 +2,10 @@
 // the reference): checkpointed forward record, segment recompute, and per
 // step the value/gradient field sums at the samples, the per-sample
 // derivatives of the MIS term and the transposed field sum at the particles,
-// each term in the forward's precision and every sum in FP64.
+// each term in the forward's precision.  FP64 path: every sum in FP64.  FP32
+// path: the sums over candidate runs and over a warp's samples as three floats
+// (more digits than FP64), a sample's value and gradient rounded once to FP32
+// (its terms read them so), what goes across warps and work items in FP64.
 #include <algorithm>
 #include <type_traits>
 #include <vector>
@@ -31,7 +34,7 @@ using namespace sim;
 
 // d(v . T)/d{x, f, Omega} of one MIS term (mis_term64's arithmetic), in R
 // arithmetic: FP64 on the FP64 path, FP32 on the FP32 path (each term is then
-// as precise as the forward's FP32 term; the caller accumulates in FP64).
+// as precise as the forward's FP32 term; the caller sums in FP64 or three floats).
 // The factor 1 - (w1 f / cum) / D of df/f is written as the disk term's share
 // w2 p2 / D, which equals it and has no cancellation when branch 1 dominates.
 // With E = w1 f r + w2a cum = D cum r the term needs the reciprocals of E and r^2
@@ -253,8 +256,9 @@ __global__ void k_adj_cum(const InstMC* __restrict__ mc, int n_inst, const float
 }
 
 // Adjoint working set (allocated on first use): per chunk of samples the
-// source index, FP64 value + gradient and dc/df; per particle the transposed
-// sums (by grid slot), two lambda buffers and dL/domega.
+// source index, value + gradient (room for FP64; FP32 on the FP32 path) and FP64
+// dc/df; per particle the transposed sums (by grid slot), two lambda buffers and
+// dL/domega.
 struct AdjBufs {
     int* src;
     double* fg;

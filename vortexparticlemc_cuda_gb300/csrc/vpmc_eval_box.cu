@@ -11,10 +11,14 @@
 // so a candidate adds its terms to 21 (degree 5) moments and every sample evaluates
 // one polynomial.  Candidates whose distance band across the box meets a kink, or
 // that are nearer than kNear half-diagonals, are evaluated pair by pair as in k_eval.
-// With boxes of at most kBoxSide h (half-diagonal rho <= 0.053) the sums are more
-// accurate than the pairwise ones, a few dozen roundings instead of 600: 9e-8 of the
+// With boxes of at most kBoxSide h (half-diagonal rho <= 0.053) the sums are, in norm,
+// more accurate than the pairwise ones, a few dozen roundings instead of 600: 9e-8 of the
 // field's scale against 4e-7 for evenly spread candidates, 2.4e-7 against 4e-7 for a
-// cluster of width 0.02 h.  (Degree 4 is 8 % faster, but velocities next to a cluster
+// cluster of width 0.02 h.  A single value may not be: by the series' tail a candidate at
+// kNear half-diagonals is off by up to 2.0e-6 of its own value at a corner of the box, one
+// of the outer piece by 1.2e-7 of W(0) (the replayed series against the exact kernel;
+// pair by pair 1e-7); the bound for every FP32 field value is 1e-5 of the field's scale.
+// (Degree 4 is 8 % faster, but velocities next to a cluster
 // were 1.3 times further from the FP64 ones than the pairwise sums, by its tail.)
 // The box, not the samples in it, fixes the centre and what is expanded, so a
 // sample's value does not depend on which other samples are drawn.

@@ -78,9 +78,8 @@ struct GenArgs {
     int lane_bits = 0;            // 2^lane_bits threads share a target (set by launch_gen)
 };
 
-// One thread per (target, sign, sample): Philox draw, branch-1 CDF / image /
-// jitter or disk draw, bin + rank (vpmc_sim.cu).
-// Queued on `st`.
+// The samples of the targets [t0, t0 + nt), 2^lane_bits threads a target: Philox draw,
+// branch-1 CDF / image / jitter or disk draw, bin + rank (vpmc_sim.cu).  Queued on `st`.
 int launch_gen(cudaStream_t st, const GenArgs& a);
 
 inline int blocks_for(long n, int threads = 256) {
