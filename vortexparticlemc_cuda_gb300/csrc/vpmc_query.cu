@@ -31,7 +31,22 @@ constexpr double kGatherPairs = double(1L << 27);
 // h_w 8: 445 -> 338 us.
 constexpr double kBinShare = 4.0;
 constexpr int kGatherRows = 4;   // sub-rows a cell
-constexpr int kQueryRows = 16;   // the same for binned points
+// Sub-rows a cell for binned points: 16, halved until the grid has at most 2^22, and no more
+// than 8 a particle or 1 for 16 points (each is a search and 4 bytes).  h_w = 0.001 of the
+// period, 4 M cells: deformed queries of 100 points in 100 particles 360 us with 16, 245
+// with 1 (271 once), FP64 ones 394 and 234; h_w = 0.1, 300,000 points in 10,000 particles:
+// 489 with 16, 583 with 1, 1,000,000 in 100: 511 and 568.
+constexpr int kQueryRows = 16;
+constexpr double kMostSubRows = double(1L << 22);
+
+// For k cells a h_w at the reach h_w cover.
+int query_rows(long N, long M, float hw, float cover, float Lx, float Ly, int k) {
+    const double reach = double(hw) * cover, cells = (double(k) * Lx / reach) * (double(k) * Ly / reach);
+    const double most = std::min(kMostSubRows, std::max(8.0 * double(N), double(M) / 16.0));
+    int rows = kQueryRows;
+    while (rows > 1 && cells * rows > most) rows /= 2;
+    return rows;
+}
 
 __global__ void k_gather_records(const uint32_t* __restrict__ perm, const uint32_t* __restrict__ start, long n, long nsub,
                                  const float2* __restrict__ pos, const float* __restrict__ omega,
@@ -222,8 +237,9 @@ int vpmc_query_vorticity(vpmc_context* ctx, int N, const float* pos, const float
     }
     Work w;
     // smaller cells and sub-rows trim the walk, as in a simulation's passes
-    VPMC_TRY(setup_work(ctx, SLOT_QUERY, N, h_w, Lx, Ly, periodic, M, 0, &w, F ? 0 : sample_k(N, kBinShare * M, Lx, Ly, h_w), cover,
-                        F != nullptr, kQueryRows));
+    const int k = F ? default_k() : sample_k(N, kBinShare * M, Lx, Ly, h_w);
+    VPMC_TRY(setup_work(ctx, SLOT_QUERY, N, h_w, Lx, Ly, periodic, M, 0, &w, k, cover, F != nullptr,
+                        query_rows(N, M, h_w, cover, Lx, Ly, k)));
     VPMC_TRY(grid_build(ctx, w.g, reinterpret_cast<const float2*>(pos), omega, set_mode,
                         reinterpret_cast<const float4*>(F)));
     VPMC_TRY(bin_points(ctx, w.g, w.q, reinterpret_cast<const float2*>(pts), M, 0, 0));
@@ -247,7 +263,8 @@ int vpmc_query_vorticity_f64(vpmc_context* ctx, int N, const float* pos, const f
     VPMC_CUDA(cudaMemsetAsync(out, 0, sizeof(double) * size_t(M), st));
     if (N == 0) return vpmc_context_sync(ctx);
     Work w;
-    VPMC_TRY(setup_work(ctx, SLOT_QUERY, N, h_w, Lx, Ly, periodic, M, 0, &w, 0, 1.f, false, kQueryRows));
+    VPMC_TRY(setup_work(ctx, SLOT_QUERY, N, h_w, Lx, Ly, periodic, M, 0, &w, 0, 1.f, false,
+                        query_rows(N, M, h_w, 1.f, Lx, Ly, default_k())));
     const int set_mode = sign > 0 ? SET_POS_ONLY
                                    : (sign < 0 ? SET_NEG_ONLY : (use_signed ? SET_ONE_SIGNED : SET_ONE_ABS));
     VPMC_TRY(grid_build(ctx, w.g, reinterpret_cast<const float2*>(pos), omega, set_mode));
