@@ -16,20 +16,28 @@ __global__ void k_scale_f32(float* __restrict__ a, long n, float s) {
 // the walk (which is trimmed to the point itself: the columns and sub-rows within
 // reach of it).  Lanes over the points of a bin (k_eval) leave most lanes idle when
 // a bin holds a few points; here a point costs about 0.6 instructions a visited
-// particle against 0.2 for a full bin of 128 points, so up to kGatherPoints points
-// a bin are gathered, and up to kGatherMost with at most kGatherPairs particles in reach
-// of them in all: so few points leave the device idle when they are binned (h_w 16
-// spacings, the call: 50,000 points in 200^2 particles 316 us binned, 167 gathered;
-// 150,000 in 422^2 332 and 302, 250,000 395 and 405).  Needs no binning of the points.  20,011 points in 262,144
+// particle against 0.2 for a full bin of 128 points, and a point has a price of its own
+// (0.4 ns) that binned ones have not.  Gathered are up to kGatherPoints points a
+// half-support cell of up to kGatherSome; up to kGatherMost with at most kGatherPairs
+// particles in reach of them in all (so few points leave the device idle when they are
+// binned); and any number where the cells hold kGatherSparse points or fewer (us a call
+// gathered / binned: 50,000 points in 200^2 particles, h_w 16 spacings: 167 / 316; 200,000 in
+// 600,000, h_w 0.02, 20 a cell: 369 / 390, 400,000, 40 a cell: 596 / 401; 1,000,000 in
+// 300,000, h_w 0.01, 25 a cell: 608 / 286; h_w 0.002, 1 a cell: 502 / 562; 3,000,000,
+// 3 a cell: 1,213 / 669).  Needs no binning of the points.  20,011 points in 262,144
 // particles, h_w = 16 spacings: 224 us binned (half-support cells), 36 us gathered; the
 // whole call 401 -> 143 us.
 constexpr double kGatherPoints = 40.0;
+constexpr long kGatherSome = 3L << 16;
 constexpr long kGatherMost = 1L << 17;
 constexpr double kGatherPairs = double(1L << 27);
+constexpr double kGatherSparse = 1.0;
 // Binned points take cells a quarter as full as a simulation's samples do (37 points):
 // 476,719 points in 422^2 particles, h_w 16 spacings: 557 -> 424 us, 700,000 in 300^2,
 // h_w 8: 445 -> 338 us.
 constexpr double kBinShare = 4.0;
+constexpr double kCrowdedCell = 64.0;     // points a half-support cell
+constexpr double kCrowdedPairs = 7000.0;  // and particles in reach of each
 constexpr int kGatherRows = 4;   // sub-rows a cell
 // Sub-rows a cell for binned points: 16, halved until the grid has at most 2^22, and no more
 // than 8 a particle or 1 for 16 points (each is a search and 4 bytes).  h_w = 0.001 of the
@@ -227,7 +235,8 @@ int vpmc_query_vorticity(vpmc_context* ctx, int N, const float* pos, const float
     // (the gathered form has no staging wait to give up: a limit of 0 polls keeps the
     // binned one, whose first wait then expires)
     const double reach = 3.14159265 * double(N) * h_w * h_w / (double(Lx) * Ly);   // particles within h_w
-    const bool few = double(M) <= kGatherPoints * (2.0 * Lx / h_w) * (2.0 * Ly / h_w) ||
+    const double per_cell = double(M) / ((2.0 * Lx / h_w) * (2.0 * Ly / h_w));
+    const bool few = per_cell <= kGatherSparse || (M <= kGatherSome && per_cell <= kGatherPoints) ||
                      (M <= kGatherMost && double(M) * reach <= kGatherPairs);
     if (!F && ctx->wait_limit > 0 && few) {
         VPMC_TRY(query_gather(ctx, N, reinterpret_cast<const float2*>(pos), omega, M, reinterpret_cast<const float2*>(pts),
@@ -237,7 +246,12 @@ int vpmc_query_vorticity(vpmc_context* ctx, int N, const float* pos, const float
     }
     Work w;
     // smaller cells and sub-rows trim the walk, as in a simulation's passes
-    const int k = F ? default_k() : sample_k(N, kBinShare * M, Lx, Ly, h_w);
+    // one cell a h_w only while its bins are not crowded (the points of a bin are counted and
+    // placed one after the other: 1,000,000 points, 100 particles, h_w 0.05: 470 us with 400
+    // bins, 227 with 1,600; 1,000,000, 10,000, h_w 0.01, 100 a bin: 221 and 259) and their
+    // pairs are few (200,000 points, 600,000 particles, h_w 0.02: 506 and 390)
+    int k = F ? default_k() : sample_k(N, kBinShare * M, Lx, Ly, h_w);
+    if (k == 1 && (per_cell > kCrowdedCell || per_cell * reach > kCrowdedPairs)) k = default_k();
     VPMC_TRY(setup_work(ctx, SLOT_QUERY, N, h_w, Lx, Ly, periodic, M, 0, &w, k, cover, F != nullptr,
                         query_rows(N, M, h_w, cover, Lx, Ly, k)));
     VPMC_TRY(grid_build(ctx, w.g, reinterpret_cast<const float2*>(pos), omega, set_mode,
