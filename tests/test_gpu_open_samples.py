@@ -1,0 +1,45 @@
+"""The library's choice of cells in an open domain counts the samples that fall inside it."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("L", [(1.0, 1.0), (1.0, 0.25), (3.0, 5.0)])
+@pytest.mark.parametrize("law", [0, 1])
+def test_share_of_the_samples(cuda, L, law):
+    """The share of a disk's samples inside: what the plan takes for the unbiased law is close to it."""
+    from vortexparticlemc_cuda_gb300 import phash as P
+    rng = np.random.default_rng(1)
+    pos = (rng.random((2000, 2)) * L).astype(np.float32)
+    sim = P.Simulation(P.SimParam(dt=1e-3, Nx=64, hwr=4, N1=0, N2=64, Lx=L[0], Ly=L[1], periodic=False, law=law, seed=3), [2000])
+    sim.set_particles(torch.from_numpy(pos).cuda(), torch.from_numpy(rng.normal(size=2000).astype(np.float32)).cuda())
+    sim.prepare()
+    sim.velocity(1)
+    xy = sim.read_samples(0, 2000 * 128)[1]
+    inside = float(((xy >= 0) & (xy <= np.array(L, np.float32))).all(1).mean())
+    area, R = L[0] * L[1], np.hypot(*L)
+    taken = 2.973 * np.sqrt(area) / (2 * np.pi * R)
+    # measured to 3 standard errors of 256,000 samples, grouped by target; a long domain's share is
+    # smaller (its points are further apart), the reference law's too
+    assert inside <= taken + 0.01
+    if law == 1:
+        assert inside >= taken * (1.0 - 0.02 if L == (1.0, 1.0) else 0.75) - 0.01
+    sim.close()
+
+
+# 64^2 particles, h_w 11 spacings: boxes of h_w / 14 have 1.28 n samples of all n + n, and
+# 0.854 n of those inside an open domain
+@pytest.mark.parametrize("n,periodic,boxed", [(38, True, True), (36, False, False), (56, False, True)])
+def test_boxes_by_them(cuda, n, periodic, boxed):
+    from vortexparticlemc_cuda_gb300 import phash as P
+    rng = np.random.default_rng(n)
+    sim = P.Simulation(P.SimParam(dt=1e-3, Nx=64, hwr=11, N1=n, N2=n, periodic=periodic), [4096])
+    sim.set_particles(torch.from_numpy(rng.random((4096, 2)).astype(np.float32)).cuda(),
+                      torch.from_numpy((rng.normal(size=4096) / 4096).astype(np.float32)).cuda())
+    sim.prepare()
+    got = sim.velocity(1)
+    sim.set_tuning(sim.tuning()[0], 6)         # the same cells pair by pair
+    assert torch.equal(got, sim.velocity(1)) == (not boxed)
+    sim.close()
