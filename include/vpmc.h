@@ -431,9 +431,9 @@ int vpmc_sim_freeze_sampling(vpmc_sim* sim, int on);
  * run on several GPUs all-gathers the updated positions after each step.  Both
  * must sum on the same grid: with a walk given to vpmc_sim_set_tuning they
  * always do; with the library's choice (0) unless the shard draws fewer than
- * 32 samples of a sign in a box of the local expansions, or 64 in a bin, on
- * average, where it takes the grid that suits its own samples and agrees with
- * the whole run to FP32 rounding.  (An explicit walk with 4 queries a thread
+ * 28 + 7000 / (particles within h_w) samples of a sign in a box of the local
+ * expansions, or 64 in a bin, on average, where it takes the grid that suits
+ * its own samples and agrees with the whole run to FP32 rounding.  (An explicit walk with 4 queries a thread
  * keeps the run's expansions although a thin shard is slower with them; 6 and
  * 8 queries sum pair by pair at any range.)  Setting a range may re-plan and
  * grow the working set, as vpmc_sim_set_tuning does.

@@ -18,13 +18,14 @@ def simulation(P, counts, walk=0, qpt=4, **kw):
     return sim
 
 
-# 64^2 particles, 128 samples of a sign each: 6 cells a h_w in boxes of 1 / 4 cell (57 samples
-# each) hold to 2,304 targets, then 7 in boxes of 1 / 2 cell to 784, then pairs on 6 and fewer
+# 64^2 particles, 804 of them within h_w, 128 samples of a sign each: boxes ask for 36.7; 6 cells
+# a h_w in boxes of 1 / 4 cell hold to 2,643 targets, then 7 in boxes of 1 / 2 cell to 900, then
+# pairs on 6 and fewer
 DENSE = dict(Nx=64, hwr=16, N1=64, N2=64)
 
 
-@pytest.mark.parametrize("begin,end,k,qpt", [(0, 4095, 6, 4), (1700, 4004, 6, 4), (0, 2303, 7, 4), (100, 884, 7, 4),
-                                             (0, 783, 6, 6), (5, 55, 2, 6)])   # 6 queries a thread: pair by pair
+@pytest.mark.parametrize("begin,end,k,qpt", [(0, 4095, 6, 4), (1400, 4050, 6, 4), (0, 2640, 7, 4), (100, 1002, 7, 4),
+                                             (0, 898, 6, 6), (5, 55, 2, 6)])   # 6 queries a thread: pair by pair
 def test_dense_run(cuda, begin, end, k, qpt):
     from vortexparticlemc_cuda_gb300 import phash as P
     sim = simulation(P, [4096], **DENSE)

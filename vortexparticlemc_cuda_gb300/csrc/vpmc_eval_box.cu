@@ -385,11 +385,12 @@ int launch_eval_box(vpmc_context* ctx, const EvalBoxArgs& a, bool field9) {
 }
 
 int box_split(long n, double samples, float Lx, float Ly, float hw, int gx, int gy) {
-    if (3.14159265 * double(n) * hw * hw < kBoxReach * double(Lx) * Ly) return 0;
+    const double reach = 3.14159265 * double(n) * hw * hw / (double(Lx) * Ly);
+    if (reach < kBoxReach) return 0;
     const double side = std::max(double(Lx) / gx, double(Ly) / gy);
-    const double per_bin = samples / (double(gx) * gy);
+    const double per_bin = samples / (double(gx) * gy), least = kBoxSamples + kBoxFixed / reach;
     for (int nb = 1; nb <= 4; nb *= 2)
-        if (side / nb <= double(kBoxSide) * hw) return per_bin >= kBoxSamples * nb * nb ? nb : 0;
+        if (side / nb <= double(kBoxSide) * hw) return per_bin >= least * nb * nb ? nb : 0;
     return 0;
 }
 

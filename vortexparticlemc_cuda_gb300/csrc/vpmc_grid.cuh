@@ -420,7 +420,8 @@ int launch_eval_tc(vpmc_context* ctx, const EvalTcArgs& a, bool field9);
 // The FIELD / FIELD9 evaluation of boxed instances by local expansions (vpmc_eval_box.cu).
 constexpr int kBoxChunk = 192;        // samples an item
 constexpr float kBoxSide = 0.075f;    // largest box side, in h_w
-constexpr double kBoxSamples = 32.0;  // samples a box gathers at least (on average)
+constexpr double kBoxSamples = 28.0;  // samples a box gathers at least (on average), with many particles,
+constexpr double kBoxFixed = 7000.0;  // and this many more divided by the particles within h_w
 constexpr double kBoxReach = 80.0;    // particles within h_w at least (on average)
 struct EvalBoxArgs {
     const GridInst* inst;
@@ -437,10 +438,12 @@ struct EvalBoxArgs {
 };
 int launch_eval_box(vpmc_context* ctx, const EvalBoxArgs& a, bool field9);
 // Boxes per cell and axis for an instance of n particles with `samples` points a sign
-// set and pass (0: pair by pair).  512^2 particles, evaluation of a step by boxes and
-// pair by pair: 84 samples a box 4.2 and 8.5 ms, 63: 3.5 and 6.6, 42: 4.5 and 5.3 (and
-// 0.82 and 1.26 for 256^2), 21: 3.9 and 2.8; 113 particles within h_w 9.9 and 12.9, 50
-// particles 11.7 and 8.7.
+// set and pass (0: pair by pair).  What a box costs, its walk and the sum of its moments,
+// is spread over its samples, and saves more the more particles are in reach.  A step of
+// 256^2 particles by boxes of h_w / 14 over one pair by pair, at 32, 40, 50, 64, 84 and 120
+// samples a box: 804 particles within h_w 1.02 0.91 0.79 0.75 0.68 0.58; 452: 1.13 1.01 0.89
+// 0.83 0.76 0.64; 201: 1.38 1.23 1.06 0.98 0.91 0.85; 113: 1.51 1.33 1.20 1.12 1.06 1.01; 82:
+// 1.58 1.41 1.28 1.18 1.06 (128^2: 0.91 at 120); 512^2 and 1024^2 the same within 0.04.
 int box_split(long n, double samples, float Lx, float Ly, float hw, int gx, int gy);
 
 }  // namespace vpmc

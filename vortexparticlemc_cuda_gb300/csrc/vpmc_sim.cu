@@ -818,9 +818,9 @@ int upload_mc(vpmc_sim* s) {
 //
 // Cells and boxes are chosen by the samples of a whole run, so that a shard of one sums as
 // the run does, bit for bit.  Where the walk is the library's choice, that holds for as
-// long as it pays with the samples the shard draws: with fewer than kBoxSamples a box, or
-// kShardSamples a bin, it chooses by its own, never fewer cells than the default walk
-// unless the run has fewer.  A pass over 1 / 8 of 1024^2 targets, h_w 16 spacings, 64 + 64
+// long as it pays with the samples the shard draws: with too few for the run's boxes
+// (box_split), or fewer than kShardSamples a bin, it chooses by its own, never fewer cells
+// than the default walk unless the run has fewer.  A pass over 1 / 8 of 1024^2 targets, h_w 16 spacings, 64 + 64
 // samples: 26.1 ms with the run's boxes (7 samples each), 11.4 with its own cells; 1 / 16:
 // 24.6 and 6.4; 1 / 16 of the same with h_w 8, 32 + 32: 2.16 ms with the run's cells (28 a
 // bin), 1.80 with its own, 1 / 8 (57 a bin) 3.03 and 2.85, 1 / 4 (114) 4.91 and 4.85.
@@ -866,9 +866,9 @@ long plan_instances(const vpmc_sim* s, std::vector<GridInst>& plan) {
     for (int i = 0; i < s->n_inst; ++i) {
         GridInst& g = plan[i];
         g.nb = boxes(g, i);
-        const double bins = double(g.gx) * g.gy;
-        if (s->k_walk || drawn[i] <= 0.0 || drawn[i] >= bins * (g.nb ? kBoxSamples * g.nb * g.nb : kShardSamples) ||
-            drawn[i] >= by[i])
+        if (s->k_walk || drawn[i] <= 0.0 || drawn[i] >= by[i]) continue;
+        if (g.nb ? box_split(s->counts[i], drawn[i], g.Lx, g.Ly, g.hw, g.gx, g.gy) == g.nb
+                 : drawn[i] >= kShardSamples * g.gx * g.gy)
             continue;
         by[i] = drawn[i];
         d[i].k = std::max(sample_k(s->counts[i], by[i], g.Lx, g.Ly, g.hw, can_box), std::min(d[i].k, default_k()));

@@ -10,8 +10,8 @@ the path's one exchange (8 bytes per particle per step).  A sample's Philox
 counter is keyed by its target's instance-local index and the step, so a
 sharded run gives, bit for bit, the positions of the one-GPU run in the same
 explicit tuning.  With the library's own choice of walk it does as long as a
-rank's samples are dense enough for the whole run's grid (32 of a sign in each
-box of the local expansions, 64 in each bin); a thinner shard takes the grid
+rank's samples are dense enough for the whole run's grid (28 + 7000 / (particles
+within h_w) of a sign in each box of the local expansions, 64 in each bin); a thinner shard takes the grid
 that suits its samples and agrees to FP32 rounding.
 
 Ensembles: instances are independent, so they are split over ranks by
