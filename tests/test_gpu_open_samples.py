@@ -43,3 +43,13 @@ def test_boxes_by_them(cuda, n, periodic, boxed):
     sim.set_tuning(sim.tuning()[0], 6)         # the same cells pair by pair
     assert torch.equal(got, sim.velocity(1)) == (not boxed)
     sim.close()
+
+
+@pytest.mark.parametrize("n,periodic,k", [(8, True, 3), (12, True, 4), (4, False, 2), (8, False, 2), (12, False, 2), (16, False, 3)])
+def test_cells_by_them(cuda, n, periodic, k):
+    """64^2 particles, h_w 11 spacings: a bin of k cells a h_w holds 242 n / k^2 samples, 161 n / k^2 inside an open
+    domain; 150 are asked for, 250 there for more than two cells."""
+    from vortexparticlemc_cuda_gb300 import phash as P
+    sim = P.Simulation(P.SimParam(dt=1e-3, Nx=64, hwr=11, N1=n, N2=n, periodic=periodic), [4096])
+    assert sim.tuning()[0] == k
+    sim.close()

@@ -269,8 +269,10 @@ struct InstDesc {
 long grid_plan(const InstDesc* in, int n, int k, int nsets, GridInst* out);
 int default_k();
 // Walk cells per h_w for an instance of n particles that evaluates `samples` points
-// of each sign set a pass (boxes: whether local expansions may sum them).
-int sample_k(long n, double samples, float Lx, float Ly, float hw, bool boxes = false);
+// of each sign set a pass (boxes: whether local expansions may sum them; fill: samples a
+// bin of more than two cells gathers at least).
+constexpr double kBinFill = 150.0, kOpenBinFill = 250.0;
+int sample_k(long n, double samples, float Lx, float Ly, float hw, bool boxes = false, double fill = kBinFill);
 
 // Device-side working set of one grid (caller owns the memory).
 struct GridBufs {

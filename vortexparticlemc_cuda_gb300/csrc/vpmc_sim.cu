@@ -854,7 +854,8 @@ long plan_instances(const vpmc_sim* s, std::vector<GridInst>& plan) {
         by[i] = std::min(double(s->counts[i]) * per, most);
         d[i] = InstDesc{s->prm[i].Lx, s->prm[i].Ly, s->mc[i].hw, s->prm[i].periodic, int(b), int(e),
                         s->deform ? s->cover : 1.f,
-                        sample_k(s->counts[i], by[i], s->prm[i].Lx, s->prm[i].Ly, s->mc[i].hw, can_box)};
+                        sample_k(s->counts[i], by[i], s->prm[i].Lx, s->prm[i].Ly, s->mc[i].hw, can_box,
+                                 s->prm[i].periodic ? kBinFill : kOpenBinFill)};
     }
     auto boxes = [&](const GridInst& g, int i) {
         return can_box ? box_split(s->counts[i], by[i], g.Lx, g.Ly, g.hw, g.gx, g.gy) : 0;
@@ -871,7 +872,8 @@ long plan_instances(const vpmc_sim* s, std::vector<GridInst>& plan) {
                  : drawn[i] >= kShardSamples * g.gx * g.gy)
             continue;
         by[i] = drawn[i];
-        d[i].k = std::max(sample_k(s->counts[i], by[i], g.Lx, g.Ly, g.hw, can_box), std::min(d[i].k, default_k()));
+        d[i].k = std::max(sample_k(s->counts[i], by[i], g.Lx, g.Ly, g.hw, can_box, g.periodic ? kBinFill : kOpenBinFill),
+                          std::min(d[i].k, default_k()));
         again = true;
     }
     if (!again) return nb;
