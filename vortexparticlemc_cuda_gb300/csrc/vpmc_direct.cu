@@ -659,7 +659,12 @@ extern "C" int vpmc_direct_velocity_f32(vpmc_context* ctx, int kernel, int N, co
     if (nchunk > 4096) nchunk = 4096;
     long chunk = (long(N) + nchunk - 1) / nchunk;
     if (packed) chunk = (chunk + tile - 1) / tile * tile;
-    if (chunk < tile) chunk = tile;
+    // (few targets: the chunks' partials are added one after the other, 55 ns each, so a
+    // chunk is four tiles at least: 50,000 sources, 100 targets, no period, 102 us a call
+    // with 782 chunks, 63 with 196, 83 before the tiles were packed; 600 targets 121, 74
+    // and 100)
+    const long least = packed && tblocks <= 2 ? 4 * tile : tile;
+    if (chunk < least) chunk = least;
     nchunk = N > 0 ? (long(N) + chunk - 1) / chunk : 1;
     char* base = nullptr;
     VPMC_TRY(scratch(ctx, SLOT_DIRECT, sizeof(float2) * size_t(nchunk) * size_t(M) + 256, &base));
