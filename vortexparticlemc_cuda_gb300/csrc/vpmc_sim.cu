@@ -329,9 +329,10 @@ struct AccArgs {
     const unsigned* flags;        // FLAG_TIMEOUT: the field values were not all written
 };
 
-// The samples a sum may read: none after an evaluation that gave up (the particles then
-// stay where they are, and the call returns the timeout).
-__device__ __forceinline__ int sampled(const unsigned* flags, int n) { return (*flags & FLAG_TIMEOUT) ? 0 : n; }
+// Whether the samples' values are this pass's: after an evaluation that gave up the
+// velocities are 0 (the particles then stay where they are, and the call returns the
+// timeout).  Read first and used last, so that nothing waits for it.
+__device__ __forceinline__ bool evaluated(const unsigned* flags) { return !(*flags & FLAG_TIMEOUT); }
 
 // mis_contrib_dev (src/cuda/monte_carlo_bs.cu:35-51) for the reference law;
 // the balance-heuristic estimator with the true sampling densities for the
@@ -385,7 +386,8 @@ __global__ void __launch_bounds__(256) k_accum(AccArgs a) {
     constexpr int kPerWarp = 32 / kAccLanes;
     const long warp = (long(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const long nwarps = (long(gridDim.x) * blockDim.x) >> 5;
-    const int Q = a.N1 + a.N2, nq = sampled(a.flags, Q);
+    const int Q = a.N1 + a.N2;
+    const bool whole = evaluated(a.flags);
     const float w1 = float(a.N1) / float(Q), w2 = float(a.N2) / float(Q);
     const float inv = 1.f / float(Q);
     // the loop runs the same trips in every lane of a warp (the group sums shuffle)
@@ -402,7 +404,7 @@ __global__ void __launch_bounds__(256) k_accum(AccArgs a) {
             KSum sx, sy;
             const long base = (tl * 2 + s) * Q;
             const float cum = I.cum9[s], inv_cum = 1.f / cum;
-            for (int j0 = sub; j0 < nq; j0 += 4 * kAccLanes) {
+            for (int j0 = sub; j0 < Q; j0 += 4 * kAccLanes) {
                 float2 y[4];
                 float f[4];
 #pragma unroll
@@ -429,8 +431,8 @@ __global__ void __launch_bounds__(256) k_accum(AccArgs a) {
         if (live && sub == 0) {
             // u(+) - u(-) with the leading parts subtracted exactly: a near-singular
             // sample makes both sign sums large, their difference small
-            const float vx = comp_diff(u[0][0], uc[0][0], u[1][0], uc[1][0]) * inv;
-            const float vy = comp_diff(u[0][1], uc[0][1], u[1][1], uc[1][1]) * inv;
+            const float vx = whole ? comp_diff(u[0][0], uc[0][0], u[1][0], uc[1][0]) * inv : 0.f;
+            const float vy = whole ? comp_diff(u[0][1], uc[0][1], u[1][1], uc[1][1]) * inv : 0.f;
             a.vel[t] = make_float2(vx, vy);
             if (a.advect) {
                 double nx = double(x.x) + double(I.dt) * double(vx);
@@ -485,7 +487,8 @@ __global__ void __launch_bounds__(256) k_accum5(Acc5Args a) {
     constexpr int kPerWarp = 32 / kAccLanes;
     const long warp = (long(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const long nwarps = (long(gridDim.x) * blockDim.x) >> 5;
-    const int Q = a.N1 + 5 * a.N2, n1 = sampled(a.flags, a.N1), n2 = sampled(a.flags, a.N2);
+    const int Q = a.N1 + 5 * a.N2;
+    const bool whole = evaluated(a.flags);
     const float w1 = float(a.N1) / float(a.N1 + a.N2), w2 = float(a.N2) / float(a.N1 + a.N2);
     const float inv = 1.f / float(a.N1 + a.N2);
     // the loop runs the same trips in every lane of a warp (the group sums shuffle)
@@ -511,7 +514,7 @@ __global__ void __launch_bounds__(256) k_accum5(Acc5Args a) {
             const long base = (tl * 2 + s) * Q;
             const float cum = I.cum9[s], inv_cum = 1.f / cum;
 #pragma unroll 2
-            for (int j = sub; j < n1; j += kAccLanes) {
+            for (int j = sub; j < a.N1; j += kAccLanes) {
                 const float2 y = live ? a.ys[base + j] : make_float2(0.f, 0.f);
                 const float f = live ? a.fv[base + j] : 0.f;
 #pragma unroll
@@ -525,7 +528,7 @@ __global__ void __launch_bounds__(256) k_accum5(Acc5Args a) {
             for (int k = 0; k < 5; ++k) {
                 const long b0 = base + a.N1 + long(k) * a.N2;
 #pragma unroll 2
-                for (int j = sub; j < n2; j += kAccLanes) {
+                for (int j = sub; j < a.N2; j += kAccLanes) {
                     const float2 y = live ? a.ys[b0 + j] : make_float2(0.f, 0.f);
                     const float f = live ? a.fv[b0 + j] : 0.f;
                     const float2 c = mis_term(I.law, xa[k], y, f, w1, w2, cum, inv_cum, alpha[k], R[k], I, inv_Lx, inv_Ly);
@@ -546,7 +549,8 @@ __global__ void __launch_bounds__(256) k_accum5(Acc5Args a) {
 #pragma unroll
         for (int k = 0; k < 5; ++k)
 #pragma unroll
-            for (int d = 0; d < 2; ++d) u[k][d] = comp_diff(su[0][k][d], cu[0][k][d], su[1][k][d], cu[1][k][d]) * inv;
+            for (int d = 0; d < 2; ++d)
+                u[k][d] = whole ? comp_diff(su[0][k][d], cu[0][k][d], su[1][k][d], cu[1][k][d]) * inv : 0.f;
         if (live && sub == 0) {
             const float vx = u[0][0], vy = u[0][1];
             a.vel[t] = make_float2(vx, vy);
@@ -638,7 +642,8 @@ __global__ void __launch_bounds__(256) k_accum64(AccArgs64 a) {
     const int lane = threadIdx.x & 31;
     const long warp = (long(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const long nwarps = (long(gridDim.x) * blockDim.x) >> 5;
-    const int Q = a.N1 + a.N2, nq = sampled(a.flags, Q);
+    const int Q = a.N1 + a.N2;
+    const bool whole = evaluated(a.flags);
     const double w1 = double(a.N1) / Q, w2 = double(a.N2) / Q;
     // an instance's constants, kept over the warp's targets
     int cur = -1;
@@ -660,7 +665,7 @@ __global__ void __launch_bounds__(256) k_accum64(AccArgs64 a) {
         for (int s = 0; s < 2; ++s) {
             double sx = 0.0, sy = 0.0;
             const long base = (tl * 2 + s) * Q;
-            for (int j = lane; j < nq; j += 32) {
+            for (int j = lane; j < Q; j += 32) {
                 const double2 c = mis_term64(I.law, x, a.ys[base + j], a.fv[base + j], w1, w2a, cum[s], R, I);
                 sx += c.x;
                 sy += c.y;
@@ -680,6 +685,7 @@ __global__ void __launch_bounds__(256) k_accum64(AccArgs64 a) {
         for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
         v /= Q;
         v -= __shfl_xor_sync(0xffffffffu, v, 16);   // lanes below 16: u+ - u-
+        if (!whole) v = 0.0;
         if (lane == 0 || lane == 8) {
             reinterpret_cast<float*>(a.vel)[2 * t + (hy ? 1 : 0)] = float(v);
             if (a.advect) {
